@@ -185,9 +185,14 @@ __device__ __forceinline__ bool sol_ref_rinv3_fast(double a, double& rij, double
   return ok;
 }
 
-static __device__ __noinline__ void sol_ref_rinv3_slow(double a, double& rij, double& rijm3) {
-  rij = __dsqrt_rn(a);
-  rijm3 = __ddiv_rn(1.0, a * rij);
+static __device__ __noinline__ double2 sol_ref_rinv3_ieee(double a) {
+  const double r = __dsqrt_rn(a);
+  return make_double2(r, __ddiv_rn(1.0, a * r));
+}
+__device__ __forceinline__ void sol_ref_rinv3_slow(double a, double& rij, double& rijm3) {
+  const double2 v = sol_ref_rinv3_ieee(a);
+  rij = v.x;
+  rijm3 = v.y;
 }
 
 // rij = RN(sqrt(a)), rijm3 = RN(1 / RN(a * rij)), bit-identical to IEEE
@@ -199,38 +204,74 @@ __device__ __forceinline__ void sol_ref_rinv3(double a, double& rij, double& rij
 // ---- IEEE double multiplication on the integer pipe ----------------------------
 // Round-to-nearest-even product of two doubles from 32-bit integer
 // multiplies of the significands (the 106-bit product in three words, the
-// leading 53 bits, guard and sticky bits): the textbook IEEE 754 multiply.
-// It is exact wherever the inputs are finite and normal or zero and the
-// product is normal or zero; ok turns false elsewhere (the caller then takes
-// the FP64 instruction).  A pair's term multiplies move here from the FP64
-// pipe, which binds the reference form, to the integer pipe, which it leaves
-// mostly idle.
+// leading 53 bits, the bits below them compared with one half): the textbook
+// IEEE 754 multiply.  It serves operands that are zero or of magnitude
+// [2^-423, 2^424), whose product is a normal number, so the product's own
+// exponent needs no test; ok turns false elsewhere (the caller then takes the
+// FP64 instruction).  The FP64 pipe binds the reference form; the integer
+// pipe, which it leaves mostly idle, takes a pair's multiplications.
+
+// (t3, w1, w0): a 106-bit significand product in [2^104, 2^106); its sign
+// and the exponent field of its 2^104 binade in place (hi).  The result's
+// high and low words, rounded to nearest even; a rounding carry out of the
+// significand moves into the exponent field.
+__device__ __forceinline__ void exact_round(unsigned long long t3, unsigned w1, unsigned w0, unsigned hi,
+                                            unsigned& rh, unsigned& rl) {
+  const unsigned t3h = (unsigned)(t3 >> 32), t3l = (unsigned)t3;
+  const unsigned n = t3h >> 9;  // product >= 2^105: one more place to drop
+  const unsigned s = 20 + n;
+  const unsigned ml = __funnelshift_r(w1, t3l, s), mh = __funnelshift_r(t3l, t3h, s);  // the leading 53 bits
+  const unsigned rem = (w1 << (12 - n)) | (w0 != 0u ? 1u : 0u);  // the rest, its half at bit 31
+  const unsigned up = rem > 0x80000000u - (ml & 1u) ? 1u : 0u;
+  const unsigned long long r = (((unsigned long long)(mh + hi + (n << 20) - 0x100000u) << 32) | ml) + up;
+  rh = (unsigned)(r >> 32);
+  rl = (unsigned)r;
+}
+// Operand exponent fields this multiply serves: [600, 1447) (high word, sign shifted out)
+__device__ __forceinline__ bool exact_range(unsigned h) { return (h << 1) - (600u << 21) < (847u << 21); }
+
+// AZ / BZ: whether a / b may be zero on the fast path (else a zero counts as
+// out of range): a component that is zero by symmetry (a planar system's z).
+template <bool AZ = true, bool BZ = true>
 __device__ __forceinline__ double sol_exact_dmul(double a, double b, bool& ok) {
   const unsigned ah = (unsigned)__double2hiint(a), al = (unsigned)__double2loint(a);
   const unsigned bh = (unsigned)__double2hiint(b), bl = (unsigned)__double2loint(b);
-  const int ea = (int)((ah >> 20) & 0x7FFu), eb = (int)((bh >> 20) & 0x7FFu);
-  const unsigned sign = (ah ^ bh) & 0x80000000u;
   const unsigned mah = (ah & 0xFFFFFu) | 0x100000u, mbh = (bh & 0xFFFFFu) | 0x100000u;
-  // Ma Mb in [2^104, 2^106): bits 64.. in t3, 32..63 in w1, 0..31 in w0
   const unsigned long long t0 = (unsigned long long)al * bl;
-  const unsigned long long t1 = (unsigned long long)mah * bl + (t0 >> 32);
-  const unsigned long long t2 = (unsigned long long)al * mbh + (t1 & 0xFFFFFFFFull);
-  const unsigned long long t3 = (unsigned long long)mah * mbh + (t1 >> 32) + (t2 >> 32);
-  const unsigned w1 = (unsigned)t2, w0 = (unsigned)t0;
-  const int n = (int)(t3 >> 41);  // product >= 2^105: one more place to drop
-  const int s = 20 + n;
-  const unsigned long long m = (t3 << (32 - s)) | (unsigned long long)(w1 >> s);  // the leading 53 bits
-  const unsigned guard = (w1 >> (s - 1)) & 1u;
-  const unsigned sticky = (w1 & ((1u << (s - 1)) - 1u)) | w0;
-  const unsigned long long rnd = guard & ((sticky != 0u) | (unsigned)(m & 1ull));
-  const int e = ea + eb - 1023 + n;
-  const bool za = (ea == 0) & (((ah & 0xFFFFFu) | al) == 0u);
-  const bool zb = (eb == 0) & (((bh & 0xFFFFFu) | bl) == 0u);
+  const unsigned long long t1 = (unsigned long long)mah * bl + (unsigned)(t0 >> 32);
+  const unsigned long long t2 = (unsigned long long)al * mbh + (unsigned)t1;
+  const unsigned long long t3 = (unsigned long long)mah * mbh + (unsigned)(t1 >> 32) + (unsigned)(t2 >> 32);
+  const unsigned sign = (ah ^ bh) & 0x80000000u;
+  unsigned rh, rl;
+  exact_round(t3, (unsigned)t2, (unsigned)t0, (ah & 0x7FF00000u) + (bh & 0x7FF00000u) - (1023u << 20), rh, rl);
+  const bool za = AZ && (ah << 1 | al) == 0u, zb = BZ && (bh << 1 | bl) == 0u;
   const bool zero = za | zb;
-  ok = ok && ((ea != 0) | za) && ((eb != 0) | zb) && (ea != 0x7FF) && (eb != 0x7FF) && (zero | ((e >= 1) & (e <= 2045)));
-  // a rounding carry out of the significand moves into the exponent field
-  const unsigned long long bits = zero ? 0ull : ((unsigned long long)e << 52) + (m - (1ull << 52)) + rnd;
-  return __longlong_as_double((long long)(bits | ((unsigned long long)sign << 32)));
+  ok = ok & (za | exact_range(ah)) & (zb | exact_range(bh));
+  return __hiloint2double((int)((zero ? 0u : rh) | sign), (int)(zero ? 0u : rl));
+}
+
+// The square of a double, likewise (three partial products, no sign).
+template <bool AZ = true>
+__device__ __forceinline__ double sol_exact_dsqr(double a, bool& ok) {
+  const unsigned ah = (unsigned)__double2hiint(a), al = (unsigned)__double2loint(a);
+  const unsigned mah = (ah & 0xFFFFFu) | 0x100000u;
+  const unsigned long long t0 = (unsigned long long)al * al;
+  const unsigned long long t1 = (unsigned long long)(mah << 1) * al + (unsigned)(t0 >> 32);
+  const unsigned long long t3 = (unsigned long long)mah * mah + (unsigned)(t1 >> 32);
+  unsigned rh, rl;
+  exact_round(t3, (unsigned)t1, (unsigned)t0, ((ah & 0x7FF00000u) << 1) - (1023u << 20), rh, rl);
+  const bool zero = AZ && (ah << 1 | al) == 0u;
+  ok = ok & (zero | exact_range(ah));
+  return __hiloint2double((int)(zero ? 0u : rh), (int)(zero ? 0u : rl));
+}
+
+struct SolVec3 {
+  double x, y, z;
+};
+// (by value: a reference argument of a function that is not inlined would keep its variable in local memory)
+static __device__ __noinline__ SolVec3 sol_ref_terms_slow(double gm, double rijm3, double dx, double dy, double dz,
+                                                          double px, double py, double pz) {
+  return SolVec3{gm * (dx * rijm3 - px), gm * (dy * rijm3 - py), gm * (dz * rijm3 - pz)};
 }
 
 // The reference's pair term gm (d rijm3 - p) per component
@@ -239,16 +280,17 @@ __device__ __forceinline__ double sol_exact_dmul(double a, double b, bool& ok) {
 __device__ __forceinline__ void sol_ref_terms(double gm, double rijm3, double dx, double dy, double dz, double px,
                                               double py, double pz, double& tx, double& ty, double& tz) {
   bool ok = true;
-  const double ux = sol_exact_dmul(dx, rijm3, ok) - px;
-  const double uy = sol_exact_dmul(dy, rijm3, ok) - py;
-  const double uz = sol_exact_dmul(dz, rijm3, ok) - pz;
-  tx = sol_exact_dmul(gm, ux, ok);
-  ty = sol_exact_dmul(gm, uy, ok);
-  tz = sol_exact_dmul(gm, uz, ok);
+  const double ux = sol_exact_dmul<false, false>(dx, rijm3, ok) - px;
+  const double uy = sol_exact_dmul<false, false>(dy, rijm3, ok) - py;
+  const double uz = sol_exact_dmul<true, false>(dz, rijm3, ok) - pz;
+  tx = sol_exact_dmul<false, false>(gm, ux, ok);
+  ty = sol_exact_dmul<false, false>(gm, uy, ok);
+  tz = sol_exact_dmul<false, true>(gm, uz, ok);
   if (!ok) {
-    tx = gm * (dx * rijm3 - px);
-    ty = gm * (dy * rijm3 - py);
-    tz = gm * (dz * rijm3 - pz);
+    const SolVec3 t = sol_ref_terms_slow(gm, rijm3, dx, dy, dz, px, py, pz);
+    tx = t.x;
+    ty = t.y;
+    tz = t.z;
   }
 }
 

@@ -202,7 +202,8 @@ __global__ void __launch_bounds__(kRateThreads) k_fp32_rate(float b, float c, fl
 //   5: a = (1 + u, 2 +- u or 4 - u) 4^k, u log-uniform over [2^-60, 2^-10]:
 //      square roots and reciprocals next to powers of two;
 //   6: the integer-pipe multiply sol_exact_dmul against the FP64 instruction,
-//      random signed operands with exponents over [2^-300, 2^300];
+//      random signed operands with exponents over [2^-300, 2^300], and its
+//      square sol_exact_dsqr;
 //   7: the same with significands whose product sits next to 2^104 or 2^106,
 //      zeros and squares;
 //   8, 9: the step-size powers pow(em, -0.2) and pow(em, -0.25)
@@ -282,6 +283,9 @@ __global__ void k_check_rinv3(int mode, long long n, unsigned long long seed, un
       const double b = __longlong_as_double((long long)((eb << 52) | mb | ((h2 & 1ull) << 63)));
       const double e = sol_exact_dmul(a, b, ok);
       bad = ok && (__double_as_longlong(e) != __double_as_longlong(__dmul_rn(a, b)));
+      bool ok2 = true;
+      const double e2 = sol_exact_dsqr(a, ok2);
+      bad = bad || (ok2 && (__double_as_longlong(e2) != __double_as_longlong(__dmul_rn(a, a))));
     } else if (mode <= 2 || mode == 5) {
       double a;
       if (mode == 5) {

@@ -404,316 +404,194 @@ __global__ void __launch_bounds__(kSinkBlock) k_gravity_ac(ForceCtx fc, const do
   out[5] = a[2];
 }
 
-// ---- FP64 GravityAC for systems of up to a few ten thousand bodies ----------
-// One thread per sink leaves most SMs idle when the sinks number a few
-// thousand or fewer.  Here a CTA takes kFewSinks sinks: producer warps compute
-// the pair terms of a tile of kFewTile sources for all of them in parallel
-// (the reference's arithmetic, Acceleration.cpp:294-317) into a
-// double-buffered shared tile, while warp 0 adds the previous tile's terms
-// per sink and component in ascending source order.  The sums are the
-// reference's sequential sums, so the result is bit-identical to it and to
-// k_gravity_ac, with kFewSinks x kFewTile-way parallelism per CTA.  Measured
-// on the GB300 it matches or beats k_gravity_ac from 1,033 to 65,536 bodies
-// (9.0 / 13.7 G pairs/s at 1,033 / 32,768 all-massive bodies), so it serves
-// every system whose sinks see at least one tile of sources.
-constexpr int kFewSinks = 4;
-constexpr int kFewProducers = 7;                      // warps 1..7
-constexpr int kFewTile = kFewProducers * 32;          // 224 sources per round
-constexpr int kFewTerms = kFewSinks * 3;              // (sink, component) lanes of warp 0
+// ---- FP64 GravityAC for sinks with many sources -------------------------------
+// A CTA takes spc sinks.  Its PW producing warps compute the pair terms of a
+// tile of kRefTile sources for all of them (the reference's arithmetic,
+// Acceleration.cpp:294-317; a warp takes one sink and half a tile at a time)
+// into one of two shared tiles, while its SW summing warps -- one lane per
+// (sink, component) -- add the previous tile's terms in ascending source
+// order: the reference's sequential sums, bit for bit.
+//
+// What bounds it.  The FP64 pipe is shared by the SM's four sub-partitions
+// and takes one warp instruction per 16 cycles (19 for additions and
+// multiplications), and one warp's instructions follow each other at 64
+// cycles at the earliest, dependent or not.  So a pair costs its warp's FP64
+// instructions, and a source costs each summing warp one more however few of
+// its lanes have a sink: the sums fill 30 of 32 lanes (10 sinks a summing
+// warp) where a warp per component would leave most of them empty, and the
+// squares of the displacement join the term multiplications on the integer
+// pipe: 11 FP64 instructions a pair instead of 14, beside ~430 integer ones
+// (333 before), which is where both pipes are about equally loaded.  (With
+// the product r^2 r moved there too the integer pipe leads: 1-3% slower.)  A
+// system of a few sinks per SM is bound by the sums' serial chain instead,
+// 64 cycles a source and ~80 measured, hence warps of their own for them
+// rather than a phase in which the producers wait.
+//
+// Measured (one evaluation, us; before: the two kernels this one replaces,
+// 4 sinks x 224 sources with 12 summing lanes, and 32 sinks alternating
+// between producing and summing): 300 bodies 37 -> 21, 1,033 94 -> 67, 2,049
+// 305 -> 168, 4,099 900 -> 565, 16,411 10,800 -> 7,970.
+constexpr int kRefTile = 64;      // sources per round
+constexpr int kRefPerWarp = 10;   // sinks per summing warp: 30 of its 32 lanes
+constexpr int kRefMaxSinks = 21;  // of the two-warp form: 63 of 64 lanes
+// at least this many sources per sink (fewer: one thread per sink is cheaper)
+constexpr int kRefMinSources = 224;
+constexpr int kMaxDevices = 64;
 
-__global__ void __launch_bounds__(256) k_gravity_ac_few(ForceCtx fc, const double* __restrict__ y,
-                                                        double* __restrict__ dydt, TimeSpec ts, uint32_t flags) {
-  // the nearest-neighbour candidates reuse the term tiles once the last one
-  // has been added
-  static_assert(sizeof(long long) * kFewSinks * kFewTile + sizeof(int) * kFewSinks * kFewTile <=
-                    sizeof(double) * 2 * kFewTile * kFewTerms,
-                "candidate arrays must fit in the term tiles");
-  __shared__ __align__(16) double terms[2][kFewTile][kFewTerms];
-  long long(*nn_r)[kFewTile] = reinterpret_cast<long long(*)[kFewTile]>(&terms[0][0][0]);
-  int(*nn_j)[kFewTile] = reinterpret_cast<int(*)[kFewTile]>(&terms[0][0][0] + kFewSinks * kFewTile);
-  __shared__ double sink_pos[kFewSinks][3];
-  __shared__ int sink_ns[kFewSinks];
-  __shared__ double acc[kFewTerms];
+constexpr size_t ref_smem(int sw, int spc) {
+  return sizeof(double) * (2 * 7 * kRefTile + 2 * (size_t)kRefTile * (32 * sw + 1)) +
+         (sizeof(long long) + sizeof(int)) * (size_t)kRefTile * spc;
+}
+
+// IEEE arithmetic for a pair the fast path hands over
+static __device__ __noinline__ double2 ref_pair_slow(double xij, double yij, double zij) {
+  double2 v;
+  sol_ref_rinv3_slow(xij * xij + yij * yij + zij * zij, v.x, v.y);
+  return v;
+}
+
+// rij and 1 / rij^3 of a displacement, the squares on the integer pipe (a z
+// that is zero for every pair, a planar system, stays on the fast path)
+__device__ __forceinline__ void ref_pair(double xij, double yij, double zij, bool valid, double& rij, double& rijm3) {
+  bool ok = true;
+  const double qx = sol_exact_dsqr<false>(xij, ok);
+  const double qy = sol_exact_dsqr<false>(yij, ok);
+  const double qz = sol_exact_dsqr<true>(zij, ok);
+  ok = ok & sol_ref_rinv3_fast(qx + qy + qz, rij, rijm3);
+  if (!ok & valid) {
+    const double2 v = ref_pair_slow(xij, yij, zij);
+    rij = v.x;
+    rijm3 = v.y;
+  }
+}
+
+// 32 warps per SM (64 registers): four CTAs of the one-warp form, two of the other
+template <int SW, int PW>
+__global__ void __launch_bounds__((SW + PW) * 32, 32 / (SW + PW))
+    k_gravity_ac_ref(ForceCtx fc, const double* __restrict__ y, double* __restrict__ dydt, TimeSpec ts, uint32_t flags,
+                     int spc) {
+  extern __shared__ __align__(16) double ref_dyn[];
+  __shared__ double sink_pos[kRefMaxSinks][3];
+  __shared__ int sink_ns[kRefMaxSinks];
+  __shared__ double acc[SW * 32];
+  __shared__ double nn_d[kRefMaxSinks];
+  __shared__ int nn_i[kRefMaxSinks];
+  constexpr int row = 32 * SW + 1;             // doubles per source row (odd: conflict-free columns)
+  double* srct = ref_dyn;                      // [2][7][kRefTile] source tiles
+  double* terms = srct + 2 * 7 * kRefTile;     // [2][kRefTile][row]
+  long long* nn_r = reinterpret_cast<long long*>(terms + 2 * kRefTile * row);  // [2 spc][32] nearest so far
+  int* nn_j = reinterpret_cast<int*>(nn_r + kRefTile * spc);
   const Classes& c = fc.cls;
   const int n = sol_sink_hi(fc);  // sinks [sink_lo, n)
-  const int i0 = fc.sink_lo + blockIdx.x * kFewSinks;
+  const int i0 = fc.sink_lo + blockIdx.x * spc;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x < kFewSinks) {
+  if (threadIdx.x < spc) {
     const int i = i0 + threadIdx.x;
     const bool live = i < n && i >= 1;
     sink_ns[threadIdx.x] = live ? ((fc.type[i] <= SOL_PROTO_PLANET) ? c.nm + c.n_spl : c.nm) : 0;
     for (int k = 0; k < 3; ++k) sink_pos[threadIdx.x][k] = i < n ? y[6 * i + k] : 0.0;
   }
-  __syncthreads();
-  int ns_cta = 0;
-  for (int s = 0; s < kFewSinks; ++s) ns_cta = max(ns_cta, sink_ns[s]);
-  const int rounds = (ns_cta + kFewTile - 1) / kFewTile;
+  for (int q = threadIdx.x; q < kRefTile * spc; q += blockDim.x) {
+    nn_r[q] = __double_as_longlong(1.0e10);
+    nn_j[q] = -1;
+  }
   const double* src = fc.src;
   const int np = fc.npad;
-
-  // producer state: the first minimum over this thread's columns, per sink
-  long long rminb[kFewSinks];
-  int nn[kFewSinks];
-  for (int s = 0; s < kFewSinks; ++s) {
-    rminb[s] = __double_as_longlong(1.0e10);
-    nn[s] = -1;
-  }
-  // accumulator state (warp 0, lanes < kFewTerms): lane = component * kFewSinks + sink
-  const int a_s = lane % kFewSinks;
-  const int a_i = i0 + a_s;
-  const int a_ns = (lane < kFewTerms) ? sink_ns[a_s] : 0;
+  constexpr int kLoads = (7 * kRefTile + PW * 32 - 1) / (PW * 32);
+  const int pt = (warp - SW) * 32 + lane;  // producing thread
+  if (warp >= SW)
+    for (int q = pt; q < 7 * kRefTile; q += PW * 32) srct[q] = src[(size_t)(q / kRefTile) * np + (q % kRefTile)];
+  __syncthreads();
+  int ns_cta = 0;
+  for (int s = 0; s < spc; ++s) ns_cta = max(ns_cta, sink_ns[s]);
+  const int rounds = (ns_cta + kRefTile - 1) / kRefTile;
   double a_sum = 0.0;
-
-  // round r: producers fill buffer r & 1 with sources [r * kFewTile, ...);
-  // warp 0 adds buffer (r - 1) & 1
+  // round r: the producers fill term tile r & 1 from source tile r & 1 and
+  // fetch the next sources; the summing warps add term tile (r - 1) & 1
   for (int r = 0; r <= rounds; ++r) {
-    if (warp > 0 && r < rounds) {
-      const int p = threadIdx.x - 32;
-      const int j = r * kFewTile + p;
-      if (j < ns_cta) {
-        const double xj = src[SX * np + j], yj = src[SY * np + j], zj = src[SZ * np + j];
-        const double gm = src[SGM * np + j], px = src[SPX * np + j], py = src[SPY * np + j],
-                     pz = src[SPZ * np + j];
-        double* out = &terms[r & 1][p][0];
-        // two sinks per step, branch-free up to the stores (their chains interleave)
+    if (warp >= SW) {
+      if (r < rounds) {
+        double pre[kLoads];
+        const bool more = r + 1 < rounds;
 #pragma unroll
-        for (int s = 0; s < kFewSinks; s += 2) {
-          double xij[2], yij[2], zij[2], rij2[2];
-          bool valid[2];
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            valid[u] = j >= 1 && j < sink_ns[s + u] && j != i0 + s + u;
-            xij[u] = xj - sink_pos[s + u][0];
-            yij[u] = yj - sink_pos[s + u][1];
-            zij[u] = zj - sink_pos[s + u][2];
-            const double q = xij[u] * xij[u] + yij[u] * yij[u] + zij[u] * zij[u];
-            rij2[u] = valid[u] ? q : 1.0;
-          }
-          double rij[2], rijm3[2];
-          sol_ref_rinv3_x2(rij2[0], rij2[1], rij[0], rijm3[0], rij[1], rijm3[1]);
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            double tx, ty, tz;
-            sol_ref_terms(gm, rijm3[u], xij[u], yij[u], zij[u], px, py, pz, tx, ty, tz);
-            if (valid[u]) {
-              const long long rb = __double_as_longlong(rij[u]);
-              if (rb < rminb[s + u]) {
-                rminb[s + u] = rb;
-                nn[s + u] = j;
-              }
-              out[0 * kFewSinks + s + u] = tx;
-              out[1 * kFewSinks + s + u] = ty;
-              out[2 * kFewSinks + s + u] = tz;
-            }
+        for (int u = 0; u < kLoads; ++u) {
+          const int q = pt + u * PW * 32;
+          pre[u] = (more && q < 7 * kRefTile)
+                       ? src[(size_t)(q / kRefTile) * np + (r + 1) * kRefTile + (q % kRefTile)]
+                       : 0.0;
+        }
+        const double* st = srct + (r & 1) * 7 * kRefTile;
+        double* out = terms + (size_t)(r & 1) * kRefTile * row;
+#pragma unroll 1
+        for (int item = warp - SW; item < 2 * spc; item += PW) {  // (sink, half of the tile)
+          const int s = item >> 1;
+          const int p = (item & 1) * 32 + lane;
+          const int j = r * kRefTile + p;
+          const bool valid = j >= 1 && j < sink_ns[s] && j != i0 + s;
+          const double xij = st[SX * kRefTile + p] - sink_pos[s][0];
+          const double yij = st[SY * kRefTile + p] - sink_pos[s][1];
+          const double zij = st[SZ * kRefTile + p] - sink_pos[s][2];
+          double rij, rijm3;
+          ref_pair(xij, yij, zij, valid, rij, rijm3);
+          double tx, ty, tz;
+          sol_ref_terms(st[SGM * kRefTile + p], rijm3, xij, yij, zij, st[SPX * kRefTile + p], st[SPY * kRefTile + p],
+                        st[SPZ * kRefTile + p], tx, ty, tz);
+          // a source the sink does not take adds +0, which changes no sum:
+          // a sum that starts at +0 is never -0
+          double* o = out + (size_t)p * row + 3 * s;
+          o[0] = tx;
+          o[1] = ty;
+          o[2] = tz;
+          if (!valid) o[0] = o[1] = o[2] = 0.0;
+          const long long rb = __double_as_longlong(rij);
+          if (valid && rb < nn_r[item * 32 + lane]) {
+            nn_r[item * 32 + lane] = rb;
+            nn_j[item * 32 + lane] = j;
           }
         }
+        double* nx = srct + ((r + 1) & 1) * 7 * kRefTile;
+#pragma unroll
+        for (int u = 0; u < kLoads; ++u) {
+          const int q = pt + u * PW * 32;
+          if (q < 7 * kRefTile) nx[q] = pre[u];
+        }
       }
-    } else if (warp == 0 && r > 0 && lane < kFewTerms) {
-      const int rr = r - 1;
-      const int j0 = rr * kFewTile;
-      const int pmax = min(kFewTile, a_ns - j0);
-      for (int p = 0; p < pmax; ++p) {
-        const int j = j0 + p;
-        if (j >= 1 && j != a_i) a_sum += terms[rr & 1][p][lane];
-      }
-    }
-    __syncthreads();
-  }
-  // nearest neighbour: the smallest distance, ties to the lowest index -- the
-  // reference's first strict minimum in ascending order
-  if (warp > 0) {
-    const int p = threadIdx.x - 32;
-    for (int s = 0; s < kFewSinks; ++s) {
-      nn_r[s][p] = rminb[s];
-      nn_j[s][p] = nn[s];
-    }
-  }
-  if (warp == 0 && lane < kFewTerms) acc[lane] = a_sum;
-  __syncthreads();
-  if (threadIdx.x >= kFewSinks) return;
-  const int s = threadIdx.x;
-  const int i = i0 + s;
-  if (i >= n) return;
-  double* out = dydt + 6 * i;
-  if (i == 0) {  // GravityAC :253-254, :266
-    for (int k = 0; k < 6; ++k) out[k] = 0.0;
-    fc.nn_idx[0] = -1;
-    fc.nn_dist[0] = 0.0;
-    return;
-  }
-  long long best = __double_as_longlong(1.0e10);
-  int bj = -1;
-  const int pmax = min(kFewTile, ns_cta);  // producers beyond the source count hold no candidate
-  for (int p = 0; p < pmax; ++p) {
-    const long long rb = nn_r[s][p];
-    const int jb = nn_j[s][p];
-    if (jb >= 0 && (rb < best || (rb == best && jb < bj))) {
-      best = rb;
-      bj = jb;
-    }
-  }
-  const double* yv = y + 6 * i;
-  const double xi = sink_pos[s][0], yi = sink_pos[s][1], zi = sink_pos[s][2];
-  const double mu = SOL_GAUSS2 * (fc.mass[0] + fc.mass[i]);
-  const double rm3i = fc.rm3[i];
-  double a[3];
-  a[0] = -mu * rm3i * xi;  // Kepler term first (:281-283)
-  a[1] = -mu * rm3i * yi;
-  a[2] = -mu * rm3i * zi;
-  a[0] += acc[0 * kFewSinks + s];
-  a[1] += acc[1 * kFewSinks + s];
-  a[2] += acc[2 * kFewSinks + s];
-  fc.nn_idx[i] = bj;
-  fc.nn_dist[i] = bj >= 0 ? __longlong_as_double(best) : 0.0;
-  add_gas_terms(fc, i, yv, eval_time(ts), flags, a);
-  out[0] = yv[3];
-  out[1] = yv[4];
-  out[2] = yv[5];
-  out[3] = a[0];
-  out[4] = a[1];
-  out[5] = a[2];
-}
-
-// ---- FP64 GravityAC, 32 sinks per CTA ----------------------------------------
-// The FP64 pipe spends 64 cycles on every warp instruction however many of
-// its lanes are active, so the in-order sums of k_gravity_ac_few (12 of 32
-// lanes) cost almost a third of its pair work.  Here a CTA takes up to 32
-// sinks and alternates two phases per round of kWideTile sources:
-//  A. every thread computes one source's terms against a quarter of the
-//     sinks (the reference arithmetic, Acceleration.cpp:294-317) into a
-//     shared row; the nearest-neighbour candidates of each sink are reduced
-//     across the warp with three 32-bit minimum reductions (high word, low
-//     word, index) and kept by one lane of the warp;
-//  B. three full warps -- warp c for component c, lane s for sink s -- add the
-//     round's terms in ascending source order.
-// The sums are the reference's sequential sums (bit-identical to
-// k_gravity_ac_few); a sum costs 3 FP64 warp instructions per round.  A CTA
-// takes spc <= 32 sinks: the host picks spc so that the CTAs fill whole
-// waves of three per SM (the per-round cost 14/32 spc + 3 FP64 warp
-// instructions per source, times the waves, is smallest).  A 64-source tile
-// (49.7 KB) and 85 registers give three CTAs, 24 warps, per SM: measured at
-// 65,536 bodies 151 ms, against 157 ms with four CTAs per SM (64 registers,
-// spilling) and 169 ms with a 128-source tile and two.
-constexpr int kWideSinks = 32;
-constexpr int kWideWarps = 8;
-constexpr int kWideCtasPerSm = 3;                      // 24 warps per SM: six per sub-partition
-constexpr int kWideTile = 64;                          // sources per round
-constexpr int kWideGroups = kWideWarps * 32 / kWideTile;  // sink quarters: thread = (quarter, source)
-constexpr int kWideRow = 3 * kWideSinks + 1;           // doubles per source row (odd: conflict-free columns)
-constexpr size_t kWideSmem = sizeof(double) * kWideTile * kWideRow;  // 49,664 bytes
-constexpr int kMaxDevices = 64;
-// below this many sinks per CTA the 4-sink kernel's finer grid wins (measured)
-constexpr int kWideMinSinks = 6;
-
-// Phase A of k_gravity_ac_wide for sink s: the pair term into the shared
-// row, the warp's nearest-neighbour candidate.
-__device__ __forceinline__ void wide_sink(int s, int s0, int j, bool jin, int i0, int lane, double xj, double yj,
-                                          double zj, double gm, double px, double py, double pz,
-                                          const double (*sink_pos)[3], const int* sink_ns, double* row,
-                                          unsigned long long& best, int& best_j) {
-  const bool valid = jin && j >= 1 && j < sink_ns[s] && j != i0 + s;
-  const double xij = xj - sink_pos[s][0];
-  const double yij = yj - sink_pos[s][1];
-  const double zij = zj - sink_pos[s][2];
-  const double q = xij * xij + yij * yij + zij * zij;
-  double rij, rijm3;
-  sol_ref_rinv3(valid ? q : 1.0, rij, rijm3);
-  double tx, ty, tz;
-  sol_ref_terms(gm, rijm3, xij, yij, zij, px, py, pz, tx, ty, tz);
-  if (valid) {
-    row[0 * kWideSinks + s] = tx;
-    row[1 * kWideSinks + s] = ty;
-    row[2 * kWideSinks + s] = tz;
-  }
-  // the warp's smallest (rij, j): high word, then low word, then index
-  const unsigned long long key = valid ? (unsigned long long)__double_as_longlong(rij) : ~0ull;
-  const unsigned hi = (unsigned)(key >> 32);
-  const unsigned mhi = __reduce_min_sync(0xFFFFFFFFu, hi);
-  const unsigned lo = (hi == mhi) ? (unsigned)key : 0xFFFFFFFFu;
-  const unsigned mlo = __reduce_min_sync(0xFFFFFFFFu, lo);
-  const unsigned jj = (hi == mhi && (unsigned)key == mlo) ? (unsigned)j : 0xFFFFFFFFu;
-  const unsigned mj = __reduce_min_sync(0xFFFFFFFFu, jj);
-  const unsigned long long mkey = ((unsigned long long)mhi << 32) | mlo;
-  if (lane == s - s0 && mkey < best) {  // later rounds hold larger indices: ties keep the earlier
-    best = mkey;
-    best_j = (int)mj;
-  }
-}
-
-__global__ void __launch_bounds__(kWideWarps * 32, kWideCtasPerSm) k_gravity_ac_wide(ForceCtx fc, const double* __restrict__ y,
-                                                                        double* __restrict__ dydt, TimeSpec ts,
-                                                                        uint32_t flags, int spc) {
-  extern __shared__ __align__(16) double wide_terms[];  // [kWideTile][kWideRow]
-  __shared__ double sink_pos[kWideSinks][3];
-  __shared__ int sink_ns[kWideSinks];
-  __shared__ double acc[3][kWideSinks];
-  __shared__ unsigned long long nn_key[kWideWarps][kWideSinks];
-  __shared__ int nn_j[kWideWarps][kWideSinks];
-  const Classes& c = fc.cls;
-  const int n = sol_sink_hi(fc);  // sinks [sink_lo, n)
-  const int i0 = fc.sink_lo + blockIdx.x * spc;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x < kWideSinks) {
-    const int i = i0 + threadIdx.x;
-    const bool live = i < n && i >= 1 && threadIdx.x < spc;
-    sink_ns[threadIdx.x] = live ? ((fc.type[i] <= SOL_PROTO_PLANET) ? c.nm + c.n_spl : c.nm) : 0;
-    for (int k = 0; k < 3; ++k) sink_pos[threadIdx.x][k] = i < n ? y[6 * i + k] : 0.0;
-  }
-  __syncthreads();
-  int ns_cta = 0;
-  for (int s = 0; s < kWideSinks; ++s) ns_cta = max(ns_cta, sink_ns[s]);
-  const int rounds = (ns_cta + kWideTile - 1) / kWideTile;
-  const double* src = fc.src;
-  const int np = fc.npad;
-
-  // lane s of every warp: the first minimum of sink g ceil(spc/4) + s
-  // (g = warp / 2, its quarter of the sinks) over this warp's sources
-  unsigned long long best = (unsigned long long)__double_as_longlong(1.0e10);
-  int best_j = -1;
-  // phase-B lanes: component warp, sink lane
-  const int b_i = i0 + lane;
-  const int b_ns = sink_ns[lane];
-  double a_sum = 0.0;
-
-  for (int r = 0; r < rounds; ++r) {
-    // ---- phase A ----
-    {
-      const int p = threadIdx.x % kWideTile;
-      const int quarter = (spc + kWideGroups - 1) / kWideGroups;
-      const int s0 = (threadIdx.x / kWideTile) * quarter;
-      const int s1 = min(s0 + quarter, spc);
-      const int j = r * kWideTile + p;
-      const bool jin = j < ns_cta;
-      double xj = 0, yj = 0, zj = 0, gm = 0, px = 0, py = 0, pz = 0;
-      if (jin) {
-        xj = src[SX * np + j];
-        yj = src[SY * np + j];
-        zj = src[SZ * np + j];
-        gm = src[SGM * np + j];
-        px = src[SPX * np + j];
-        py = src[SPY * np + j];
-        pz = src[SPZ * np + j];
-      }
-      double* row = wide_terms + (size_t)p * kWideRow;
-      for (int s = s0; s < s1; ++s)
-        wide_sink(s, s0, j, jin, i0, lane, xj, yj, zj, gm, px, py, pz, sink_pos, sink_ns, row, best, best_j);
-    }
-    __syncthreads();
-    // ---- phase B ----
-    if (warp < 3) {
-      const int j0 = r * kWideTile;
-      const int pmax = min(kWideTile, b_ns - j0);
-      const double* col = wide_terms + warp * kWideSinks + lane;
-      for (int p = 0; p < pmax; ++p) {
-        const int j = j0 + p;
-        if (j >= 1 && j != b_i) a_sum += col[(size_t)p * kWideRow];
+    } else if (r > 0) {
+      const int L = warp * 32 + lane;  // 3 sink + component
+      if (L < 3 * spc) {
+        const double* col = terms + (size_t)((r - 1) & 1) * kRefTile * row + L;
+#pragma unroll
+        for (int p = 0; p < kRefTile; ++p) a_sum += col[p * row];
       }
     }
     __syncthreads();
   }
-  nn_key[warp][lane] = best;
-  nn_j[warp][lane] = best_j;
-  if (warp < 3) acc[warp][lane] = a_sum;
+  if (warp < SW) acc[warp * 32 + lane] = a_sum;
+  // nearest neighbour of a sink: the smallest distance over its 64 columns,
+  // ties to the lowest index (each column keeps its first minimum)
+  for (int s = warp; s < spc; s += SW + PW) {
+    long long b = nn_r[(2 * s) * 32 + lane];
+    int bj = nn_j[(2 * s) * 32 + lane];
+    const long long b2 = nn_r[(2 * s + 1) * 32 + lane];
+    const int j2 = nn_j[(2 * s + 1) * 32 + lane];
+    if (b2 < b || (b2 == b && (unsigned)j2 < (unsigned)bj)) {
+      b = b2;
+      bj = j2;
+    }
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) {
+      const long long ob = __shfl_xor_sync(0xFFFFFFFFu, b, w);
+      const int oj = __shfl_xor_sync(0xFFFFFFFFu, bj, w);
+      if (ob < b || (ob == b && (unsigned)oj < (unsigned)bj)) {
+        b = ob;
+        bj = oj;
+      }
+    }
+    if (lane == 0) {
+      nn_d[s] = bj >= 0 ? __longlong_as_double(b) : 0.0;
+      nn_i[s] = bj;
+    }
+  }
   __syncthreads();
   if (threadIdx.x >= spc) return;
   const int s = threadIdx.x;
@@ -726,20 +604,6 @@ __global__ void __launch_bounds__(kWideWarps * 32, kWideCtasPerSm) k_gravity_ac_
     fc.nn_dist[0] = 0.0;
     return;
   }
-  constexpr int kWarpsPerGroup = kWideTile / 32;
-  const int quarter = (spc + kWideGroups - 1) / kWideGroups;
-  const int w0 = (s / quarter) * kWarpsPerGroup;
-  const int hl = s % quarter;
-  unsigned long long bk = nn_key[w0][hl];
-  int bj = nn_j[w0][hl];
-  for (int w = w0 + 1; w < w0 + kWarpsPerGroup; ++w) {
-    const unsigned long long k2 = nn_key[w][hl];
-    const int j2 = nn_j[w][hl];
-    if (j2 >= 0 && (bj < 0 || k2 < bk || (k2 == bk && j2 < bj))) {
-      bk = k2;
-      bj = j2;
-    }
-  }
   const double* yv = y + 6 * i;
   const double xi = sink_pos[s][0], yi = sink_pos[s][1], zi = sink_pos[s][2];
   const double mu = SOL_GAUSS2 * (fc.mass[0] + fc.mass[i]);
@@ -748,11 +612,11 @@ __global__ void __launch_bounds__(kWideWarps * 32, kWideCtasPerSm) k_gravity_ac_
   a[0] = -mu * rm3i * xi;  // Kepler term first (:281-283)
   a[1] = -mu * rm3i * yi;
   a[2] = -mu * rm3i * zi;
-  a[0] += acc[0][s];
-  a[1] += acc[1][s];
-  a[2] += acc[2][s];
-  fc.nn_idx[i] = bj;
-  fc.nn_dist[i] = bj >= 0 ? __longlong_as_double((long long)bk) : 0.0;
+  a[0] += acc[3 * s + 0];
+  a[1] += acc[3 * s + 1];
+  a[2] += acc[3 * s + 2];
+  fc.nn_idx[i] = nn_i[s];
+  fc.nn_dist[i] = nn_d[s];
   add_gas_terms(fc, i, yv, eval_time(ts), flags, a);
   out[0] = yv[3];
   out[1] = yv[4];
@@ -1461,6 +1325,59 @@ static int split_chunk(const sol_ctx* c, int precision) {
   return best_ct * kTile;
 }
 
+// Sinks per CTA and summing warps of k_gravity_ac_ref: the CTAs spread over
+// the SMs, so an SM's work is its CTAs (the busiest SM's, k) times what one
+// costs a source: spc sinks' pairs and the summing warps', which cost about
+// 1.9 sinks each (16 cycles of the FP64 pipe against ~9 a sink).  For each k
+// the fewest sinks that reach it; the cheapest of one summing warp (up to
+// kRefPerWarp sinks) and two.  Measured at 4,099 bodies (us): 9 sinks 575, 7
+// sinks 564, 14 sinks with two summing warps 569; at 16,411 18 with two 7,970.
+static void ref_shape(int nsink, int nsm, int& spc, int& sw) {
+  double best = 1e300;
+  spc = 1;
+  sw = 1;
+  for (int w = 1; w <= 2; ++w) {
+    const int most = w == 1 ? kRefPerWarp : kRefMaxSinks;
+    const long k0 = ((long)nsink + (long)nsm * most - 1) / ((long)nsm * most);
+    for (long k = k0; k < k0 + 3; ++k) {
+      const int sp = (int)(((long)nsink + k * nsm - 1) / (k * nsm));
+      const double cost = (double)k * (sp + 1.9 * w);
+      if (cost < best) {
+        best = cost;
+        spc = sp;
+        sw = w;
+      }
+    }
+  }
+}
+
+static int launch_ref(sol_ctx* c, const ForceCtx& fc, const double* d_y, double* d_dydt, TimeSpec ts, uint32_t flags,
+                      int nsink) {
+  // per device: the SM count, once the kernels' shared-memory sizes are
+  // allowed (contexts of several host threads may race to set it: the same
+  // values, hence an atomic published after the attribute calls)
+  static std::atomic<int> ref_sms[kMaxDevices];
+  const int dev = (c->device >= 0 && c->device < kMaxDevices) ? c->device : 0;
+  int nsm = ref_sms[dev].load(std::memory_order_acquire);
+  if (nsm == 0) {
+    SOL_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
+    SOL_CUDA(cudaFuncSetAttribute(k_gravity_ac_ref<1, 7>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)ref_smem(1, kRefPerWarp)));
+    SOL_CUDA(cudaFuncSetAttribute(k_gravity_ac_ref<2, 14>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)ref_smem(2, kRefMaxSinks)));
+    ref_sms[dev].store(nsm, std::memory_order_release);
+  }
+  int spc, sw;
+  ref_shape(nsink, nsm, spc, sw);
+  const int grid = (nsink + spc - 1) / spc;
+  if (sw == 1)
+    k_gravity_ac_ref<1, 7><<<grid, 8 * 32, ref_smem(1, spc), c->stream>>>(fc, d_y, d_dydt, ts, flags, spc);
+  else
+    k_gravity_ac_ref<2, 14><<<grid, 16 * 32, ref_smem(2, spc), c->stream>>>(fc, d_y, d_dydt, ts, flags, spc);
+  SOL_LAUNCHED();
+  return SOL_OK;
+}
+
 // The sinks of fc's range [sink_lo, sol_sink_hi) (every body by default);
 // the prepass always covers every body (the sources).
 static int force_launch(sol_ctx* c, const ForceCtx& fc, const double* d_y, double* d_dydt, TimeSpec ts,
@@ -1489,47 +1406,7 @@ static int force_launch(sol_ctx* c, const ForceCtx& fc, const double* d_y, doubl
     SOL_LAUNCHED();
     return SOL_OK;
   }
-  // sinks with fewer sources than one producer tile (a few massive bodies and
-  // many light ones) are cheaper with one thread per sink
-  if (!split && c->cls.nm + c->cls.n_spl >= kFewTile) {
-    // per device: the SM count, once the wide kernel's shared-memory size is
-    // allowed (contexts of several host threads may race to set it: the same
-    // values, hence an atomic published after the attribute call)
-    static std::atomic<int> wide_sms[kMaxDevices];
-    const int dev = (c->device >= 0 && c->device < kMaxDevices) ? c->device : 0;
-    int wsm = wide_sms[dev].load(std::memory_order_acquire);
-    if (wsm == 0) {
-      int nsm = 0;
-      SOL_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
-      SOL_CUDA(cudaFuncSetAttribute(k_gravity_ac_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWideSmem));
-      wide_sms[dev].store(nsm, std::memory_order_release);
-      wsm = nsm;
-    }
-    // sinks per CTA: the fewest whole waves of two CTAs per SM, then the
-    // cheapest of that and the next two wave counts
-    const int slots = kWideCtasPerSm * wsm;
-    int spc = 0;
-    {
-      const int k0 = (nsink + slots * kWideSinks - 1) / (slots * kWideSinks);
-      double best = 1e300;
-      for (int k = k0; k < k0 + 3; ++k) {
-        const int sp = (nsink + k * slots - 1) / (k * slots);
-        const double cost = k * (0.4375 * sp + 3.0);
-        if (cost < best) {
-          best = cost;
-          spc = sp;
-        }
-      }
-    }
-    if (spc >= kWideMinSinks) {
-      k_gravity_ac_wide<<<(nsink + spc - 1) / spc, kWideWarps * 32, kWideSmem, c->stream>>>(fc, d_y, d_dydt, ts,
-                                                                                            flags, spc);
-    } else {
-      k_gravity_ac_few<<<(nsink + kFewSinks - 1) / kFewSinks, 256, 0, c->stream>>>(fc, d_y, d_dydt, ts, flags);
-    }
-    SOL_LAUNCHED();
-    return SOL_OK;
-  }
+  if (!split && c->cls.nm + c->cls.n_spl >= kRefMinSources) return launch_ref(c, fc, d_y, d_dydt, ts, flags, nsink);
   if (split && !sol_force_uses_chunk_partials(c, c->precision)) {
     const int grid = (nsink + kFewSplitWarps - 1) / kFewSplitWarps;
     if (c->precision == SOL_PRECISION_SPLIT_FF)
