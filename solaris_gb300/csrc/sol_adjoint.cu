@@ -17,14 +17,16 @@
 #include <cstring>
 #include <vector>
 
-#include "sol_internal.cuh"
+#include "sol_pair.cuh"
 
 int sol_rkf78_stages(sol_ctx* c, const double* d_y0, double* d_y, double* const* stage_out);
 
 namespace {
 
 constexpr int kBlock = 256;
-constexpr int kWarpsPerBlock = 8;
+constexpr int kVjpThreads = 128;  // threads of k_vjp: one body's pairs
+constexpr int kVjpWarps = kVjpThreads / 32;
+constexpr int kPreBodies = 42;    // bodies per CTA of k_vjp_cotangent: 252 elements
 constexpr int kAdjStages = 11;  // stages 0..10 reach y_{n+1}
 
 // RKF78 tableau (RungeKuttaFehlberg78.cpp:41-56): a[j][k] and the weights b
@@ -62,18 +64,84 @@ __global__ void k_lincomb(int nv, double* __restrict__ out, const double* __rest
   }
 }
 
-// Structure-of-arrays view of (state, cotangent) for the VJP: x, y, z, m, wx, wy, wz
-__global__ void k_vjp_prepass(int n, const double* __restrict__ Y, const double* __restrict__ w,
-                              const double* __restrict__ mass, double* __restrict__ soa) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  soa[0 * n + i] = Y[6 * i];
-  soa[1 * n + i] = Y[6 * i + 1];
-  soa[2 * n + i] = Y[6 * i + 2];
-  soa[3 * n + i] = mass[i];
-  soa[4 * n + i] = w[6 * i + 3];
-  soa[5 * n + i] = w[6 * i + 4];
-  soa[6 * n + i] = w[6 * i + 5];
+// The stage's cotangent w = h b_k lambda + h sum_j a_jk nu_j (L, scaled by h),
+// the structure-of-arrays view of (state, cotangent) that k_vjp streams -- x,
+// y, z, m, wx, wy, wz -- and this CTA's sums of the cotangent's velocity part
+// over its bodies: [0..2] those with index >= 1, [3..5] those below nm.  One
+// thread per element, kPreBodies bodies per CTA.
+__global__ void __launch_bounds__(6 * kPreBodies) k_vjp_cotangent(int n, int nm, const double* __restrict__ Y,
+                                                                  const double* __restrict__ mass, double h, Lin L,
+                                                                  double* __restrict__ w, double* __restrict__ soa,
+                                                                  double* __restrict__ wsum) {
+  __shared__ double sw[6 * kPreBodies];
+  const int i0 = blockIdx.x * kPreBodies;
+  const int b = threadIdx.x / 6, k = threadIdx.x - 6 * b;
+  const int i = i0 + b;
+  double acc = 0.0;
+  if (i < n) {
+    const size_t e = 6 * (size_t)i + k;
+    for (int q = 0; q < L.k; ++q) acc = __fma_rn(L.c[q], L.v[q][e], acc);
+    acc = h * acc;
+    w[e] = acc;
+    if (k < 3) {
+      soa[(size_t)k * n + i] = Y[e];
+      if (k == 0) soa[(size_t)3 * n + i] = mass[i];
+    } else {
+      soa[(size_t)(k + 1) * n + i] = acc;
+    }
+  }
+  sw[threadIdx.x] = acc;
+  __syncthreads();
+  if (threadIdx.x < 6) {
+    const int c = 3 + threadIdx.x % 3;
+    const int hi = min(i0 + kPreBodies, threadIdx.x < 3 ? n : nm);
+    double t = 0.0;
+    for (int j = max(i0, 1); j < hi; ++j) t += sw[6 * (j - i0) + c];
+    wsum[6 * (size_t)blockIdx.x + threadIdx.x] = t;
+  }
+}
+
+// r^-3 and r^-2 of r^2: the FP32 seed y of 1/r, its square (exact) and cube
+// from the integer pipe, and one FP64 residual e = 1 - r^2 y^2 (|e| < 2^-20):
+// r^-3 = y^3 (1 + 3/2 e + 15/8 e^2), r^-2 = y^2 (1 + e + e^2), both within
+// about an ulp, for four FP64 instructions.  r^2 outside [2^-100, 2^100]
+// (coincident bodies, infinities, NaN) takes rsqrt.
+static __device__ __noinline__ double2 rinv32_slow(double r2) {
+  const double r = rsqrt(r2);
+  return make_double2(r * r * r, r * r);
+}
+__device__ __forceinline__ void rinv32(double r2, double& rm3, double& rm2) {
+  double u, y3;
+  sol_seed_square_cube(sol_rsqrt_seed(r2), u, y3);
+  const double e = __fma_rn(-r2, u, 1.0);
+  rm3 = __fma_rn(y3, sol_split_t(e), y3);
+  rm2 = __fma_rn(u, __fma_rn(e, e, e), u);
+  const unsigned ex = ((unsigned)__double2hiint(r2)) >> 20;
+  if (ex - 923u >= 200u) {
+    const double2 v = rinv32_slow(r2);
+    rm3 = v.x;
+    rm2 = v.y;
+  }
+}
+
+// Eight sums over the warp in 9 additions a lane (40 for eight shuffle
+// trees): at the first three steps a lane hands half of its sums to its
+// partner and takes the other half.  Lane l ends with sum
+// 4 (l >> 4 & 1) + 2 (l >> 3 & 1) + (l >> 2 & 1).
+__device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
+#pragma unroll
+  for (int half = 4, off = 16; half >= 1; half >>= 1, off >>= 1) {
+    const bool up = (lane & off) != 0;
+#pragma unroll
+    for (int q = 0; q < half; ++q) {
+      const double send = up ? v[q] : v[q + half];
+      const double keep = up ? v[q + half] : v[q];
+      v[q] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    }
+  }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+  return v[0];
 }
 
 __device__ __forceinline__ void tensor_apply(double dx, double dy, double dz, double rm3, double rm5, double vx,
@@ -86,102 +154,114 @@ __device__ __forceinline__ void tensor_apply(double dx, double dy, double dz, do
   oz = __fma_rn(vz, rm3, -s * dz);
 }
 
-// nu = J(Y)^T w for the heliocentric gravity with Kepler and indirect terms.
-// One warp per body k; lanes split the other bodies j and the warp sums in a
-// fixed shuffle order.  Also dm[k] += w . d(dydt)/d m_k, and the per-body
-// terms of d/d m_0 into m0_part[k].
-__global__ void k_vjp(int n, int nm, int nspl, const double* __restrict__ soa, const double* __restrict__ w,
-                      double* __restrict__ nu, double* __restrict__ dm, double* __restrict__ m0_part) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const int k = warp;
-  if (k >= n) return;
-  const double* X = soa;
-  const double* Yy = soa + n;
-  const double* Z = soa + 2 * n;
-  const double* M = soa + 3 * n;
-  const double* WX = soa + 4 * n;
-  const double* WY = soa + 5 * n;
-  const double* WZ = soa + 6 * n;
+// nu = J(Y)^T w for the heliocentric gravity with Kepler and indirect terms:
+// one CTA per body k, its threads split the other bodies j and the CTA sums
+// in a fixed order.  Also dm[k] += w . d(dydt)/d m_k, and the per-body terms
+// of d/d m_0 into m0_part[k] (added over the calls; summed once at the end).
+//
+// With d = r_j - r_k, v = [k source of j] m_k w_j - [j source of k] m_j w_k,
+// the pair adds T(d) v = v / r^3 - 3 d (d . v) / r^5 to the gradient.  m_k and
+// w_k are the CTA's own, so the first part is m_k sum w_j / r^3 -
+// w_k sum m_j / r^3 (four FMAs), and d . v = m_k (d . w_j) - m_j (d . w_k)
+// shares d . w_j with the mass gradient.  The sum of w_j over the sinks of k,
+// which the indirect term wants, is k_vjp_cotangent's total less k's own.
+//
+// FP64 pipe: 28 FP64 instructions a pair (about 55 with rsqrt, v and T(d) v
+// by component), 16 cycles of the SM's pipe each: 55 us at 1,033 bodies with the sums; a
+// body per CTA of four warps rather than per warp spreads 1,033 bodies evenly
+// over the SMs (7 CTAs each) and keeps 28 warps in flight.  Measured at 1,033
+// bodies: 72 us a product (76% of the pipe), from 116 (and three more launches, one now).
+__global__ void __launch_bounds__(kVjpThreads) k_vjp(int n, int nm, int nspl, const double* __restrict__ soa,
+                                                     const double* __restrict__ wsum, int nwsum,
+                                                     const double* __restrict__ w, double* __restrict__ nu,
+                                                     double* __restrict__ dm, double* __restrict__ m0_part) {
+  __shared__ double red[kVjpWarps][8];
+  __shared__ double tot[8];
+  __shared__ double W[3];
+  const int k = blockIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (k == 0) {  // the central body's state is fixed: its dydt is 0 (Acceleration.cpp:266)
-    if (lane < 6) nu[lane] = 0.0;
-    if (lane == 0) m0_part[0] = 0.0;
+    if (threadIdx.x < 6) nu[threadIdx.x] = 0.0;
     return;
   }
+  const double* X = soa;
+  const double* Yy = soa + n;
+  const double* Z = soa + 2 * (size_t)n;
+  const double* M = soa + 3 * (size_t)n;
+  const double* WX = soa + 4 * (size_t)n;
+  const double* WY = soa + 5 * (size_t)n;
+  const double* WZ = soa + 6 * (size_t)n;
   const double xk = X[k], yk = Yy[k], zk = Z[k], mk = M[k];
   const double wkx = WX[k], wky = WY[k], wkz = WZ[k];
-  const int ns_k = k < nm ? nm + nspl : nm;
-  const bool k_is_source = k < nm + nspl;  // source of some sink
-  const double G = SOL_GAUSS2;
-  double gx = 0, gy = 0, gz = 0;     // J_r^T w from pair terms
-  double Wx = 0, Wy = 0, Wz = 0;     // sum of w_v over the sinks that have k as a source
-  double dmk = 0;                    // pair part of dL/dm_k
-  for (int j = 1 + lane; j < n; j += 32) {
-    if (j == k) continue;
-    const int ns_j = j < nm ? nm + nspl : nm;
-    const bool k_src_of_j = k < ns_j;
-    const bool j_src_of_k = j < ns_k;
-    if (!k_src_of_j && !j_src_of_k) continue;
+  const int ns_k = k < nm ? nm + nspl : nm;   // sources of k: j < ns_k
+  // k is a source of the sinks j < jk: every body (k massive), the massive
+  // ones (k a super-planetesimal) or none
+  const int jk = k < nm ? n : (k < nm + nspl ? nm : 0);
+  const int jmax = max(jk, ns_k);
+  if (warp < 3) {  // component `warp` of the sum of w_v over the sinks of k
+    double t = 0.0;
+    if (jk > 0)
+      for (int b = lane; b < nwsum; b += 32) t += wsum[6 * (size_t)b + (k < nm ? warp : 3 + warp)];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) W[warp] = k < nm ? t - (warp == 0 ? wkx : (warp == 1 ? wky : wkz)) : t;
+  }
+  double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // sum w_j / r^3 (3), m_j / r^3, d (d . v) / r^5 (3), -(d . w_j) / r^3
+  for (int j = 1 + threadIdx.x; j < jmax; j += kVjpThreads) {
     const double dx = X[j] - xk, dy = Yy[j] - yk, dz = Z[j] - zk;  // r_j - r_k
+    const bool sink = j < jk, source = j < ns_k;
+    const double wjx = sink ? WX[j] : 0.0, wjy = sink ? WY[j] : 0.0, wjz = sink ? WZ[j] : 0.0;
+    const double mj = source ? M[j] : 0.0;
+    if (j == k) continue;
     const double r2 = __fma_rn(dx, dx, __fma_rn(dy, dy, dz * dz));
-    const double rinv = rsqrt(r2);
-    const double rm3 = rinv * rinv * rinv;
-    const double rm5 = rm3 * rinv * rinv;
-    const double wjx = WX[j], wjy = WY[j], wjz = WZ[j];
-    // v = [k source of j] m_k w_j - [j source of k] m_j w_k
-    double vx = 0, vy = 0, vz = 0;
-    if (k_src_of_j) {
-      vx = mk * wjx;
-      vy = mk * wjy;
-      vz = mk * wjz;
-      Wx += wjx;
-      Wy += wjy;
-      Wz += wjz;
-      // d a_j / d m_k = G (r_k - r_j) / |r_k - r_j|^3 (direct part)
-      dmk -= rm3 * __fma_rn(dx, wjx, __fma_rn(dy, wjy, dz * wjz));
-    }
-    if (j_src_of_k) {
-      const double mj = M[j];
-      vx = __fma_rn(-mj, wkx, vx);
-      vy = __fma_rn(-mj, wky, vy);
-      vz = __fma_rn(-mj, wkz, vz);
-    }
-    double tx, ty, tz;
-    tensor_apply(dx, dy, dz, rm3, rm5, vx, vy, vz, tx, ty, tz);
-    gx += tx;
-    gy += ty;
-    gz += tz;
+    double rm3, rm2;
+    rinv32(r2, rm3, rm2);
+    const double p = __fma_rn(dx, wjx, __fma_rn(dy, wjy, dz * wjz));
+    const double q = __fma_rn(dx, wkx, __fma_rn(dy, wky, dz * wkz));
+    // d a_j / d m_k = G (r_k - r_j) / |r_k - r_j|^3 (direct part)
+    v[7] = __fma_rn(-rm3, p, v[7]);
+    const double s = (__fma_rn(mk, p, -mj * q) * rm2) * rm3;
+    v[0] = __fma_rn(rm3, wjx, v[0]);
+    v[1] = __fma_rn(rm3, wjy, v[1]);
+    v[2] = __fma_rn(rm3, wjz, v[2]);
+    v[3] = __fma_rn(rm3, mj, v[3]);
+    v[4] = __fma_rn(s, dx, v[4]);
+    v[5] = __fma_rn(s, dy, v[5]);
+    v[6] = __fma_rn(s, dz, v[6]);
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    gx += __shfl_down_sync(0xffffffffu, gx, o);
-    gy += __shfl_down_sync(0xffffffffu, gy, o);
-    gz += __shfl_down_sync(0xffffffffu, gz, o);
-    Wx += __shfl_down_sync(0xffffffffu, Wx, o);
-    Wy += __shfl_down_sync(0xffffffffu, Wy, o);
-    Wz += __shfl_down_sync(0xffffffffu, Wz, o);
-    dmk += __shfl_down_sync(0xffffffffu, dmk, o);
+  const double mine = warp_sum8(v, lane);
+  if ((lane & 3) == 0) red[warp][4 * (lane >> 4 & 1) + 2 * (lane >> 3 & 1) + (lane >> 2 & 1)] = mine;
+  __syncthreads();
+  if (threadIdx.x < 8) {
+    double t = red[0][threadIdx.x];
+    for (int u = 1; u < kVjpWarps; ++u) t += red[u][threadIdx.x];
+    tot[threadIdx.x] = t;
   }
-  if (lane != 0) return;
+  __syncwarp();
+  if (threadIdx.x != 0) return;
+  const double G = SOL_GAUSS2;
+  const double gx = __fma_rn(mk, tot[0], __fma_rn(-wkx, tot[3], -3.0 * tot[4]));
+  const double gy = __fma_rn(mk, tot[1], __fma_rn(-wky, tot[3], -3.0 * tot[5]));
+  const double gz = __fma_rn(mk, tot[2], __fma_rn(-wkz, tot[3], -3.0 * tot[6]));
   // Kepler term -G (m0 + m_k) r_k / |r_k|^3 and indirect term -G m_k r_k / |r_k|^3 (for the sinks of k)
   const double r2 = __fma_rn(xk, xk, __fma_rn(yk, yk, zk * zk));
-  const double rinv = rsqrt(r2);
-  const double rm3 = rinv * rinv * rinv;
-  const double rm5 = rm3 * rinv * rinv;
-  const double m0 = M[0];
+  double rm3, rm2;
+  rinv32(r2, rm3, rm2);
+  const double mu = -(M[0] + mk);
+  const double Wx = W[0], Wy = W[1], Wz = W[2];  // 0 when k is no source
   double kx, ky, kz;
-  tensor_apply(xk, yk, zk, rm3, rm5, -(m0 + mk) * wkx - (k_is_source ? mk * Wx : 0.0),
-               -(m0 + mk) * wky - (k_is_source ? mk * Wy : 0.0), -(m0 + mk) * wkz - (k_is_source ? mk * Wz : 0.0),
-               kx, ky, kz);
-  nu[6 * k + 0] = G * (gx + kx);
-  nu[6 * k + 1] = G * (gy + ky);
-  nu[6 * k + 2] = G * (gz + kz);
-  nu[6 * k + 3] = w[6 * k + 0];  // d(position)/dt = velocity
-  nu[6 * k + 4] = w[6 * k + 1];
-  nu[6 * k + 5] = w[6 * k + 2];
+  tensor_apply(xk, yk, zk, rm3, rm3 * rm2, __fma_rn(mu, wkx, -mk * Wx), __fma_rn(mu, wky, -mk * Wy),
+               __fma_rn(mu, wkz, -mk * Wz), kx, ky, kz);
+  nu[6 * (size_t)k + 0] = G * (gx + kx);
+  nu[6 * (size_t)k + 1] = G * (gy + ky);
+  nu[6 * (size_t)k + 2] = G * (gz + kz);
+  nu[6 * (size_t)k + 3] = w[6 * (size_t)k + 0];  // d(position)/dt = velocity
+  nu[6 * (size_t)k + 4] = w[6 * (size_t)k + 1];
+  nu[6 * (size_t)k + 5] = w[6 * (size_t)k + 2];
   const double rk_w = __fma_rn(xk, wkx, __fma_rn(yk, wky, zk * wkz)) * rm3;  // w_k . r_k / |r_k|^3
-  const double rk_W = k_is_source ? __fma_rn(xk, Wx, __fma_rn(yk, Wy, zk * Wz)) * rm3 : 0.0;
-  dm[k] += G * (dmk - rk_w - rk_W);
-  m0_part[k] = -G * rk_w;
+  const double rk_W = __fma_rn(xk, Wx, __fma_rn(yk, Wy, zk * Wz)) * rm3;
+  dm[k] += G * (tot[7] - rk_w - rk_W);
+  m0_part[k] -= G * rk_w;
 }
 
 // dm[0] += sum of the per-body parts, one block, fixed order
@@ -221,6 +301,7 @@ struct sol_adjoint_state {
   double* d_lam = nullptr;    // 6N
   double* d_w = nullptr;      // 6N
   double* d_soa = nullptr;    // 7N
+  double* d_wsum = nullptr;   // 6 per CTA of k_vjp_cotangent
   double* d_dm = nullptr;     // N
   double* d_m0p = nullptr;    // N
   double* d_tmp = nullptr;    // 6N
@@ -228,7 +309,7 @@ struct sol_adjoint_state {
 
 void sol_adjoint_free(sol_adjoint_state* a) {
   if (!a) return;
-  double* p[] = {a->d_cp, a->d_stages, a->d_nu, a->d_lam, a->d_w, a->d_soa, a->d_dm, a->d_m0p, a->d_tmp};
+  double* p[] = {a->d_cp, a->d_stages, a->d_nu, a->d_lam, a->d_w, a->d_soa, a->d_wsum, a->d_dm, a->d_m0p, a->d_tmp};
   for (double* q : p)
     if (q) cudaFree(q);
   delete a;
@@ -245,15 +326,15 @@ int set_fixed_h(sol_ctx* c, double h) {
   return SOL_OK;
 }
 
-int vjp(sol_ctx* c, sol_adjoint_state* a, const double* Y, const double* w, double* nu) {
+// nu = J(Y)^T w of the cotangent w = h sum_i L.c[i] L.v[i]
+int vjp(sol_ctx* c, sol_adjoint_state* a, const double* Y, double h, const Lin& L, double* nu) {
   const int n = c->n;
-  k_vjp_prepass<<<(n + kBlock - 1) / kBlock, kBlock, 0, c->stream>>>(n, Y, w, c->d_mass, a->d_soa);
+  const int nb = (n + kPreBodies - 1) / kPreBodies;
+  k_vjp_cotangent<<<nb, 6 * kPreBodies, 0, c->stream>>>(n, c->cls.nm, Y, c->d_mass, h, L, a->d_w, a->d_soa,
+                                                        a->d_wsum);
   SOL_LAUNCHED();
-  const int threads = kWarpsPerBlock * 32;
-  k_vjp<<<(n + kWarpsPerBlock - 1) / kWarpsPerBlock, threads, 0, c->stream>>>(
-      n, c->cls.nm, c->cls.n_spl, a->d_soa, w, nu, a->d_dm, a->d_m0p);
-  SOL_LAUNCHED();
-  k_sum_m0<<<1, kBlock, 0, c->stream>>>(n, a->d_m0p, a->d_dm);
+  k_vjp<<<n, kVjpThreads, 0, c->stream>>>(n, c->cls.nm, c->cls.n_spl, a->d_soa, a->d_wsum, nb, a->d_w, nu, a->d_dm,
+                                          a->d_m0p);
   SOL_LAUNCHED();
   return SOL_OK;
 }
@@ -323,11 +404,13 @@ extern "C" int sol_adjoint_backward(sol_ctx* c, const double* dl_dy_final, doubl
   RET(alloc(&a->d_lam, nv));
   RET(alloc(&a->d_w, nv));
   RET(alloc(&a->d_soa, 7 * (size_t)n));
+  RET(alloc(&a->d_wsum, 6 * (size_t)((n + kPreBodies - 1) / kPreBodies)));
   RET(alloc(&a->d_dm, n));
   RET(alloc(&a->d_m0p, n));
   RET(alloc(&a->d_tmp, nv));
   SOL_CUDA(cudaMemcpyAsync(a->d_lam, dl_dy_final, sizeof(double) * nv, cudaMemcpyHostToDevice, c->stream));
   SOL_CUDA(cudaMemsetAsync(a->d_dm, 0, sizeof(double) * n, c->stream));
+  SOL_CUDA(cudaMemsetAsync(a->d_m0p, 0, sizeof(double) * n, c->stream));
   RET(set_fixed_h(c, a->h));
   const double h = a->h;
   const int g = grid_for((int)nv);
@@ -357,9 +440,7 @@ extern "C" int sol_adjoint_backward(sol_ctx* c, const double* dl_dy_final, doubl
             L.v[L.k] = a->d_nu + (size_t)j * nv;
             L.c[L.k++] = kA[j][k];
           }
-        k_lincomb<<<g, kBlock, 0, c->stream>>>((int)nv, a->d_w, nullptr, h, L);
-        SOL_LAUNCHED();
-        RET(vjp(c, a, Ys + (size_t)k * nv, a->d_w, a->d_nu + (size_t)k * nv));
+        RET(vjp(c, a, Ys + (size_t)k * nv, h, L, a->d_nu + (size_t)k * nv));
       }
       Lin L;
       memset(&L, 0, sizeof(L));
@@ -372,6 +453,8 @@ extern "C" int sol_adjoint_backward(sol_ctx* c, const double* dl_dy_final, doubl
       std::swap(a->d_w, a->d_lam);
     }
   }
+  k_sum_m0<<<1, kBlock, 0, c->stream>>>(n, a->d_m0p, a->d_dm);
+  SOL_LAUNCHED();
   if (dl_dy0) SOL_CUDA(cudaMemcpyAsync(dl_dy0, a->d_lam, sizeof(double) * nv, cudaMemcpyDeviceToHost, c->stream));
   if (dl_dmass) SOL_CUDA(cudaMemcpyAsync(dl_dmass, a->d_dm, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
   SOL_CUDA(cudaStreamSynchronize(c->stream));
