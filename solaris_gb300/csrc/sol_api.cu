@@ -870,9 +870,15 @@ int sol_integrals(sol_ctx* c, const double* y0_or_null, double o[16]) {
       }
     }
   } else {
-    double unordered = 0.0;
-    for (int b = 0; b < nparts; b++) unordered += pe[b];
-    pes = 2.0 * unordered;
+    // compensated (Neumaier): there are up to a few ten thousand parts
+    double unordered = 0.0, comp = 0.0;
+    for (int b = 0; b < nparts; b++) {
+      const double u = unordered + pe[b];
+      if (std::isfinite(u))
+        comp += fabs(unordered) >= fabs(pe[b]) ? (unordered - u) + pe[b] : (pe[b] - u) + unordered;
+      unordered = u;
+    }
+    pes = 2.0 * (unordered + comp);
   }
   o[14] = pes * (0.5 * 2.959122082855911025e-4);
   o[15] = o[13] - o[14];
