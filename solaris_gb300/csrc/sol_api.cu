@@ -110,6 +110,8 @@ GasDev make_gas_dev(const sol_gas_component* g, int barycentric) {
   return d;
 }
 
+constexpr size_t kStagedBytes = 256 * 1024;  // dydt of up to 5,461 bodies comes back through the pinned slab
+
 template <class T>
 int dev_alloc(T** p, size_t count) {
   *p = nullptr;
@@ -138,9 +140,9 @@ int upload(T* d, const T* h, size_t count, T fill) {
 void free_ctx(sol_ctx* c) {
   if (!c) return;
   void* ptrs[] = {c->d_type, c->d_mig_type, c->d_mig_stop_at, c->d_mass, c->d_radius, c->d_density, c->d_cd,
-                  c->d_gs, c->d_ge, c->d_rm3, c->d_nn_dist, c->d_src, c->d_drag, c->d_mig1, c->d_mig2,
-                  c->d_ind_part, c->d_ind_sum, c->d_nn_idx, c->d_y0, c->d_y, c->d_accel, c->d_yscale, c->d_err,
-                  c->d_ytmp, c->d_io_in, c->d_io_out, c->d_partial, c->d_ctrl, c->d_part};
+                  c->d_gs, c->d_ge, c->d_src, c->d_drag, c->d_mig1, c->d_mig2,
+                  c->d_ind_part, c->d_ind_sum, c->d_y0, c->d_y, c->d_accel, c->d_yscale, c->d_err,
+                  c->d_ytmp, c->d_io_in, c->d_partial, c->d_slab, c->d_part};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (int k = 0; k < 13; ++k)
@@ -153,6 +155,7 @@ void free_ctx(sol_ctx* c) {
   free(c->h_id);
   if (c->h_ctrl) cudaFreeHost(c->h_ctrl);
   if (c->h_stage) cudaFreeHost(c->h_stage);
+  if (c->h_slab) cudaFreeHost(c->h_slab);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
 }
@@ -305,8 +308,7 @@ int sol_create(const sol_body_data* b, const sol_gas_component* gas, int32_t bar
   if ((rc = dev_alloc(&c->d_type, N)) || (rc = dev_alloc(&c->d_mig_type, N)) ||
       (rc = dev_alloc(&c->d_mig_stop_at, N)) || (rc = dev_alloc(&c->d_mass, N)) ||
       (rc = dev_alloc(&c->d_radius, N)) || (rc = dev_alloc(&c->d_density, N)) || (rc = dev_alloc(&c->d_cd, N)) ||
-      (rc = dev_alloc(&c->d_gs, N)) || (rc = dev_alloc(&c->d_ge, N)) || (rc = dev_alloc(&c->d_rm3, N)) ||
-      (rc = dev_alloc(&c->d_nn_dist, N)) || (rc = dev_alloc(&c->d_nn_idx, N)) ||
+      (rc = dev_alloc(&c->d_gs, N)) || (rc = dev_alloc(&c->d_ge, N)) ||
       (rc = dev_alloc(&c->d_src, (size_t)sol_force_src_doubles() * c->npad)) ||
       (rc = dev_alloc(&c->d_drag, 3 * (size_t)(cl.n_spl + cl.n_pl))) ||
       (rc = dev_alloc(&c->d_mig1, 3 * (size_t)(cl.n_rocky + cl.n_proto))) ||
@@ -314,15 +316,27 @@ int sol_create(const sol_body_data* b, const sol_gas_component* gas, int32_t bar
       (rc = dev_alloc(&c->d_ind_part, 6 * (size_t)sol_force_prepass_blocks(c->npad))) ||
       (rc = dev_alloc(&c->d_ind_sum, 8)) || (rc = dev_alloc(&c->d_y0, NV)) || (rc = dev_alloc(&c->d_y, NV)) ||
       (rc = dev_alloc(&c->d_accel, NV)) || (rc = dev_alloc(&c->d_yscale, NV)) || (rc = dev_alloc(&c->d_err, NV)) ||
-      (rc = dev_alloc(&c->d_ytmp, NV)) || (rc = dev_alloc(&c->d_io_in, NV)) || (rc = dev_alloc(&c->d_io_out, NV)))
+      (rc = dev_alloc(&c->d_ytmp, NV)) || (rc = dev_alloc(&c->d_io_in, NV)))
     return fail(rc);
   for (int q = 0; q < 13; ++q)
     if ((rc = dev_alloc(&c->d_fk[q], NV))) return fail(rc);
   c->n_partial = sol_integrate_partials_needed(NV);
   // d_part (chunk partials of the 2-D split kernel) is allocated when a split
   // precision is first selected for a system that uses that kernel
-  if ((rc = dev_alloc(&c->d_partial, (size_t)c->n_partial + 16)) || (rc = dev_alloc(&c->d_ctrl, 1))) return fail(rc);
+  if ((rc = dev_alloc(&c->d_partial, (size_t)c->n_partial + 16))) return fail(rc);
+  auto aligned = [](size_t b) { return (b + 255) & ~(size_t)255; };
+  const size_t o_rm3 = aligned(sizeof(double) * NV), o_nd = o_rm3 + aligned(sizeof(double) * N),
+               o_nn = o_nd + aligned(sizeof(double) * N), o_ctrl = o_nn + aligned(sizeof(int32_t) * N);
+  c->slab_from = sizeof(double) * NV <= kStagedBytes ? 0 : o_rm3;
+  c->slab_bytes = o_ctrl + sizeof(sol_ctrl);
+  if ((rc = dev_alloc(&c->d_slab, c->slab_bytes))) return fail(rc);
+  c->d_io_out = reinterpret_cast<double*>(c->d_slab);
+  c->d_rm3 = reinterpret_cast<double*>(c->d_slab + o_rm3);
+  c->d_nn_dist = reinterpret_cast<double*>(c->d_slab + o_nd);
+  c->d_nn_idx = reinterpret_cast<int32_t*>(c->d_slab + o_nn);
+  c->d_ctrl = reinterpret_cast<sol_ctrl*>(c->d_slab + o_ctrl);
   if (cudaMallocHost((void**)&c->h_ctrl, sizeof(sol_ctrl)) != cudaSuccess ||
+      cudaMallocHost((void**)&c->h_slab, c->slab_bytes - c->slab_from) != cudaSuccess ||
       cudaMallocHost((void**)&c->h_stage, sizeof(double) * NV) != cudaSuccess) {
     sol_set_error("cudaMallocHost failed");
     return fail(SOL_ERR_NOMEM);
@@ -427,16 +441,24 @@ int sol_accel_compute(sol_ctx* c, double t, const double* y, double* dydt, doubl
   RET(set_device(c));
   SOL_CUDA(cudaMemcpyAsync(c->d_io_in, y, sizeof(double) * c->nv, cudaMemcpyHostToDevice, c->stream));
   TimeSpec ts{nullptr, nullptr, 0.0, t};
-  SOL_CUDA(cudaMemsetAsync(&c->d_ctrl->dev_status, 0, sizeof(int), c->stream));
-  RET(sol_force_launch(c, c->d_io_in, c->d_io_out, ts, c->eval_flags));
-  SOL_CUDA(cudaMemcpyAsync(dydt, c->d_io_out, sizeof(double) * c->nv, cudaMemcpyDeviceToHost, c->stream));
-  if (rm3) SOL_CUDA(cudaMemcpyAsync(rm3, c->d_rm3, sizeof(double) * c->n, cudaMemcpyDeviceToHost, c->stream));
-  if (nn_idx)
-    SOL_CUDA(cudaMemcpyAsync(nn_idx, c->d_nn_idx, sizeof(int32_t) * c->n, cudaMemcpyDeviceToHost, c->stream));
-  if (nn_dist)
-    SOL_CUDA(cudaMemcpyAsync(nn_dist, c->d_nn_dist, sizeof(double) * c->n, cudaMemcpyDeviceToHost, c->stream));
-  SOL_CUDA(cudaMemcpyAsync(c->h_ctrl, c->d_ctrl, sizeof(sol_ctrl), cudaMemcpyDeviceToHost, c->stream));
+  RET(sol_force_launch_parts(c, c->d_io_in, c->d_io_out, ts, c->eval_flags, 3, &c->d_ctrl->dev_status));
+  // A copy into pageable memory blocks for ~8 us whatever its size (measured
+  // up to 100 KB; 12 us at 480 KB), so rm3, the neighbours and the status
+  // come back in one asynchronous copy into the pinned slab.  dydt joins it
+  // while moving it again on the host (~30 us per MB) costs less than a copy
+  // of its own.
+  const size_t nb = sizeof(double) * c->nv;
+  const size_t from = c->slab_from;
+  const bool staged = from == 0;
+  SOL_CUDA(cudaMemcpyAsync(c->h_slab, c->d_slab + from, c->slab_bytes - from, cudaMemcpyDeviceToHost, c->stream));
+  if (!staged) SOL_CUDA(cudaMemcpyAsync(dydt, c->d_io_out, nb, cudaMemcpyDeviceToHost, c->stream));
   SOL_CUDA(cudaStreamSynchronize(c->stream));
+  auto host = [&](const void* d) { return c->h_slab + ((const char*)d - c->d_slab - from); };
+  if (staged) memcpy(dydt, host(c->d_io_out), nb);
+  if (rm3) memcpy(rm3, host(c->d_rm3), sizeof(double) * c->n);
+  if (nn_idx) memcpy(nn_idx, host(c->d_nn_idx), sizeof(int32_t) * c->n);
+  if (nn_dist) memcpy(nn_dist, host(c->d_nn_dist), sizeof(double) * c->n);
+  memcpy(c->h_ctrl, host(c->d_ctrl), sizeof(sol_ctrl));
   c->last_eval_valid = 1;
   if (c->h_ctrl->dev_status & SOL_DEV_TIMEOUT) {
     sol_set_error("a bounded device wait ran out in the force kernel");

@@ -52,10 +52,12 @@ __device__ __forceinline__ float* ftab(const ForceCtx& fc) { return reinterpret_
 
 // prec: SOL_PRECISION_*.  The split forms also sum the indirect term; SPLIT_FF
 // (2-D kernel, ff = 1) also takes the largest |coordinate| and writes G m as
-// float (hi, lo) arrays of the float table.
-__global__ void k_prepass(ForceCtx fc, const double* __restrict__ y, int split, int ff) {
+// float (hi, lo) arrays of the float table.  clear: a status word to zero for
+// the kernels that follow (or null).
+__global__ void k_prepass(ForceCtx fc, const double* __restrict__ y, int split, int ff, int* clear) {
   const int n = fc.cls.n;
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (clear && j == 0) *clear = 0;
   double q[6] = {0, 0, 0, 0, 0, 0};  // indirect contributions: massive range, super-planetesimal range
   unsigned mbits = 0;                 // |coordinate| maximum as FP32 bits, rounded up
   if (j < fc.npad) {
@@ -1381,14 +1383,14 @@ static int launch_ref(sol_ctx* c, const ForceCtx& fc, const double* d_y, double*
 // The sinks of fc's range [sink_lo, sol_sink_hi) (every body by default);
 // the prepass always covers every body (the sources).
 static int force_launch(sol_ctx* c, const ForceCtx& fc, const double* d_y, double* d_dydt, TimeSpec ts,
-                        uint32_t flags, int parts) {
+                        uint32_t flags, int parts, int* d_clear) {
   const int nsink = sol_sink_hi(fc) - fc.sink_lo;
   const int split = (c->precision != SOL_PRECISION_FP64 && !c->barycentric) ? 1 : 0;
   // SPLIT_FF systems beyond the warp-per-sink kernel run k_pairs_ff on the float table
   const int ff2d = split && c->precision == SOL_PRECISION_SPLIT_FF && sol_force_uses_chunk_partials(c, c->precision);
   if (parts & 1) {
     const int nb_pre = (fc.npad + kPrepassBlock - 1) / kPrepassBlock;
-    k_prepass<<<nb_pre, kPrepassBlock, 0, c->stream>>>(fc, d_y, split, ff2d);
+    k_prepass<<<nb_pre, kPrepassBlock, 0, c->stream>>>(fc, d_y, split, ff2d, d_clear);
     SOL_LAUNCHED();
     if (split && !c->barycentric) {
       k_ind_reduce<<<1, 256, 0, c->stream>>>(fc);
@@ -1439,8 +1441,9 @@ static int force_launch(sol_ctx* c, const ForceCtx& fc, const double* d_y, doubl
   return SOL_OK;
 }
 
-int sol_force_launch_parts(sol_ctx* c, const double* d_y, double* d_dydt, TimeSpec ts, uint32_t flags, int parts) {
-  return force_launch(c, c->fc, d_y, d_dydt, ts, flags, parts);
+int sol_force_launch_parts(sol_ctx* c, const double* d_y, double* d_dydt, TimeSpec ts, uint32_t flags, int parts,
+                           int* d_clear) {
+  return force_launch(c, c->fc, d_y, d_dydt, ts, flags, parts, d_clear);
 }
 
 int sol_force_launch(sol_ctx* c, const double* d_y, double* d_dydt, TimeSpec ts, uint32_t flags) {
@@ -1454,7 +1457,7 @@ int sol_force_launch_sinks(sol_ctx* c, const double* d_y, double* d_dydt, TimeSp
   ForceCtx fc = c->fc;
   fc.sink_lo = lo;
   fc.sink_hi = hi;
-  return force_launch(c, fc, d_y, d_dydt, ts, flags, 3);
+  return force_launch(c, fc, d_y, d_dydt, ts, flags, 3, nullptr);
 }
 
 int sol_force_tile() { return kTile; }
@@ -1612,13 +1615,13 @@ extern "C" int sol_gravity_noalloc(const sol_nbodies* counts, const int32_t* d_t
   fc.n_ind_blocks = (fc.npad + kPrepassBlock - 1) / kPrepassBlock;
   int* status = noalloc_status_word(scratch);
   // The array keeps the previous call's contents: the source table and the
-  // partials are rewritten in full below, the status word must start at zero.
-  SOL_CUDA(cudaMemsetAsync(status, 0, sizeof(int), st));
+  // partials are rewritten in full below, the status word must start at zero
+  // (the prepass clears it).
   // rm3[0] (the central body) is never computed and reads as 0, as in the
   // reference, whose rm3 array starts zeroed (Acceleration.cpp:65-69).
   SOL_CUDA(cudaMemsetAsync(d_rm3, 0, sizeof(double), st));
   const int split = precision == SOL_PRECISION_SPLIT;
-  k_prepass<<<fc.n_ind_blocks, kPrepassBlock, 0, st>>>(fc, d_y, split, 0);
+  k_prepass<<<fc.n_ind_blocks, kPrepassBlock, 0, st>>>(fc, d_y, split, 0, status);
   SOL_LAUNCHED();
   if (split) {
     k_ind_reduce<<<1, 256, 0, st>>>(fc);

@@ -158,6 +158,12 @@ struct sol_ctx {
   int32_t* d_nn_idx;
   double *d_y0, *d_y, *d_accel, *d_yscale, *d_err, *d_ytmp, *d_fk[13];
   double *d_io_in, *d_io_out;  // boundary staging for host-buffer calls
+  // what a host-buffer evaluation brings back, in one allocation so that one
+  // copy moves it: d_io_out, d_rm3, d_nn_dist, d_nn_idx and d_ctrl point into
+  // it, and h_slab (pinned) mirrors it from slab_from on (0, or behind dydt
+  // where that is large)
+  char *d_slab, *h_slab;
+  size_t slab_bytes, slab_from;
   double* d_partial;           // block partial maxima of the error norm
   double* d_part;              // per-chunk partial sums of the split pair kernels
   int n_partial;
@@ -183,7 +189,8 @@ struct sol_ctx {
 
 // ---- launch helpers (defined in sol_force.cu / sol_integrate.cu) --------------
 int sol_force_launch(sol_ctx* c, const double* d_y, double* d_dydt, TimeSpec ts, uint32_t flags);
-int sol_force_launch_parts(sol_ctx* c, const double* d_y, double* d_dydt, TimeSpec ts, uint32_t flags, int parts);
+int sol_force_launch_parts(sol_ctx* c, const double* d_y, double* d_dydt, TimeSpec ts, uint32_t flags, int parts,
+                           int* d_clear = nullptr);
 int sol_integrator_run(sol_ctx* c, int integrator, int n_steps);
 int sol_rkf78_single_attempt(sol_ctx* c, double t, double h, const double* d_y0, double* d_y, double* d_err,
                              double* error_max);
