@@ -637,7 +637,7 @@ int events_pending(sol_ctx* c, double ej, double hc, double cf, bool* pending) {
 }
 
 // sol_sim_line + stop reason + event flags of the group driver
-constexpr size_t kSimBytes = 256 + sizeof(int) * 2 * kGroupMaxCtas;
+constexpr size_t kSimBytes = 256;
 
 int ensure_sim(sol_ctx* c) {
   if (!c->d_sim) {
@@ -707,7 +707,6 @@ int sol_run_until(sol_ctx* c, int32_t integrator, sol_sim_line* L, int32_t max_s
     sim.cf = collision_factor > 0 ? collision_factor : 0.0;
     sim.line = reinterpret_cast<sol_sim_line*>(base);
     sim.reason = reinterpret_cast<int*>(base + 128);
-    sim.ev = reinterpret_cast<int*>(base + 256);
     sim.yprev = collision_factor > 0 ? c->d_ystart : nullptr;
     sol_ctrl h0;
     memset(&h0, 0, sizeof(h0));

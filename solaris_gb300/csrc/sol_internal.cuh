@@ -210,16 +210,13 @@ int sol_persist_eligible(const sol_ctx* c);
 int sol_persist_rkf78(sol_ctx* c, int n_steps);
 int sol_group_eligible(const sol_ctx* c);
 // The Simulator's step loop inside the group driver (sol_run_until): event
-// thresholds (0: off), and device memory for the line, the stop reason and
-// double-buffered per-CTA event flags.
+// thresholds (0: off), and device memory for the line and the stop reason.
 struct GroupSim {
   double e3, h3, cf;
   sol_sim_line* line;
   int* reason;
-  int* ev;        // [2 * kGroupMaxCtas]
   double* yprev;  // when not null: the state at the start of the step that stops with an event
 };
-constexpr int kGroupMaxCtas = 2048;
 int sol_group_rkf78(sol_ctx* c, int n_steps, const GroupSim* sim = nullptr, int rk4 = 0);
 int sol_fp64_peak_launch(int device, double* flops);
 void sol_noalloc_wait_test(unsigned spin_limit, int withhold_tile);
