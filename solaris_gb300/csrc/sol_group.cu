@@ -8,7 +8,7 @@
 // each:
 //   A. worker warps: a lane per item -- a (sink, source) pair or a body and
 //      the origin (rm3 is that "pair") -- forms d, |d|, |d|^-3 and d |d|^-3;
-//      drag (in four roles) and migration in worker warps of their own;
+//      drag (in five roles) and migration in worker warps of their own;
 //   B. state warps, one lane per state element, which holds its y0, its stage
 //      sums and its error terms in registers for the whole launch: a velocity
 //      lane adds the GravityAC sum of its (sink, component) in the reference's
@@ -180,7 +180,7 @@ struct View {
   double* x;     // [3][kMaxSources] r_j rm3_j of the sources
   double* gm;    // [icap]: G m of the item's source; of the origin, -G (m_0 + m_i)
   double* gbuf;  // [3 cap]: drag or migration buffer of each sink
-  double* dv;    // [6][cap]: the drag's partial results of each planetesimal
+  double* dv;    // [kRoleValues][cap]: the drag's partial results of each planetesimal
   int* ends;     // [icap]: slot subtracted | slot << 16
   int* base;     // [cap + 1]: first item of each sink
   int* mig;      // [cap]: migType of each sink
@@ -231,12 +231,31 @@ __device__ __noinline__ void mig_compute(const ForceCtx& fc, int i, int kind, co
   buf[2] = d[2];
 }
 
-// The regime part of GasDragAC (Acceleration.cpp:364-401) from lambda(r),
-// r, the density's two factors and the gas velocity.
+// The rest of GasDragAC (Acceleration.cpp:364-401) from the roles' values: the
+// gas velocity (GasComponent.cpp:97-138) and the regime.
 __device__ __forceinline__ void drag_finish(const GasDev& g, double factor, double m0pt, const double* yi,
                                            double radius, double density, double cd, double gs, double ge,
-                                           double lambda, double r, double ex, double rp, double vgx, double vgy,
-                                           double out[3]) {
+                                           const double* dv, int cap, double out[3]) {
+  const double lambda = dv[0], r = dv[cap], p = dv[2 * cap], w = dv[3 * cap], ex = dv[4 * cap], rp = dv[5 * cap],
+               vc = dv[6 * cap], v = dv[7 * cap];
+  double vgx = 0.0, vgy = 0.0;
+  {
+    const double x = yi[0], y = yi[1];
+    if (x == 0.0 && y == 0.0) {
+    } else if (y == 0.0) {
+      vgy = x > 0.0 ? vc : -vc;
+    } else if (x == 0.0) {
+      vgx = y > 0.0 ? -vc : vc;
+    } else if (x >= y) {
+      vgy = x >= 0 ? vc / w : -vc / w;
+      vgx = -vgy * p;
+    } else {
+      vgx = y >= 0 ? -vc / w : vc / w;
+      vgy = -vgx * p;
+    }
+    vgx *= v;
+    vgy *= v;
+  }
   const double ux = yi[3] - vgx, uy = yi[4] - vgy, uz = yi[5] - 0.0;
   const double rho = rp * ex;
   const double rhoGas = factor * rho;
@@ -267,59 +286,48 @@ __device__ __forceinline__ void drag_finish(const GasDev& g, double factor, doub
   out[2] = -C * uz;
 }
 
-// One of the four independent parts of GasDragAC (Acceleration.cpp:342-363,
+// One of the five independent parts of GasDragAC (Acceleration.cpp:342-363,
 // gas_velocity and gas_density_at of GasComponent.cpp:97-157) for the
 // planetesimal of this lane, in the operations of sol_gas_drag:
-//   role 0: r and the mean free path lambda(r);
+//   role 0: r, the mean free path lambda(r), and the ratio p of the circular
+//           velocity's components with sqrt(1 + p^2);
 //   role 1: the density's vertical exponential exp(-(z / h(rc))^2);
 //   role 2: the density's power law (or the inner-edge form);
-//   role 3: the gas velocity with its eta(rc) correction.
+//   role 3: the circular velocity;
+//   role 4: its eta(rc) correction.
 // A warp takes one role for 32 planetesimals, so its lanes share the
-// exponent of their pow and run the same instructions; the four roles run in
-// four warps at once and drag_finish combines them.
-__device__ __noinline__ void drag_role(const GasDev& g, int role, double m0, const double* yi, double out[2]) {
+// exponent of their power and run the same instructions; the roles run in
+// warps side by side and drag_finish combines them.  Into dv, at stride cap:
+// lambda, r, p, sqrt(1 + p^2), the exponential, the power law, the circular
+// velocity, the correction.
+constexpr int kRoles = 5, kRoleValues = 8;
+__device__ __noinline__ void drag_role(const GasDev& g, int role, double m0, const double* yi, double* dv, int cap) {
   const double x = yi[0], y = yi[1], z = yi[2];
   if (role == 0) {
     const double r = sqrt(x * x + y * y + z * z);
-    out[0] = sol_pl(g.mfp_c, g.mfp_i, r);
-    out[1] = r;
-  } else if (role == 1) {
-    const double rc = sqrt(x * x + y * y);
+    dv[0] = sol_pl(g.mfp_c, g.mfp_i, r);
+    dv[cap] = r;
+    const double p = x >= y ? y / x : x / y;
+    dv[2 * cap] = p;
+    dv[3 * cap] = sqrt(1.0 + p * p);
+    return;
+  }
+  const double rc = sqrt(x * x + y * y);
+  if (role == 1) {
     const double hh = sol_pl(g.sh_c, g.sh_i, rc);
     const double qq = z / hh;
-    out[0] = exp(-(qq * qq));
+    dv[4 * cap] = sol_exp_neg(qq * qq);
   } else if (role == 2) {
-    const double rc = sqrt(x * x + y * y);
     if (g.inner_edge < rc) {
-      out[0] = sol_pl(g.rho_c, g.rho_i, rc);
+      dv[5 * cap] = sol_pl(g.rho_c, g.rho_i, rc);
     } else {
       const double r2c = rc * rc;
-      out[0] = (g.rho_c * pow(g.inner_edge, g.rho_i - 4.0)) * (r2c * r2c);
+      dv[5 * cap] = (g.rho_c * sol_pow(g.inner_edge, g.rho_i - 4.0)) * (r2c * r2c);
     }
+  } else if (role == 3) {
+    dv[6 * cap] = sqrt((SOL_GAUSS2 * m0) / rc);
   } else {
-    double vgx = 0.0, vgy = 0.0;
-    const double mu = SOL_GAUSS2 * m0;
-    const double rc = sqrt(x * x + y * y);
-    const double vc = sqrt(mu / rc);
-    if (x == 0.0 && y == 0.0) {
-    } else if (y == 0.0) {
-      vgy = x > 0.0 ? vc : -vc;
-    } else if (x == 0.0) {
-      vgx = y > 0.0 ? -vc : vc;
-    } else if (x >= y) {
-      const double p = y / x;
-      vgy = x >= 0 ? vc / sqrt(1.0 + p * p) : -vc / sqrt(1.0 + p * p);
-      vgx = -vgy * p;
-    } else {
-      const double p = x / y;
-      vgx = y >= 0 ? -vc / sqrt(1.0 + p * p) : vc / sqrt(1.0 + p * p);
-      vgy = -vgx * p;
-    }
-    const double v = sqrt(1.0 - 2.0 * sol_pl(g.eta_c, g.eta_i, rc));
-    vgx *= v;
-    vgy *= v;
-    out[0] = vgx;
-    out[1] = vgy;
+    dv[7 * cap] = sqrt(1.0 - 2.0 * sol_pl(g.eta_c, g.eta_i, rc));
   }
 }
 
@@ -464,7 +472,7 @@ __device__ __noinline__ void work(const GroupArgs& P, const View& V, const Ctl& 
     const uint32_t flags = S.flags;
     const bool drag = ndrag > 0 && (flags & SOL_EVAL_GAS_DRAG);
     const bool mig = nmig > 0 && (flags & (SOL_EVAL_TYPE_I | SOL_EVAL_TYPE_II));
-    const int u_drag = drag ? 4 * w_role : 0;
+    const int u_drag = drag ? kRoles * w_role : 0;
     const int u_mig = u_drag + (mig ? (nmig + 31) >> 5 : 0);
     const int units = u_mig + ((nitem + 31) >> 5);
     for (int u = w; u < units; u += nwork) {  // the longest first
@@ -475,11 +483,7 @@ __device__ __noinline__ void work(const GroupArgs& P, const View& V, const Ctl& 
         const int role = u / w_role;
         const int d = (u - role * w_role) * 32 + lane;
         if (d < ndrag) {
-          double o[2];
-          drag_role(fc.gas, role, fc.mass[0], yt + 6 * V.dlist[d], o);
-          const int k0 = role == 0 ? 0 : role == 1 ? 2 : role == 2 ? 3 : 4;
-          V.dv[k0 * V.cap + d] = o[0];
-          if (role == 0 || role == 3) V.dv[(k0 + 1) * V.cap + d] = o[1];
+          drag_role(fc.gas, role, fc.mass[0], yt + 6 * V.dlist[d], V.dv + d, V.cap);
         }
       } else {  // migration: a lane per massive body
         const int m = (u - u_drag) * 32 + lane;
@@ -504,13 +508,12 @@ __device__ __noinline__ void work(const GroupArgs& P, const View& V, const Ctl& 
       *p = second_pass(body, yt[6 * (e >> 16) + c], V.p[3 * V.icap + it], *p,
                        body ? 0.0 : V.x[c * kMaxSources + (e >> 16)], V.gm[it]);
     }
-    if (drag) {  // the drag's regime part from the four roles, a lane per planetesimal
+    if (drag) {  // the drag's regime part from the roles, a lane per planetesimal
       for (int d = w * 32 + lane; d < ndrag; d += nwork * 32) {
         const int sd = V.dlist[d], i = body_of(P, V, sd);
         double out[3];
         drag_finish(fc.gas, S.factor, S.m0pt, yt + 6 * sd, fc.radius[i], fc.density[i], fc.cd[i], fc.gamma_stokes[i],
-                    fc.gamma_epstein[i], V.dv[0 * V.cap + d], V.dv[1 * V.cap + d], V.dv[2 * V.cap + d],
-                    V.dv[3 * V.cap + d], V.dv[4 * V.cap + d], V.dv[5 * V.cap + d], out);
+                    fc.gamma_epstein[i], V.dv + d, V.cap, out);
         for (int k = 0; k < 3; ++k) V.gbuf[3 * sd + k] = out[k];
         if (S.last && (sd >= P.ns || home)) {  // the buffers hold the last evaluation's drag
           double* gb = global_gas_buf(fc, i, 1);
@@ -961,7 +964,7 @@ size_t layout(GroupArgs& P, int cap) {
   take(P.o_x, (size_t)3 * kMaxSources);
   take(P.o_gm, (size_t)P.icap);
   take(P.o_gbuf, (size_t)3 * cap);
-  take(P.o_dv, (size_t)6 * cap);
+  take(P.o_dv, (size_t)kRoleValues * cap);
   // ints: item ends (icap), first items (cap + 1), migType, gas kind, drag and
   // migration lists (cap each)
   take(P.o_int, ((size_t)P.icap + (size_t)5 * cap + 2) / 2);
@@ -1014,7 +1017,7 @@ int sol_group_rkf78(sol_ctx* c, int n_steps, const GroupSim* sim, int rk4) {
     P.icap = ns * ns + cand * c->cls.nm;
     const int cap = ns + cand;
     P.vw = (3 * cap + 31) / 32;
-    const int gas = c->has_gas ? 4 * ((cap + 31) / 32) + (ns + 31) / 32 : 0;
+    const int gas = c->has_gas ? kRoles * ((cap + 31) / 32) + (ns + 31) / 32 : 0;
     const int units = gas ? gas + (P.icap + 31) / 32 : (4 * P.icap + 31) / 32;  // four lanes an item, or one
     const int workers = std::min(std::max(units, kWorkersMin), kMaxThreads / 32 - 2 * P.vw);
     const size_t sm = std::max(layout(P, cap), (size_t)kSpreadSmem);

@@ -8,6 +8,7 @@
 #include <stdint.h>
 
 #include "../../include/solaris_gb300.h"
+#include "sol_powlaw.cuh"
 
 #define SOL_GAUSS2 2.959122082855911025e-4  // Solaris/Constants.h:29
 #define SOL_GAUSS 1.720209895e-2            // Solaris/Constants.h:28
@@ -384,7 +385,7 @@ __device__ __noinline__ double sol_pow_recip_cr(double x) {
 }
 
 // ---- gas-model device functions (restated from Solaris/GasComponent.cpp) ----
-__device__ __forceinline__ double sol_pl(double c, double idx, double x) { return c * pow(x, idx); }
+__device__ __forceinline__ double sol_pl(double c, double idx, double x) { return c * sol_pow(x, idx); }
 
 __device__ __forceinline__ double sol_reduction_factor(const GasDev& g, double t) {  // :36-61
   switch (g.decrease_type) {
@@ -437,11 +438,11 @@ __device__ __forceinline__ void sol_gas_drag(const GasDev& g, double factor, dou
     double q = z / hh;
     double arg = q * q;
     if (g.inner_edge < rc) {
-      rho = sol_pl(g.rho_c, g.rho_i, rc) * exp(-arg);
+      rho = sol_pl(g.rho_c, g.rho_i, rc) * sol_exp_neg(arg);
     } else {
-      double a = g.rho_c * pow(g.inner_edge, g.rho_i - 4.0);
+      double a = g.rho_c * sol_pow(g.inner_edge, g.rho_i - 4.0);
       double r2c = rc * rc;
-      rho = a * (r2c * r2c) * exp(-arg);
+      rho = a * (r2c * r2c) * sol_exp_neg(arg);
     }
   }
   double rhoGas = factor * rho;
