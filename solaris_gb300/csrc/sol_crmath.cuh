@@ -294,6 +294,11 @@ __device__ __forceinline__ void sol_ref_terms(double gm, double rijm3, double dx
   }
 }
 
+// IEEE arithmetic for a pair the fast paths hand over: |d| and 1 / (|d|^2 |d|)
+static __device__ __noinline__ double2 sol_ref_pair_ieee(double dx, double dy, double dz) {
+  return sol_ref_rinv3_ieee(dx * dx + dy * dy + dz * dz);
+}
+
 // Two independent pairs in one basic block (their dependency chains
 // interleave), the rare IEEE fallbacks after both.
 __device__ __forceinline__ void sol_ref_rinv3_x2(double a0, double a1, double& r0, double& w0, double& r1,

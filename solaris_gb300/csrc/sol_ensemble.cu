@@ -36,6 +36,7 @@ struct EnsCtrl {
   long long n_acc, n_rej;
 };
 
+constexpr int kMaxThreads = 736;  // 88 registers; the largest launch shape sol_ensemble_configure takes effect with
 constexpr int kVecs = 17;  // f0..f12, yscale, ytmp, y, error
 enum { V_YSCALE = 13, V_YTMP = 14, V_Y = 15, V_ERR = 16 };
 
@@ -44,21 +45,49 @@ __constant__ int c_rk_k[13];
 __constant__ int c_rk_idx[13][9];
 __constant__ double c_rk_a[13][9];
 
+// The FP64 pipe binds this kernel (73-80% of it busy, the integer pipe 12-22%
+// with every multiplication on FP64), so the multiplications that need not be
+// FP64 instructions run on the integer pipe (sol_exact_dmul, the same bits):
+// of ~2,900 FP64 instructions a body an attempt with seven sources ~1,900 are
+// left.  Where an operand is outside the integer multiply's range the element
+// is computed again in FP64.
+//
+// One element of a stage input, y0 + h (a_0 f_0 + a_1 f_1 + ...) left to right
+// (RungeKuttaFehlberg78.cpp:169-232).
+__device__ __noinline__ double stage_fp64(const double* slot, int max_nv, int r, int e, double y0, double h) {
+  double acc = c_rk_a[r][0] * slot[(size_t)c_rk_idx[r][0] * max_nv + e];
+  for (int k = 1; k < c_rk_k[r]; ++k) acc = acc + c_rk_a[r][k] * slot[(size_t)c_rk_idx[r][k] * max_nv + e];
+  return y0 + h * acc;
+}
+__device__ __forceinline__ double stage_element(const double* slot, int max_nv, int r, int K, int e, double y0,
+                                                double h) {
+  double f[9];  // every load in flight before the first product
+#pragma unroll
+  for (int k = 0; k < 9; ++k) f[k] = k < K ? slot[(size_t)c_rk_idx[r][k] * max_nv + e] : 0.0;
+  bool ok = true;
+  double acc = sol_exact_dmul<false, true>(c_rk_a[r][0], f[0], ok);
+#pragma unroll
+  for (int k = 1; k < 9; ++k)
+    if (k < K) acc = acc + sol_exact_dmul<false, true>(c_rk_a[r][k], f[k], ok);
+  const double y = y0 + sol_exact_dmul<true, true>(h, acc, ok);
+  return ok ? y : stage_fp64(slot, max_nv, r, e, y0, h);
+}
+
+// The largest v of the CTA (any number of warps), v >= 0: the order of such
+// doubles is that of their bits.
 __device__ __forceinline__ double block_max(double v, double* red) {
-  // NaN entries never replace the maximum, as GetErrorMax
-  const int tid = threadIdx.x;
-  red[tid] = v;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (tid < w) {
-      double o = red[tid + w];
-      if (o > red[tid]) red[tid] = o;
-    }
-    __syncthreads();
+  long long m = __double_as_longlong(v);
+#pragma unroll
+  for (int w = 16; w > 0; w >>= 1) {
+    const long long o = __shfl_xor_sync(0xFFFFFFFFu, m, w);
+    m = o > m ? o : m;
   }
-  double r = red[0];
+  long long* bits = reinterpret_cast<long long*>(red);
+  if ((threadIdx.x & 31) == 0) bits[threadIdx.x >> 5] = m;
   __syncthreads();
-  return r;
+  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) m = bits[w] > m ? bits[w] : m;
+  __syncthreads();
+  return __longlong_as_double(m);
 }
 
 // GravityAC for one system by one CTA.  FP64: the reference's loops and
@@ -150,17 +179,24 @@ __device__ void ens_force(const EnsSys& S, const double* __restrict__ m, const d
       // ascending order; an odd last source pairs with itself
       for (int j = 1; j < ns; j += 2) {
         const int jb[2] = {j, min(j + 1, ns - 1)};
-        double xij[2], yij[2], zij[2], rij2[2];
+        double xij[2], yij[2], zij[2], rijm3[2];
+        bool fast[2];
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           xij[u] = tx[jb[u]] - xi;
           yij[u] = ty[jb[u]] - yi;
           zij[u] = tz[jb[u]] - zi;
-          const double q = xij[u] * xij[u] + yij[u] * yij[u] + zij[u] * zij[u];
-          rij2[u] = jb[u] != i ? q : 1.0;
+          bool ok = true;
+          const double q = sol_exact_dsqr<false>(xij[u], ok) + sol_exact_dsqr<false>(yij[u], ok) +
+                           sol_exact_dsqr<true>(zij[u], ok);
+          double rij;
+          fast[u] = (ok & sol_ref_rinv3_fast(q, rij, rijm3[u])) | (jb[u] == i);
         }
-        double rij[2], rijm3[2];
-        sol_ref_rinv3_x2(rij2[0], rij2[1], rij[0], rijm3[0], rij[1], rijm3[1]);
+        if (!(fast[0] & fast[1])) {
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+            if (!fast[u]) rijm3[u] = sol_ref_pair_ieee(xij[u], yij[u], zij[u]).y;
+        }
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           double t0, t1, t2;
@@ -201,7 +237,7 @@ __device__ void ens_force(const EnsSys& S, const double* __restrict__ m, const d
 }
 
 template <int PREC>
-__global__ void k_ensemble_rkf78(const EnsSys* __restrict__ systems, const int* __restrict__ order,
+__global__ void __launch_bounds__(kMaxThreads) k_ensemble_rkf78(const EnsSys* __restrict__ systems, const int* __restrict__ order,
                                  EnsCtrl* __restrict__ ctrl, double* __restrict__ y0_all,
                                  const double* __restrict__ mass_all, double* __restrict__ scratch,
                                  size_t slot_doubles, int max_nv, int ns_cap, int* queue, int n_sys, int n_steps,
@@ -249,11 +285,7 @@ __global__ void k_ensemble_rkf78(const EnsSys* __restrict__ systems, const int* 
         const double h = C.h;
         for (int r = 1; r <= 12; ++r) {
           const int K = c_rk_k[r];
-          for (int e = tid; e < nv; e += bd) {
-            double acc = c_rk_a[r][0] * slot[(size_t)c_rk_idx[r][0] * max_nv + e];
-            for (int k = 1; k < K; ++k) acc = acc + c_rk_a[r][k] * slot[(size_t)c_rk_idx[r][k] * max_nv + e];
-            ytmp[e] = y0[e] + h * acc;
-          }
+          for (int e = tid; e < nv; e += bd) ytmp[e] = stage_element(slot, max_nv, r, K, e, y0[e], h);
           __syncthreads();
           ens_force<PREC>(S, m, ytmp, f[r], rm3, tab, ns_cap, red);
         }
@@ -416,6 +448,19 @@ int ens_run(sol_ensemble* e, int n_steps) {
 }
 }  // namespace
 
+// The launch shape until the caller sets one.  768 threads fill an SM
+// (registers), and a system's steps are a serial chain: with few systems an SM
+// the last ones decide, so each gets more threads; with many, small CTAs waste
+// the fewest lanes.  Measured (ms, four calls, FP64 / SPLIT_FF, against the 128
+// threads x 4 this rule replaces): 160 systems 8.15 / 5.08 -> 4.05 / 2.67; 512
+// 11.1 / 6.47 -> 6.49 / 3.86; 1,024 12.7 / 7.33 -> 9.63 / 5.96; 3,000 28.2 /
+// 17.4 -> 26.8 / 15.6.
+static void default_shape(int n_systems, int n_sm, int& threads, int& per_sm) {
+  const double s = (double)n_systems / n_sm;
+  threads = s <= 2 ? 512 : s <= 5 ? 384 : s <= 16 ? 256 : 128;
+  per_sm = s <= 5 ? 2 : s <= 16 ? 3 : 6;
+}
+
 extern "C" {
 
 int sol_ensemble_create(const sol_body_data* systems, int32_t n_systems, int32_t device, sol_ensemble** out) {
@@ -478,9 +523,8 @@ int sol_ensemble_create(const sol_body_data* systems, int32_t n_systems, int32_t
   e->ns_cap = (ns_cap + 1) & ~1;  // even, so the float2 table stays aligned
   e->precision = SOL_PRECISION_FP64;
   e->eps = pow(10, -10.0);
-  e->block = 128;
-  e->ctas_per_sm = 4;
   SOL_CUDA(cudaDeviceGetAttribute(&e->n_sm, cudaDevAttrMultiProcessorCount, device));
+  default_shape(n_systems, e->n_sm, e->block, e->ctas_per_sm);
   e->sys_host = sys;
   auto fail = [&](int r) {
     ens_free(e);

@@ -445,13 +445,6 @@ constexpr size_t ref_smem(int sw, int spc) {
          (sizeof(long long) + sizeof(int)) * (size_t)kRefTile * spc;
 }
 
-// IEEE arithmetic for a pair the fast path hands over
-static __device__ __noinline__ double2 ref_pair_slow(double xij, double yij, double zij) {
-  double2 v;
-  sol_ref_rinv3_slow(xij * xij + yij * yij + zij * zij, v.x, v.y);
-  return v;
-}
-
 // rij and 1 / rij^3 of a displacement, the squares on the integer pipe (a z
 // that is zero for every pair, a planar system, stays on the fast path)
 __device__ __forceinline__ void ref_pair(double xij, double yij, double zij, bool valid, double& rij, double& rijm3) {
@@ -461,7 +454,7 @@ __device__ __forceinline__ void ref_pair(double xij, double yij, double zij, boo
   const double qz = sol_exact_dsqr<true>(zij, ok);
   ok = ok & sol_ref_rinv3_fast(qx + qy + qz, rij, rijm3);
   if (!ok & valid) {
-    const double2 v = ref_pair_slow(xij, yij, zij);
+    const double2 v = sol_ref_pair_ieee(xij, yij, zij);
     rij = v.x;
     rijm3 = v.y;
   }
