@@ -11,7 +11,7 @@
 #include "sol_internal.cuh"
 
 int sol_force_tile();
-int sol_force_part_doubles(const sol_ctx* c);
+size_t sol_force_part_doubles(const sol_ctx* c);
 int sol_force_uses_chunk_partials(const sol_ctx* c, int precision);
 int sol_force_prepass_blocks(int npad);
 int sol_force_src_doubles();

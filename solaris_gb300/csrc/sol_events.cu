@@ -254,7 +254,7 @@ __global__ void k_gather_rows(int lo_old, int hi_old, int lo_new, const int* __r
 
 }  // namespace
 
-int sol_force_part_doubles(const sol_ctx* c);
+size_t sol_force_part_doubles(const sol_ctx* c);
 int sol_force_uses_chunk_partials(const sol_ctx* c, int precision);
 
 extern "C" int sol_handle_events(sol_ctx* c, double time, double ejection, double hit_centrum,

@@ -22,6 +22,7 @@
 #include "sol_pair.cuh"
 
 int sol_force_uses_chunk_partials(const sol_ctx* c, int precision);
+size_t sol_force_part_doubles(const sol_ctx* c);
 
 namespace {
 
@@ -160,8 +161,9 @@ __global__ void k_ind_reduce(ForceCtx fc) {
 // Grid triples of every coordinate (f2_grid_disp): a = G1 rint(x / G1),
 // b = G2 rint((x - a) / G2), c = float(x - a - b); a and b are exact floats
 // (at most 2^23 of their grid), x - a and x - a - b exact doubles.  Padding
-// bodies get zeros.
-__global__ void k_split_table(ForceCtx fc, const double* __restrict__ y) {
+// bodies (no mass) are set apart from the others and from each other, so that
+// k_pairs_sym, which does not mask them, meets no close pair among them.
+__global__ void k_split_table(ForceCtx fc, const double* __restrict__ y, float* __restrict__ bound) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= fc.npad) return;
   const double G1 = fc.ind_sum[kIndGrid];
@@ -179,6 +181,8 @@ __global__ void k_split_table(ForceCtx fc, const double* __restrict__ y) {
     T[(size_t)(FBX + 3 * k) * np + j] = (float)b;
     T[(size_t)(FCX + 3 * k) * np + j] = __double2float_rn(r - b);
   }
+  if (bound) bound[j] = 3.0e38f;  // for k_near_bound
+  if (j >= fc.cls.n) T[(size_t)FAX * np + j] = (float)((4194304.0 + 1024.0 * (j - fc.cls.n)) * G1);
 }
 
 // ---- tile pipeline -----------------------------------------------------------
@@ -767,7 +771,7 @@ __global__ void __launch_bounds__(kSinkBlock) k_pairs(ForceCtx fc, const double*
 
 // ---- SPLIT_FF 2-D kernel: float-float pairs with no FP64 instruction -------
 // Same grid as k_pairs (blockIdx.x: kSinkBlock sinks; blockIdx.y: a chunk of
-// sources, 1 to kChunkTiles tiles as split_chunk chooses so that the grid
+// sources, 1 to kChunkTiles tiles as ff_chunk chooses so that the grid
 // fills the GPU) and the same partial outputs for k_combine.  The sources'
 // grid triples and G m (hi, lo) arrive tile by tile in shared memory by bulk
 // copies; each thread takes two sources per step in paired FP32
@@ -926,7 +930,8 @@ __device__ __forceinline__ void ff_four_sources(const float2* va, const float2* 
 // Three CTAs per SM (up to 170 registers): the four-source step keeps both
 // halves' temporaries live at once.
 __global__ void __launch_bounds__(kSinkBlock, 3) k_pairs_ff(ForceCtx fc, const double* __restrict__ y,
-                                                         double* __restrict__ part, int* dev_status, int chunk) {
+                                                         double* __restrict__ part, int* dev_status, int chunk,
+                                                         int j_lo, int j_hi) {
   __shared__ __align__(128) FFTile sm;
   const Classes& c = fc.cls;
   const int n = sol_sink_hi(fc);  // sinks [sink_lo, n)
@@ -935,8 +940,8 @@ __global__ void __launch_bounds__(kSinkBlock, 3) k_pairs_ff(ForceCtx fc, const d
   const int i_first = fc.sink_lo + blockIdx.x * kSinkBlock;
   const int ns_cta = (fc.type[min(i_first, n - 1)] <= SOL_PROTO_PLANET) ? c.nm + c.n_spl : c.nm;
   const int ns = (i < n && fc.type[i] <= SOL_PROTO_PLANET) ? c.nm + c.n_spl : c.nm;
-  const int j_begin = blockIdx.y * chunk;
-  const int j_end = min(j_begin + chunk, ns_cta);
+  const int j_begin = j_lo + blockIdx.y * chunk;  // sources [j_lo, j_hi); j_lo a whole number of tiles
+  const int j_end = min(j_begin + chunk, min(ns_cta, j_hi));
   const int t_begin = j_begin / kTile;
   const int ntiles = j_end > j_begin ? (j_end - j_begin + kTile - 1) / kTile : 0;
   const bool live = i < n && i >= 1;
@@ -1049,17 +1054,107 @@ __global__ void __launch_bounds__(kSinkBlock, 3) k_pairs_ff(ForceCtx fc, const d
   part[base + PIDX * np] = __longlong_as_double((long long)nn);
 }
 
-// Per sink: the chunk partials in chunk order, the nearest neighbour (the
+#include "sol_pairs_sym.cuh"
+
+// Where the partials of an evaluation lie in the context's d_part (offsets in
+// doubles): of the block pairs of k_pairs_sym (bodies [0, 256 nb)), sources'
+// and sinks' sides, and of k_pairs_ff on what is left: r1, every sink and the
+// sources from `from` on; r2, the sinks from there on and the sources before.
+struct FFPlan {
+  int nb = 0, per = 1, chunks = 0;  // k_pairs_sym
+  int from = 0;                                  // 256 nb
+  int n1 = 0, chunk1 = kTile, n2 = 0, chunk2 = kTile;
+  size_t o_j = 0, o_i = 0, o_1 = 0, o_2 = 0, o_bound = 0, doubles = 0;
+};
+
+// Per sink: the partials in a fixed order, the nearest neighbour (the
 // smallest r^2, ties to the lower index as the reference's ascending scan),
 // distanceOfNN recomputed in the reference's FP64 arithmetic for the chosen
 // neighbour, the Kepler and indirect terms, and the gas terms.
-__global__ void k_combine(ForceCtx fc, const double* __restrict__ y, double* __restrict__ dydt,
-                          const double* __restrict__ part, int nchunk, TimeSpec ts, uint32_t flags) {
+// Bounded by the latency of the partials' loads (a few tens to some hundreds a
+// sink, far apart): a CTA's warps share its sinks' partials, eight loaded at a
+// time, and the first warp adds the warps' sums and finishes (10,007 bodies:
+// 21 us for 65 with one thread a sink).
+constexpr int kCombineSinks = 32, kCombineWarps = 4;
+
+__global__ void __launch_bounds__(kCombineSinks* kCombineWarps)
+    k_combine(ForceCtx fc, const double* __restrict__ y, double* __restrict__ dydt, const double* __restrict__ part,
+              FFPlan pl, TimeSpec ts, uint32_t flags) {
+  static_assert(kCombineSinks == 32, "a warp finishes");
+  __shared__ double sh_s[kCombineWarps][6][32];
+  __shared__ long long sh_r2[kCombineWarps][32];
+  __shared__ int sh_nn[kCombineWarps][32];
   const Classes& c = fc.cls;
   const int n = sol_sink_hi(fc);  // sinks [sink_lo, n)
   const int np = fc.npad;
-  const int i = fc.sink_lo + blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = fc.sink_lo + blockIdx.x * kCombineSinks + lane;
+  double sx = 0.0, sy = 0.0, sz = 0.0, ex = 0.0, ey = 0.0, ez = 0.0;
+  long long best = __double_as_longlong(1.0e300);  // r^2 >= 0: the order of doubles is that of their bits
+  int nn = -1;
+  auto near = [&](long long r2, int j) {
+    if (j >= 0 && (r2 < best || (r2 == best && j < nn))) {
+      best = r2;
+      nn = j;
+    }
+  };
+  // partials [0, count), at(k) the first word of partial k and `stride` its
+  // words' distance, loaded eight at a time; their plain sum is compensated
+  // (of_blocks: one block's terms each) or every one (a chunk's, up to 4,096)
+  auto add = [&](int count, size_t stride, bool of_blocks, auto at) {
+    for (int g = 8 * warp; g < count; g += 8 * kCombineWarps) {
+      double v[8][PART_SLOTS];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const double* p = at(min(g + u, count - 1));
+#pragma unroll
+        for (int k = 0; k < PART_SLOTS; ++k) v[u][k] = p[k * stride];
+      }
+      double t[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if (g + u >= count) break;
+        if (of_blocks) {
+          t[0] += v[u][PAX];
+          t[1] += v[u][PAY];
+          t[2] += v[u][PAZ];
+        } else {
+          two_sum(sx, ex, v[u][PAX]);
+          two_sum(sy, ey, v[u][PAY]);
+          two_sum(sz, ez, v[u][PAZ]);
+        }
+        near(__double_as_longlong(v[u][PR2]), (int)__double_as_longlong(v[u][PIDX]));
+      }
+      if (of_blocks) {
+        two_sum(sx, ex, t[0]);
+        two_sum(sy, ey, t[1]);
+        two_sum(sz, ez, t[2]);
+      }
+    }
+  };
+  if (i < n && i > 0) {
+    const int B = i / kSymBlock;
+    if (B < pl.nb) {
+      const double* pj = part + pl.o_j + (i - B * kSymBlock);  // as a source of the blocks below
+      add(B, kSymBlock, true, [&](int I) { return pj + sym_pair_index(I, B, pl.nb) * PART_SLOTS * kSymBlock; });
+      const int first = B / pl.per;  // as a sink of its own block's chunks
+      const double* pi = part + pl.o_i + (size_t)first * PART_SLOTS * np + i;
+      add(pl.chunks - first, np, true, [&](int k) { return pi + (size_t)k * PART_SLOTS * np; });
+    } else {
+      add(pl.n2, np, false, [&](int k) { return part + pl.o_2 + (size_t)k * PART_SLOTS * np + i; });
+    }
+    add(pl.n1, np, false, [&](int k) { return part + pl.o_1 + (size_t)k * PART_SLOTS * np + i; });
+  }
+  sh_s[warp][0][lane] = sx;
+  sh_s[warp][1][lane] = sy;
+  sh_s[warp][2][lane] = sz;
+  sh_s[warp][3][lane] = ex;
+  sh_s[warp][4][lane] = ey;
+  sh_s[warp][5][lane] = ez;
+  sh_r2[warp][lane] = best;
+  sh_nn[warp][lane] = nn;
+  __syncthreads();
+  if (warp > 0 || i >= n) return;
   double* out = dydt + 6 * i;
   if (i == 0) {
     for (int k = 0; k < 6; ++k) out[k] = 0.0;
@@ -1067,22 +1162,17 @@ __global__ void k_combine(ForceCtx fc, const double* __restrict__ y, double* __r
     fc.nn_dist[0] = 0.0;
     return;
   }
-  const double* yv = y + 6 * i;
-  double sx = 0.0, sy = 0.0, sz = 0.0, ex = 0.0, ey = 0.0, ez = 0.0;
-  double best = 1.0e300;
-  int nn = -1;
-  for (int ch = 0; ch < nchunk; ++ch) {
-    const size_t base = (size_t)ch * PART_SLOTS * np + i;
-    two_sum(sx, ex, part[base + PAX * np]);
-    two_sum(sy, ey, part[base + PAY * np]);
-    two_sum(sz, ez, part[base + PAZ * np]);
-    const double r2 = part[base + PR2 * np];
-    const int j = (int)__double_as_longlong(part[base + PIDX * np]);
-    if (j >= 0 && r2 < best) {
-      best = r2;
-      nn = j;
-    }
+#pragma unroll
+  for (int w = 1; w < kCombineWarps; ++w) {
+    two_sum(sx, ex, sh_s[w][0][lane]);
+    two_sum(sy, ey, sh_s[w][1][lane]);
+    two_sum(sz, ez, sh_s[w][2][lane]);
+    ex += sh_s[w][3][lane];
+    ey += sh_s[w][4][lane];
+    ez += sh_s[w][5][lane];
+    near(sh_r2[w][lane], sh_nn[w][lane]);
   }
+  const double* yv = y + 6 * i;
   const int ns = (fc.type[i] <= SOL_PROTO_PLANET) ? c.nm + c.n_spl : c.nm;
   const double mu = SOL_GAUSS2 * (fc.mass[0] + fc.mass[i]);
   const double rm3i = fc.rm3[i];
@@ -1281,36 +1371,34 @@ __global__ void __launch_bounds__(kFewSplitWarps * 32) k_pairs_few(ForceCtx fc, 
 }  // namespace
 
 // parts: 1 = prepass (and indirect totals), 2 = pair kernel, 3 = both.
-// Sources per CTA of the 2-D split kernels: SPLIT takes kChunk; SPLIT_FF a
-// chunk of 1..kChunkTiles tiles: among the grids that give every SM at least
-// the CTAs k_pairs_ff holds at once, the one whose busiest SM has the least
-// work (its CTAs times the tiles of a CTA plus half a tile of per-CTA work),
-// ties to the larger chunk; the finest chunk when no grid is that large.
-// Small systems fill the GPU, and sizes just past a whole number of CTAs
-// per SM avoid a nearly empty last round.
-static int split_chunk(const sol_ctx* c, int precision) {
-  if (precision != SOL_PRECISION_SPLIT_FF) return kChunk;
+static int device_sms(int device) {
   // per device, filled on first use; contexts of several host threads may
-  // race to fill them with the same values, hence the atomics
-  static std::atomic<int> sms[kMaxDevices], resident[kMaxDevices];
-  const int dev = (c->device >= 0 && c->device < kMaxDevices) ? c->device : 0;
-  if (sms[dev].load(std::memory_order_relaxed) == 0) {
-    int nsm = 0, per_sm = 0;
-    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess || nsm < 1) nsm = 152;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pairs_ff, kSinkBlock, 0) != cudaSuccess ||
-        per_sm < 1)
-      per_sm = 3;
-    resident[dev].store(per_sm, std::memory_order_relaxed);
+  // race to fill it with the same value, hence the atomic
+  static std::atomic<int> sms[kMaxDevices];
+  const int dev = (device >= 0 && device < kMaxDevices) ? device : 0;
+  int nsm = sms[dev].load(std::memory_order_acquire);
+  if (nsm == 0) {
+    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || nsm < 1) nsm = 152;
     sms[dev].store(nsm, std::memory_order_release);
   }
-  const long nb = (c->n + kSinkBlock - 1) / kSinkBlock;
-  const long nsm = sms[dev].load(std::memory_order_acquire);
-  const long res = resident[dev].load(std::memory_order_relaxed);
+  return nsm;
+}
+
+// Sources per CTA of k_pairs_ff for nsink sinks and nsrc sources: 1 to
+// kChunkTiles tiles; among the grids that give every SM at least the three
+// CTAs it holds at once, the one whose busiest SM has the least work (its CTAs
+// times the tiles of a CTA plus half a tile of per-CTA work), ties to the
+// larger chunk; the finest chunk when no grid is that large.  Small systems
+// fill the GPU, and sizes just past a whole number of CTAs per SM avoid a
+// nearly empty last round.
+static int ff_chunk(int device, long nsink, long nsrc) {
+  const long nsm = device_sms(device), resident = 3;
+  const long nb = (nsink + kSinkBlock - 1) / kSinkBlock;
   int best_ct = 1;
   double best = 1e300;
   for (int ct = kChunkTiles; ct >= 1; ct >>= 1) {
-    const long ctas = nb * ((c->n + ct * kTile - 1) / (ct * kTile));
-    if (ctas < res * nsm) continue;
+    const long ctas = nb * ((nsrc + ct * kTile - 1) / (ct * kTile));
+    if (ctas < resident * nsm) continue;
     const double cost = (double)((ctas + nsm - 1) / nsm) * (ct + 0.5);
     if (cost < best) {
       best = cost;
@@ -1318,6 +1406,61 @@ static int split_chunk(const sol_ctx* c, int precision) {
     }
   }
   return best_ct * kTile;
+}
+
+// How a SPLIT_FF evaluation is divided.  k_pairs_sym takes the massive bodies
+// (which attract each other) in whole blocks, the last one padded where every
+// body is massive; k_pairs_ff the rest.  From kSymMin bodies on, where the
+// block pairs fill the GPU (us an evaluation with it and without: 5,000 bodies
+// 188 and 144, 6,400 232 and 205, 7,168 232 and 256, 7,500 283 and 262, 7,936
+// 282 and 288, 9,000 341 and 378), up to kSymMax, beyond which the block pairs'
+// partials (10 KB each) would pass 1.4 GB.  One block of sources a CTA up to
+// kSymSingle blocks; above, two and then four halve the sinks' partials (336 MB
+// at 65,536 bodies) for much the same time (24,000 bodies: 1.61 ms with one,
+// 1.65 with two; 45,000: 5.36 and 5.41; 65,536: 11.17 and 11.19).
+constexpr int kSymMin = 7936, kSymMax = 131072, kSymSingle = 192;
+
+static void sym_shape(FFPlan& p, int nb) {
+  p.nb = nb;
+  p.per = nb <= kSymSingle ? 1 : (nb <= 256 ? 2 : 4);
+  p.chunks = (nb + p.per - 1) / p.per;
+}
+static size_t sym_doubles(const FFPlan& p, int npad) {
+  return ((size_t)p.nb * (p.nb - 1) / 2 * kSymBlock + (size_t)p.chunks * npad) * PART_SLOTS + npad;
+}
+
+static FFPlan ff_plan(int device, int n, const Classes& cls, int npad) {
+  FFPlan p;
+  const int nb = (cls.nm == n ? n + kSymBlock - 1 : cls.nm) / kSymBlock;
+  if (nb >= kSymMin / kSymBlock && nb <= kSymMax / kSymBlock) {
+    sym_shape(p, nb);
+    p.from = nb * kSymBlock;
+  }
+  const int sources = cls.nm + cls.n_spl;
+  if (p.nb == 0) {
+    p.chunk1 = ff_chunk(device, n, n);
+    p.n1 = (n + p.chunk1 - 1) / p.chunk1;
+  } else if (p.from < n) {
+    if (sources > p.from) {
+      p.chunk1 = ff_chunk(device, n, sources - p.from);
+      p.n1 = (sources - p.from + p.chunk1 - 1) / p.chunk1;
+    }
+    p.chunk2 = ff_chunk(device, n - p.from, p.from);
+    p.n2 = (p.from + p.chunk2 - 1) / p.chunk2;
+  }
+  size_t o = 0;
+  auto take = [&](size_t doubles) {
+    const size_t at = o;
+    o += doubles;
+    return at;
+  };
+  p.o_j = take((size_t)p.nb * (p.nb > 0 ? p.nb - 1 : 0) / 2 * kSymBlock * PART_SLOTS);
+  p.o_i = take((size_t)p.chunks * PART_SLOTS * npad);
+  p.o_1 = take((size_t)p.n1 * PART_SLOTS * npad);
+  p.o_2 = take((size_t)p.n2 * PART_SLOTS * npad);
+  p.o_bound = take(p.nb > 0 ? npad : 0);
+  p.doubles = o;
+  return p;
 }
 
 // Sinks per CTA and summing warps of k_gravity_ac_ref: the CTAs spread over
@@ -1379,8 +1522,20 @@ static int force_launch(sol_ctx* c, const ForceCtx& fc, const double* d_y, doubl
                         uint32_t flags, int parts, int* d_clear) {
   const int nsink = sol_sink_hi(fc) - fc.sink_lo;
   const int split = (c->precision != SOL_PRECISION_FP64 && !c->barycentric) ? 1 : 0;
-  // SPLIT_FF systems beyond the warp-per-sink kernel run k_pairs_ff on the float table
+  // SPLIT_FF systems beyond the warp-per-sink kernel run on the float table
   const int ff2d = split && c->precision == SOL_PRECISION_SPLIT_FF && sol_force_uses_chunk_partials(c, c->precision);
+  FFPlan plan;
+  float* bound = nullptr;
+  if (split && sol_force_uses_chunk_partials(c, c->precision)) {
+    if (!c->d_part) {
+      sol_set_error("split precision selected without sol_set_precision");
+      return SOL_ERR_STATE;
+    }
+    if (ff2d) {
+      plan = ff_plan(c->device, c->n, c->cls, fc.npad);
+      if (plan.nb > 0) bound = reinterpret_cast<float*>(c->d_part + plan.o_bound);
+    }
+  }
   if (parts & 1) {
     const int nb_pre = (fc.npad + kPrepassBlock - 1) / kPrepassBlock;
     k_prepass<<<nb_pre, kPrepassBlock, 0, c->stream>>>(fc, d_y, split, ff2d, d_clear);
@@ -1390,7 +1545,7 @@ static int force_launch(sol_ctx* c, const ForceCtx& fc, const double* d_y, doubl
       SOL_LAUNCHED();
     }
     if (ff2d) {
-      k_split_table<<<nb_pre, kPrepassBlock, 0, c->stream>>>(fc, d_y);
+      k_split_table<<<nb_pre, kPrepassBlock, 0, c->stream>>>(fc, d_y, bound);
       SOL_LAUNCHED();
     }
   }
@@ -1412,20 +1567,46 @@ static int force_launch(sol_ctx* c, const ForceCtx& fc, const double* d_y, doubl
     return SOL_OK;
   }
   if (split) {
-    if (!c->d_part) {
-      sol_set_error("split precision selected without sol_set_precision");
-      return SOL_ERR_STATE;
+    int* status = &c->d_ctrl->dev_status;
+    if (c->precision == SOL_PRECISION_SPLIT_FF) {
+      if (plan.nb > 0) {
+        static std::atomic<int> sym_ready[kMaxDevices];
+        const int dev = (c->device >= 0 && c->device < kMaxDevices) ? c->device : 0;
+        if (!sym_ready[dev].load(std::memory_order_acquire)) {
+          SOL_CUDA(cudaFuncSetAttribute(k_pairs_sym, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)sizeof(SymShared)));
+          sym_ready[dev].store(1, std::memory_order_release);
+        }
+        k_near_bound<<<dim3(plan.nb, plan.nb < kBoundBlocks ? plan.nb : kBoundBlocks), kSymBlock, 0, c->stream>>>(
+            fc, bound, plan.nb);
+        SOL_LAUNCHED();
+        const int tasks = sym_tasks_above(plan.chunks, plan.per) + plan.nb;
+        k_pairs_sym<<<tasks, kSymThreads, sizeof(SymShared), c->stream>>>(
+            fc, d_y, c->d_part + plan.o_i, c->d_part + plan.o_j, bound, plan.nb, plan.per);
+        SOL_LAUNCHED();
+      }
+      if (plan.n1 > 0) {
+        k_pairs_ff<<<dim3(nb, plan.n1), kSinkBlock, 0, c->stream>>>(fc, d_y, c->d_part + plan.o_1, status,
+                                                                    plan.chunk1, plan.from, c->n);
+        SOL_LAUNCHED();
+      }
+      if (plan.n2 > 0 && sol_sink_hi(fc) > plan.from) {
+        ForceCtx rest = fc;
+        rest.sink_lo = fc.sink_lo > plan.from ? fc.sink_lo : plan.from;
+        rest.sink_hi = sol_sink_hi(fc);
+        const int nb2 = (rest.sink_hi - rest.sink_lo + kSinkBlock - 1) / kSinkBlock;
+        k_pairs_ff<<<dim3(nb2, plan.n2), kSinkBlock, 0, c->stream>>>(rest, d_y, c->d_part + plan.o_2, status,
+                                                                     plan.chunk2, 0, plan.from);
+        SOL_LAUNCHED();
+      }
+    } else {
+      plan.chunk1 = kChunk;
+      plan.n1 = (c->n + kChunk - 1) / kChunk;
+      k_pairs<SOL_PRECISION_SPLIT><<<dim3(nb, plan.n1), kSinkBlock, 0, c->stream>>>(fc, d_y, c->d_part, status, kChunk);
+      SOL_LAUNCHED();
     }
-    const int chunk = split_chunk(c, c->precision);
-    const int nchunk = (c->n + chunk - 1) / chunk;
-    dim3 grid(nb, nchunk);
-    if (c->precision == SOL_PRECISION_SPLIT_FF)
-      k_pairs_ff<<<grid, kSinkBlock, 0, c->stream>>>(fc, d_y, c->d_part, &c->d_ctrl->dev_status, chunk);
-    else
-      k_pairs<SOL_PRECISION_SPLIT><<<grid, kSinkBlock, 0, c->stream>>>(fc, d_y, c->d_part, &c->d_ctrl->dev_status,
-                                                                      chunk);
-    SOL_LAUNCHED();
-    k_combine<<<(nsink + 255) / 256, 256, 0, c->stream>>>(fc, d_y, d_dydt, c->d_part, nchunk, ts, flags);
+    k_combine<<<(nsink + kCombineSinks - 1) / kCombineSinks, kCombineSinks * kCombineWarps, 0, c->stream>>>(
+        fc, d_y, d_dydt, c->d_part, plan, ts, flags);
   } else {
     k_gravity_ac<SOL_PRECISION_FP64><<<nb, kSinkBlock, 0, c->stream>>>(fc, d_y, d_dydt, ts, flags,
                                                                        &c->d_ctrl->dev_status, SOL_SPIN_LIMIT, -1);
@@ -1455,12 +1636,29 @@ int sol_force_launch_sinks(sol_ctx* c, const double* d_y, double* d_dydt, TimeSp
 
 int sol_force_tile() { return kTile; }
 int sol_force_src_doubles() { return kSrcDoubles; }
-// chunk partials for either split form's 2-D kernel
-int sol_force_part_doubles(const sol_ctx* c) {
-  const int a = (c->n + kChunk - 1) / kChunk;
-  const int ff = split_chunk(c, SOL_PRECISION_SPLIT_FF);
-  const int b = (c->n + ff - 1) / ff;
-  return (a > b ? a : b) * PART_SLOTS * c->npad;
+// Partials for either split form's 2-D kernels, of this system and of every
+// smaller one it can become (removed bodies): fewer blocks can have more
+// chunks.
+size_t sol_force_part_doubles(const sol_ctx* c) {
+  const size_t np = c->npad;
+  size_t most = (size_t)((c->n + kChunk - 1) / kChunk) * PART_SLOTS * np;  // SPLIT
+  // k_pairs_ff alone: the number of chunks changes at whole sink blocks only
+  for (int n = (c->n + kSinkBlock - 1) / kSinkBlock * kSinkBlock; n >= 1; n -= kSinkBlock) {
+    const int ch = ff_chunk(c->device, n, n);
+    const size_t d = (size_t)((n + ch - 1) / ch) * PART_SLOTS * np;
+    if (d > most) most = d;
+  }
+  const int top = (c->cls.nm + kSymBlock - 1) / kSymBlock;
+  size_t sym = 0;
+  for (int nb = kSymMin / kSymBlock; nb <= top && nb <= kSymMax / kSymBlock; ++nb) {
+    FFPlan p;
+    sym_shape(p, nb);
+    const size_t d = sym_doubles(p, c->npad);
+    if (d > sym) sym = d;
+  }
+  if (sym > 0 && c->cls.nm < c->n)  // k_pairs_ff on the rest, in chunks of one tile at the least
+    sym += ((size_t)(kSymBlock + c->cls.n_spl + kTile - 1) / kTile + top) * PART_SLOTS * np;
+  return sym > most ? sym : most;
 }
 // whether the split forms of this system run the 2-D kernel (and need its
 // chunk partials); the same test as the dispatch in sol_force_launch_parts
@@ -1485,6 +1683,7 @@ constexpr int kNoAllocPrepassBlocks = kNoAllocMaxBodies / kPrepassBlock;
 constexpr size_t kNoAllocSrc = (size_t)SRC_ARRAYS * kNoAllocMaxBodies;
 constexpr size_t kNoAllocPart = 6 * (size_t)kNoAllocPrepassBlocks;
 constexpr size_t kNoAllocDoubles = kNoAllocSrc + kNoAllocPart + 8 /* sums */ + 8 /* status */;
+static_assert(kSymBlock == kTile && kTile % kSinkBlock == 0, "blocks of sources are whole tiles, tiles whole sink blocks");
 static_assert(kNoAllocMaxBodies % kTile == 0, "scratch must hold whole tiles");
 }  // namespace
 

@@ -294,7 +294,8 @@ __device__ __forceinline__ void f2_ff_r2(const float2* h, const float2* l, float
 // two cross terms, stays within 3 2^-24 of the high word, and the
 // accumulation that takes it multiplies it by the displacement with one
 // rounding (f2_ff_accumulate).
-__device__ __forceinline__ void f2_ff_gm_rinv3(float2 qh, float2 ql, float2 gh, float2 gl, float2& sh, float2& se) {
+// (f2_ff_rinv3 gives r^-3, f2_ff_scale its product with G m.)
+__device__ __forceinline__ void f2_ff_rinv3(float2 qh, float2 ql, float2& Rh, float2& Rl) {
   const float2 y = make_float2(sol_rsqrt_normal(qh.x), sol_rsqrt_normal(qh.y));
   float2 y2, y2e, q, qe;
   f2_two_prod(y, y, y2, y2e);
@@ -304,10 +305,16 @@ __device__ __forceinline__ void f2_ff_gm_rinv3(float2 qh, float2 ql, float2 gh, 
   f2_two_prod(y2, y, y3h, y3e);
   y3e = f2_fma(y2e, y, y3e);
   const float2 c = f2_mul(e, f2_fma(f2_splat(1.875f), e, f2_splat(1.5f)));
-  float2 Rh, Rl;
   f2_fast_two_sum(y3h, f2_fma(y3h, c, y3e), Rh, Rl);
+}
+__device__ __forceinline__ void f2_ff_scale(float2 gh, float2 gl, float2 Rh, float2 Rl, float2& sh, float2& se) {
   f2_two_prod(gh, Rh, sh, se);
   se = f2_fma(gh, Rl, f2_fma(gl, Rh, se));
+}
+__device__ __forceinline__ void f2_ff_gm_rinv3(float2 qh, float2 ql, float2 gh, float2 gl, float2& sh, float2& se) {
+  float2 Rh, Rl;
+  f2_ff_rinv3(qh, ql, Rh, Rl);
+  f2_ff_scale(gh, gl, Rh, Rl, sh, se);
 }
 
 // A += s d without the final renormalisation: the caller renormalises

@@ -1,0 +1,422 @@
+// SPLIT_FF pairs of massive bodies, each unordered pair once (included by
+// sol_force.cu inside its namespace).
+//
+// A pair's displacement, r^2 and r^-3 are the same numbers seen from either
+// body (d changes its sign, exactly), and both bodies take a term from it:
+// G m_j r^-3 d on i, -G m_i r^-3 d on j.  k_pairs_ff forms them twice; here a
+// pair costs 62 FP32 operations shared by its two terms and 42 for each term,
+// 73 a term instead of 106.5.
+//
+// Bodies are taken in blocks of 256.  A CTA has a block I of sinks, two a
+// thread (the two lanes of its paired FP32 instructions: a warp's 64 sinks),
+// and runs over the source blocks J >= I of a chunk.  Within a warp the 32
+// lanes work on 32 different sources at a time; a source's sums travel from
+// lane to lane by shuffles, past all 64 sinks in 32 steps, while its position
+// comes from shared memory.  The sinks' sums stay in registers.  After 32
+// steps the source's sums are added in FP64 to the CTA's partial of block J:
+// the warps work on different 32-source parts of J between two barriers, so
+// every sum has a fixed order.  k_combine adds a body's partials, as source
+// of the blocks below its own and as sink of its own block's chunks.  The block
+// itself (J = I) is evaluated as sinks alone, every source.
+//
+// The arithmetic of a term is k_pairs_ff's (sol_pair.cuh), with a sum folded
+// into FP64 every 128 (sink) or 32 (source) terms a lane instead of 128.
+// Either side of a block pair can be left out (a block of sinks alone,
+// sol_accel_sinks_device): what is computed keeps its order and so its bits.
+//
+// Bounded by the FP32 pipe: 73 operations a term are 7.8 ms at 65,536 bodies;
+// the kernel takes 10.7 (73 %), an evaluation 11.2 for 13.9 before, of 10,007
+// bodies 398 us for 455, of 16,384 0.80 ms for 0.99.  Its error against the
+// reference form is no larger: bodies of comparable pull on each other as from
+// the centre, 8,000 to 16,384 of them, 24 systems: median of the largest 1.5e-13
+// for 2.0e-13, rms 9.4e-15 for 1.0e-14.
+//
+// Pairs closer than the grid (ff_close_pair) leave their FP32 terms zero: the
+// sink takes the FP64 term at once, the source's side is marked and evaluated
+// after the block pair by a pass over it in source order (sym_close_pass).
+
+constexpr int kSymBlock = 256;                   // bodies per block, and sources per tile
+constexpr int kSymWarps = kSymBlock / 64;        // two sinks a thread
+constexpr int kSymThreads = 32 * kSymWarps;
+// Four CTAs an SM (128 registers): measured at 65,536 bodies 10.7 ms against
+// 11.3 with three (144 registers), and 11.3 against 12.1 before the bounds of
+// k_near_bound; one source at a time a warp -- two interleaved take 160
+// registers and three CTAs -- 12.0.
+constexpr int kSymCtas = 4;
+
+// A source's table entries, each twice (both lanes of a paired operand), two
+// to a 16-byte load.
+constexpr int kSymRows = (kFF + 1) / 2;
+struct SymTile {
+  float4 v[kSymRows][kSymBlock];
+};
+struct SymSource {
+  float2 v[2 * kSymRows];
+};
+__device__ __forceinline__ SymSource sym_load(const SymTile& T, int q) {
+  SymSource s;
+#pragma unroll
+  for (int k = 0; k < kSymRows; ++k) {
+    const float4 w = T.v[k][q];
+    s.v[2 * k] = make_float2(w.x, w.y);
+    s.v[2 * k + 1] = make_float2(w.z, w.w);
+  }
+  return s;
+}
+struct SymShared {
+  SymTile tile;
+  double js[3][kSymBlock];  // sums of the sources of J
+  float jmh[kSymBlock], jml[kSymBlock];  // their nearest sink of I
+  int jnn[kSymBlock];
+  int close;
+  // a thread's FP64 sums of its two sinks: totals, compensation, close pairs
+  // (here, not in registers: they change every 128 sources only)
+  double sums[3][6][kSymThreads];
+};
+
+// Nearest neighbour of one body: the smallest r^2 (hi, then lo), ties to the lower index.
+struct SymNear {
+  float h, l;
+  int j;
+};
+__device__ __forceinline__ void sym_near(SymNear& m, float h, float l, bool ok, int j) {
+  const bool better = ok & ((h < m.h) | ((h == m.h) & ((l < m.l) | ((l == m.l) & ((unsigned)j < (unsigned)m.j)))));
+  m.h = better ? h : m.h;
+  m.l = better ? l : m.l;
+  m.j = better ? j : m.j;
+}
+
+struct SymSinks {  // the thread's two sinks
+  float2 a[3], b[3], c[3];  // grid triples
+  float2 gh, gl;            // -G m
+  int i0, i1;
+};
+struct SymSums {
+  float2 h[3], l[3];
+};
+
+__device__ __forceinline__ float2 sym_shift(float2 v, int from) {
+  return make_float2(__shfl_sync(0xFFFFFFFFu, v.x, from), __shfl_sync(0xFFFFFFFFu, v.y, from));
+}
+
+// d, r^2 of one source and both sinks
+__device__ __forceinline__ void sym_displacement(const SymSource& J, const SymSinks& S, float2* h, float2* l,
+                                                 float2& r2h, float2& r2l) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float2 s1 = f2_sub(J.v[FAX + 3 * k], S.a[k]);
+    const float2 s2 = f2_sub(J.v[FBX + 3 * k], S.b[k]);
+    const float2 s3 = f2_sub(J.v[FCX + 3 * k], S.c[k]);
+    float2 l0;
+    f2_fast_two_sum(s1, s2, h[k], l0);
+    l[k] = f2_add(l0, s3);
+  }
+  f2_ff_r2(h, l, r2h, r2l);
+}
+
+// A source's nearest sink in the CTA's shared arrays: read always, written
+// when a sink is nearer (about ln N times)
+__device__ __forceinline__ void sym_near_source(SymShared& sm, int q, const SymSinks& S, int ns, float2 r2h,
+                                                float2 r2l) {
+  SymNear m = {sm.jmh[q], sm.jml[q], sm.jnn[q]};
+  sym_near(m, r2h.x, r2l.x, (S.i0 >= 1) & (S.i0 < ns), S.i0);
+  sym_near(m, r2h.y, r2l.y, (S.i1 >= 1) & (S.i1 < ns), S.i1);
+  sm.jmh[q] = m.h;
+  sm.jml[q] = m.l;
+  sm.jnn[q] = m.j;
+}
+
+// A step of a warp once d and r^2 are known: the terms into the sinks' sums A
+// and the source's travelling sums B.  The float-float sums are renormalised at
+// every second step (second).
+template <bool DI, bool DJ, bool SECOND>
+__device__ __forceinline__ void sym_terms(const float2* h, const float2* l, float2 qh, float2 ql, float2 gh, float2 gl,
+                                          float2 mh, float2 ml, int from, SymSums& A, SymSums& B) {
+  float2 Rh, Rl, sh, se;
+  f2_ff_rinv3(qh, ql, Rh, Rl);
+  if (DJ) {
+    f2_ff_scale(mh, ml, Rh, Rl, sh, se);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      f2_ff_accumulate_lazy(B.h[k], B.l[k], sh, se, h[k], l[k]);
+      if (SECOND) f2_fast_two_sum(B.h[k], B.l[k], B.h[k], B.l[k]);
+      // the source's sums move on with it
+      B.h[k] = sym_shift(B.h[k], from);
+      B.l[k] = sym_shift(B.l[k], from);
+    }
+  }
+  if (DI) {
+    f2_ff_scale(gh, gl, Rh, Rl, sh, se);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      f2_ff_accumulate_lazy(A.h[k], A.l[k], sh, se, h[k], l[k]);
+      if (SECOND) f2_fast_two_sum(A.h[k], A.l[k], A.h[k], A.l[k]);
+    }
+  }
+}
+
+template <bool DI, bool DJ, bool SECOND>
+__device__ __forceinline__ void sym_step(SymShared& sm, const ForceCtx& fc, const double* __restrict__ y, int q,
+                                         int from, int j0, int ns, float thr, const SymSinks& S, SymSums& A,
+                                         SymNear& n0, SymNear& n1, SymSums& B) {
+  float2 h[3], l[3], r2h, r2l;
+  const SymSource J = sym_load(sm.tile, q);
+  sym_displacement(J, S, h, l, r2h, r2l);
+  // (the whole warp takes one way: the sources' sums pass through shuffles)
+  if (__builtin_expect(!__any_sync(0xFFFFFFFFu, fminf(r2h.x, r2h.y) < thr), 1)) {
+    sym_terms<DI, DJ, SECOND>(h, l, r2h, r2l, J.v[FGH], J.v[FGL], S.gh, S.gl, from, A, B);
+  } else {
+    float2 qh = r2h, ql = r2l, gh = J.v[FGH], gl = J.v[FGL], mh = S.gh, ml = S.gl;
+    const int j = j0 + q;
+    if (r2h.x < thr) {
+      const double* p = y + 6 * (size_t)S.i0;
+      double f[3] = {0.0, 0.0, 0.0};
+      if (S.i0 < ns && j < ns) ff_close_pair(fc, j, p[0], p[1], p[2], gh.x, gl.x, f[0], f[1], f[2], r2h.x, r2l.x);
+      if (DI)
+        for (int k = 0; k < 3; ++k) sm.sums[2][k][threadIdx.x] += f[k];
+      gh.x = gl.x = mh.x = ml.x = ql.x = 0.0f;
+      qh.x = 1.0f;
+      sm.close = 1;
+    }
+    if (r2h.y < thr) {
+      const double* p = y + 6 * (size_t)S.i1;
+      double f[3] = {0.0, 0.0, 0.0};
+      if (S.i1 < ns && j < ns) ff_close_pair(fc, j, p[0], p[1], p[2], gh.y, gl.y, f[0], f[1], f[2], r2h.y, r2l.y);
+      if (DI)
+        for (int k = 0; k < 3; ++k) sm.sums[2][3 + k][threadIdx.x] += f[k];
+      gh.y = gl.y = mh.y = ml.y = ql.y = 0.0f;
+      qh.y = 1.0f;
+      sm.close = 1;
+    }
+    __syncwarp();
+    sym_terms<DI, DJ, SECOND>(h, l, qh, ql, gh, gl, mh, ml, from, A, B);
+  }
+  const bool near_i = DI && (r2h.x <= n0.h || r2h.y <= n1.h);
+  const bool near_j = DJ && fminf(r2h.x, r2h.y) <= sm.jmh[q];
+  if (near_i | near_j) {
+    if (DI) {
+      const int j = j0 + q;
+      const bool src = (j >= 1) & (j < ns);
+      sym_near(n0, r2h.x, r2l.x, src & (j != S.i0), j);
+      sym_near(n1, r2h.y, r2l.y, src & (j != S.i1), j);
+    }
+    if (DJ) sym_near_source(sm, q, S, ns, r2h, r2l);
+  }
+}
+
+// 32 steps of a warp: its 64 sinks past the 32 sources of part `sub` of the
+// tile.  DI / DJ: the sinks' / the sources' sums.
+template <bool DI, bool DJ>
+__device__ __forceinline__ void sym_part(SymShared& sm, const ForceCtx& fc, const double* __restrict__ y, int sub,
+                                         int lane, int j0, int ns, float thr, const SymSinks& S, SymSums& A,
+                                         SymNear& n0, SymNear& n1, SymSums& B) {
+  const int from = (lane + 1) & 31;
+#pragma unroll 1
+  for (int t = 0; t < 32; t += 2) {
+    sym_step<DI, DJ, false>(sm, fc, y, sub * 32 + ((lane + t) & 31), from, j0, ns, thr, S, A, n0, n1, B);
+    sym_step<DI, DJ, true>(sm, fc, y, sub * 32 + ((lane + t + 1) & 31), from, j0, ns, thr, S, A, n0, n1, B);
+    __syncwarp();
+  }
+}
+
+// The source side of the close pairs of a block pair, in sink order.
+__device__ __noinline__ void sym_close_pass(SymShared& sm, const ForceCtx& fc, const double* __restrict__ y, int i0,
+                                            int j0, int ns, float thr) {
+  const float* T = ftab(fc);
+  const int np = fc.npad;
+  for (int q = threadIdx.x; q < kSymBlock; q += kSymThreads) {
+    const int j = j0 + q;
+    if (j >= ns) continue;
+    const double* p = y + 6 * (size_t)j;
+    const SymSource J = sym_load(sm.tile, q);
+    double f[3] = {0.0, 0.0, 0.0};
+    for (int i = i0; i < min(i0 + kSymBlock, ns); ++i) {
+      float2 h[3], l[3], r2h, r2l;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const float2 s1 = f2_sub(J.v[FAX + 3 * k], f2_splat(T[(size_t)(FAX + 3 * k) * np + i]));
+        const float2 s2 = f2_sub(J.v[FBX + 3 * k], f2_splat(T[(size_t)(FBX + 3 * k) * np + i]));
+        const float2 s3 = f2_sub(J.v[FCX + 3 * k], f2_splat(T[(size_t)(FCX + 3 * k) * np + i]));
+        float2 l0;
+        f2_fast_two_sum(s1, s2, h[k], l0);
+        l[k] = f2_add(l0, s3);
+      }
+      f2_ff_r2(h, l, r2h, r2l);
+      if (!(r2h.x < thr)) continue;
+      float a, b;
+      ff_close_pair(fc, i, p[0], p[1], p[2], T[(size_t)FGH * np + i], T[(size_t)FGL * np + i], f[0], f[1], f[2], a, b);
+    }
+    for (int k = 0; k < 3; ++k) sm.js[k][q] += f[k];
+  }
+}
+
+// An upper bound of every body's squared distance to its nearest neighbour:
+// the smallest among the sources of its own block and the next ones
+// (kBoundBlocks in all), in FP32 from the grid triples' two leading parts
+// (relative error ~2^-22, covered by the factor).  A sink starts its search
+// there, so that a new minimum is rare (without it every block pair begins
+// with ~5 updates a body, and hardly a step of a warp has none).
+constexpr int kBoundBlocks = 4;
+__global__ void __launch_bounds__(kSymBlock) k_near_bound(ForceCtx fc, float* __restrict__ bound, int nb) {
+  __shared__ float2 sx[kSymBlock], sy[kSymBlock], sz[kSymBlock];
+  const float* T = ftab(fc);
+  const int np = fc.npad, ns = fc.cls.nm;
+  const int i = blockIdx.x * kSymBlock + threadIdx.x;
+  const int j0 = ((blockIdx.x + blockIdx.y) % nb) * kSymBlock;
+  auto at = [&](int k, int j) {
+    return make_float2(T[(size_t)(FAX + 3 * k) * np + j], T[(size_t)(FBX + 3 * k) * np + j]);
+  };
+  const float2 x = at(0, i), yy = at(1, i), z = at(2, i);
+  sx[threadIdx.x] = at(0, j0 + threadIdx.x);
+  sy[threadIdx.x] = at(1, j0 + threadIdx.x);
+  sz[threadIdx.x] = at(2, j0 + threadIdx.x);
+  __syncthreads();
+  float m = 3.0e38f;
+  const int q1 = min(kSymBlock, ns - j0);
+#pragma unroll 8
+  for (int q = j0 == 0 ? 1 : 0; q < q1; ++q) {
+    const float dx = (sx[q].x - x.x) + (sx[q].y - x.y), dy = (sy[q].x - yy.x) + (sy[q].y - yy.y),
+                dz = (sz[q].x - z.x) + (sz[q].y - z.y);
+    const float r2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
+    m = (j0 + q != i && r2 < m) ? r2 : m;
+  }
+  // k_split_table set 3e38; the order of floats that are not negative is that of their bits
+  atomicMin(reinterpret_cast<int*>(bound) + i, __float_as_int(fminf(m * 1.0001f + 1.0e-37f, 3.0e38f)));
+}
+
+// part_i: [chunk][PART_SLOTS][npad] as k_pairs_ff's; part_j: per block pair
+// I < J, packed by I, [PART_SLOTS][kSymBlock].
+__device__ __forceinline__ size_t sym_pair_index(int I, int J, int nb) {
+  return (size_t)I * (nb - 1) - (size_t)I * (I - 1) / 2 + (J - I - 1);
+}
+
+// CTAs of chunks 0 .. C - 1 whose sinks lie in blocks below the chunk's: chunk c
+// has per c of them.
+__host__ __device__ __forceinline__ int sym_tasks_above(int C, int per) { return per * (C * (C - 1) / 2); }
+
+__global__ void __launch_bounds__(kSymThreads, kSymCtas)
+    k_pairs_sym(ForceCtx fc, const double* __restrict__ y, double* __restrict__ part_i, double* __restrict__ part_j,
+                const float* __restrict__ bound, int nb, int per) {
+  extern __shared__ __align__(16) unsigned char sym_dyn[];
+  SymShared& sm = *reinterpret_cast<SymShared*>(sym_dyn);
+  // The CTA's block of sinks I and its chunk C of `per` blocks of sources: first
+  // the chunks above I's own, by chunk, then the nb of I's own, whose diagonal
+  // block takes less, so that the last to start are short.  No CTA is launched
+  // for nothing: on a grid of I x C whose lower half returned at once the CTAs
+  // left gathered on some of the SMs (10,007 bodies: 529 us an evaluation, 424
+  // on this one).
+  const int task = blockIdx.x;
+  const int above = sym_tasks_above((nb + per - 1) / per, per);
+  int I, C;
+  if (task < above) {
+    C = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)(task / per))) * 0.5f);
+    while (sym_tasks_above(C, per) > task) --C;
+    while (sym_tasks_above(C + 1, per) <= task) ++C;
+    I = task - sym_tasks_above(C, per);
+  } else {
+    I = task - above;
+    C = I / per;
+  }
+  const int Jlo = max(I, C * per), Jhi = min(nb, (C + 1) * per);
+  const int np = fc.npad, ns = fc.cls.nm;
+  const int lo = fc.sink_lo, hi = sol_sink_hi(fc);
+  auto wanted = [&](int B) { return B * kSymBlock < hi && (B + 1) * kSymBlock > lo; };
+  const bool want_i = wanted(I);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float* T = ftab(fc);
+  SymSinks S;
+  S.i0 = I * kSymBlock + warp * 64 + lane;
+  S.i1 = S.i0 + 32;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    S.a[k] = make_float2(T[(size_t)(FAX + 3 * k) * np + S.i0], T[(size_t)(FAX + 3 * k) * np + S.i1]);
+    S.b[k] = make_float2(T[(size_t)(FBX + 3 * k) * np + S.i0], T[(size_t)(FBX + 3 * k) * np + S.i1]);
+    S.c[k] = make_float2(T[(size_t)(FCX + 3 * k) * np + S.i0], T[(size_t)(FCX + 3 * k) * np + S.i1]);
+  }
+  S.gh = make_float2(-T[(size_t)FGH * np + S.i0], -T[(size_t)FGH * np + S.i1]);
+  S.gl = make_float2(-T[(size_t)FGL * np + S.i0], -T[(size_t)FGL * np + S.i1]);
+  const double G1 = fc.ind_sum[kIndGrid];
+  const float thr = fmaxf((float)(G1 * G1), 7.888609052210118e-31f);  // as k_pairs_ff
+  for (int k = 0; k < 18; ++k) sm.sums[k / 6][k % 6][threadIdx.x] = 0.0;
+  SymNear n0 = {bound[S.i0], 3.0e38f, -1}, n1 = {bound[S.i1], 3.0e38f, -1};
+  for (int J = Jlo; J < Jhi; ++J) {
+    const bool want_j = J != I && wanted(J);
+    if (!want_i && !want_j) continue;
+    const int j0 = J * kSymBlock;
+    __syncthreads();
+#pragma unroll 1
+    for (int k = 0; k < kSymRows; ++k)
+      for (int q = threadIdx.x; q < kSymBlock; q += kSymThreads) {
+        const float v = T[(size_t)(2 * k) * np + j0 + q];
+        const float w = 2 * k + 1 < kFF ? T[(size_t)(2 * k + 1) * np + j0 + q] : 0.0f;
+        sm.tile.v[k][q] = make_float4(v, v, w, w);
+      }
+    for (int q = threadIdx.x; q < kSymBlock; q += kSymThreads) {
+      sm.js[0][q] = sm.js[1][q] = sm.js[2][q] = 0.0;
+      sm.jmh[q] = bound[j0 + q];
+      sm.jml[q] = 3.0e38f;
+      sm.jnn[q] = -1;
+    }
+    if (threadIdx.x == 0) sm.close = 0;
+    __syncthreads();
+    SymSums A;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) A.h[k] = A.l[k] = make_float2(0.0f, 0.0f);
+#pragma unroll 1
+    for (int p = 0; p < 8; ++p) {
+      const int sub = (p + 2 * warp) & 7;  // a part of its own for every warp
+      const int q = sub * 32 + lane;
+      SymSums B;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) B.h[k] = B.l[k] = make_float2(0.0f, 0.0f);
+      if (want_i && want_j)
+        sym_part<true, true>(sm, fc, y, sub, lane, j0, ns, thr, S, A, n0, n1, B);
+      else if (want_i)
+        sym_part<true, false>(sm, fc, y, sub, lane, j0, ns, thr, S, A, n0, n1, B);
+      else
+        sym_part<false, true>(sm, fc, y, sub, lane, j0, ns, thr, S, A, n0, n1, B);
+      if (want_j) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          sm.js[k][q] += ((double)B.h[k].x + (double)B.l[k].x) + ((double)B.h[k].y + (double)B.l[k].y);
+      }
+      if (want_i && (p & 3) == 3) {  // the sinks' float-float sums of 128 sources into FP64
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          double* t = &sm.sums[0][k][threadIdx.x];
+          double* c = &sm.sums[1][k][threadIdx.x];
+          two_sum(t[0], c[0], (double)A.h[k].x + (double)A.l[k].x);
+          two_sum(t[3 * kSymThreads], c[3 * kSymThreads], (double)A.h[k].y + (double)A.l[k].y);
+          A.h[k] = A.l[k] = make_float2(0.0f, 0.0f);
+        }
+      }
+      __syncthreads();
+    }
+    if (want_j) {
+      if (sm.close) {
+        sym_close_pass(sm, fc, y, I * kSymBlock, j0, ns, thr);
+        __syncthreads();
+      }
+      double* out = part_j + sym_pair_index(I, J, nb) * PART_SLOTS * kSymBlock;
+      for (int q = threadIdx.x; q < kSymBlock; q += kSymThreads) {
+        out[PAX * kSymBlock + q] = sm.js[0][q];
+        out[PAY * kSymBlock + q] = sm.js[1][q];
+        out[PAZ * kSymBlock + q] = sm.js[2][q];
+        out[PR2 * kSymBlock + q] = sm.jnn[q] >= 0 ? (double)sm.jmh[q] + (double)sm.jml[q] : 1.0e300;
+        out[PIDX * kSymBlock + q] = __longlong_as_double((long long)sm.jnn[q]);
+      }
+    }
+  }
+  if (!want_i) return;
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const SymNear& m = u ? n1 : n0;
+    double* out = part_i + (size_t)C * PART_SLOTS * np + (u ? S.i1 : S.i0);
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      out[(size_t)(PAX + k) * np] = (sm.sums[0][3 * u + k][threadIdx.x] + sm.sums[1][3 * u + k][threadIdx.x]) +
+                                    sm.sums[2][3 * u + k][threadIdx.x];
+    out[(size_t)PR2 * np] = m.j >= 0 ? (double)m.h + (double)m.l : 1.0e300;
+    out[(size_t)PIDX * np] = __longlong_as_double((long long)m.j);
+  }
+}
