@@ -1,125 +1,88 @@
 // Correctly rounded r = sqrt(a) and r^-3 = 1 / (a * r) for the reference-form
 // pair (GravityAC, Acceleration.cpp:294-317: rij = sqrt(rij2),
-// rijm3 = 1.0 / (rij2 * rij)) with two FP64 instructions besides the product
+// rijm3 = 1.0 / (rij2 * rij)) with no FP64 instruction besides the product
 // a * r, bit-identical to IEEE sqrt and division.
 //
 // The GPU's FP64 pipe issues one warp instruction per 64 cycles per
 // sub-partition; IEEE square root and division take about sixteen of them
 // per pair, so they, not the twenty-one additions and multiplications of the
 // pair, bound the reference form.  Here the approximations come from the FP32
-// and integer pipes and FP64 only measures the remainders:
+// pipe and the remainders are measured on the integer pipe:
 //
 //  1. a = m 4^k with m in [1, 4).  From an FP32 rsqrt seed y and one Newton
 //     correction evaluated with exact products (TwoProduct by FMA) come
 //     float-float approximations (relative error ~2^-45) of m^-1/2, of
 //     m^1/2 and of m^-3/2.
-//  2. Integer operations on the bit patterns turn them into doubles
-//     q0 ~ sqrt(a) and z0 ~ 1/d (d = RN(a r)), a few hundred ulps at most
-//     from the exact values.
-//  3. One FMA gives each remainder, a - q0^2 and 1 - d z0, to full
-//     precision (its rounding error is 2^-53 of itself).  The remainder over
-//     the derivative, in float-float, is the distance of the exact result
-//     from q0 (z0) in units in the last place, to ~2^-35 ulp; rounding it to
-//     the nearest integer and adding that to the bit pattern gives the
-//     correctly rounded result.  This is the remainder-based rounding
-//     decision of Markstein (IA-64 and Elementary Functions, 2000, ch. 8;
-//     Tuckerman's test for the square root), with the remainder measured
-//     rather than only its sign.
+//  2. They become 53-bit integers Q ~ m^1/2 2^52 and Z ~ 1/d (d = RN(a r),
+//     scaled), at most ~350 and ~1,150 units from the exact values.
+//  3. The remainders m 2^104 - Q^2 and 2^105 - D Z (D the significand of d)
+//     are small, so the words of the products in their middle are enough:
+//     the remainder over 2 Q (over D), times m^-1/2 (times Z) as 31-bit fixed
+//     point, is the distance of the exact result from Q (Z) in units in the
+//     last place, to 2^-18 (2^-17) unit; rounding it to the nearest integer
+//     and adding that gives the correctly rounded result.  This is the
+//     remainder-based rounding decision of Markstein (IA-64 and Elementary
+//     Functions, 2000, ch. 8; Tuckerman's test for the square root), with the
+//     remainder measured rather than only its sign.
 //
 // Neither quotient can fall exactly on a midpoint between doubles (a
 // midpoint needs 54 significant bits; its square, or its product with a
 // 53-bit d, cannot be a double, resp. 1).  Where the measured distance lies
-// within 2^-16 ulp of a midpoint (probability ~2^-15 per function), where
-// it exceeds 2^20 ulp (an approximation gone astray), where the result would
-// land on or cross a power of two, or where a is outside [2^-600, 2^600]
-// (zero, denormal, infinite or NaN included) the fast path reports failure
-// and the caller takes IEEE sqrt and division, so the result is the
-// correctly rounded one in every case.
+// within 2^-16 ulp of a midpoint (probability 2^-15 per function), where a
+// distance exceeds its range, where the result would lie next to a power of
+// two, or where a is outside [2^-600, 2^600] (zero, denormal, infinite or NaN
+// included) the fast path reports failure and the caller takes IEEE sqrt and
+// division, so the result is the correctly rounded one in every case.
+//
+// With the remainders by FP64 FMA (two of a pair's 14.7 FP64 instructions, and
+// their conversions to float-float) an evaluation of 16,411 bodies took 7.96 ms
+// for 7.01, of 2,049 173 us for 156.
 #pragma once
 
 #include "sol_pair.cuh"
 
 namespace solcr {
 
-constexpr float kMidTol = 0.5f - 1.52587890625e-05f;  // 0.5 - 2^-16: beyond it the rounding is decided exactly
-
-// (h, l) floats, h > 0 normal, |l| <= ulp(h)/2, scaled by 2^escale -> the bit
-// pattern of a double within one ulp of (h + l) 2^escale.  The 53-bit
-// significand is built as an integer; when a negative l takes it below 2^52
-// (h a power of two) it is shifted up one place and the exponent lowered, and
-// |l| <= ulp(h)/2 keeps the sum below the next power of two.
-__device__ __forceinline__ long long ff_to_double_bits(float h, float l, int escale) {
-  const unsigned hb = __float_as_uint(h);
-  const int eh = (int)(hb >> 23);  // h > 0
-  const unsigned mh = (hb & 0x7FFFFFu) | 0x800000u;
-  const unsigned lb = __float_as_uint(l);
-  const int el = (int)((lb >> 23) & 0xFFu);
-  const unsigned ml = el ? ((lb & 0x7FFFFFu) | 0x800000u) : 0u;
-  const int sh = el - eh + 29;  // l's unit in units of 2^(E_h - 52); <= 5
-  unsigned long long add = 0;
-  if (sh >= 0)
-    add = (unsigned long long)ml << sh;
-  else if (sh > -32)
-    add = (unsigned long long)(ml >> (-sh));
-  long long m = ((long long)mh << 29);
-  m = (lb & 0x80000000u) ? m - (long long)add : m + (long long)add;
-  const bool low = m < (1LL << 52);
-  m = low ? (m << 1) : m;
-  return ((long long)(eh - 127 + 1023 + escale - (low ? 1 : 0)) << 52) + (m - (1LL << 52));
+// h + l (floats, |l| <= ulp(h)) in units of 2^(e - 52), as an integer; h_units:
+// h in units of 2^(e - 23), unit: 2^(52 - e).
+__device__ __forceinline__ long long ff_significand(unsigned h_units, float l, float unit) {
+  return ((long long)h_units << 29) + (long long)__float2int_rn(l * unit);
 }
 
-// d 2^sh -> (h, l) floats from the bit pattern (h: the leading 24 bits
-// truncated, l: the next 29 rounded to 24).  Scaled values below 2^-74 give
-// 0 (the callers scale remainders to distances in ulps, where 2^-74 is
-// nothing); ok turns false if the scaled value is too large.
-__device__ __forceinline__ void double_to_ff_scaled(double d, int sh, float& h, float& l, bool& ok) {
-  const unsigned hi = (unsigned)__double2hiint(d);
-  const unsigned lo = (unsigned)__double2loint(d);
-  const int e = (int)((hi >> 20) & 0x7FFu);
-  const unsigned sign = hi & 0x80000000u;
-  const int ef = e - 1023 + sh + 127;  // biased float exponent of h
-  ok = ok && (ef < 200);
-  const bool live = (e != 0) && (ef >= 53);
-  h = live ? __uint_as_float(sign | ((unsigned)ef << 23) | ((hi & 0x000FFFFFu) << 3) | (lo >> 29)) : 0.0f;
-  const float scale = live ? __uint_as_float((unsigned)(ef - 52) << 23) : 0.0f;
-  l = __uint_as_float(__float_as_uint(__uint2float_rn(lo & 0x1FFFFFFFu) * scale) | sign);
+// t: a distance in units of 2^-B ulp.  The nearest whole number of ulps; ok
+// turns false within 2^-16 ulp of a midpoint.
+template <int B>
+__device__ __forceinline__ int round_distance(int t, bool& ok) {
+  const int u = t + (1 << (B - 1));
+  ok = ok & ((unsigned)(u & ((1 << B) - 1)) - (1u << (B - 16)) <= (1u << B) - (2u << (B - 16)));
+  return u >> B;
 }
 
-// Nearest integer n to (h + l), and whether it is decided: |h| < 2^20 (the
-// approximations are within a few hundred ulps; anything else goes to the
-// IEEE path) and |h + l - n| <= 0.5 - 2^-16.
-__device__ __forceinline__ int round_ff(float h, float l, bool& ok) {
-  const float t = h + 12582912.0f;  // 1.5 * 2^23: the sum rounds h to an integer
-  const int n = __float_as_int(t) - 0x4B400000;
-  const float frac = (h - (t - 12582912.0f)) + l;
-  ok = ok && (fabsf(frac) <= kMidTol) && (fabsf(h) < 1048576.0f);
-  return n;
+// The double with significand S (2^52 < S < 2^53) and exponent e; ok turns
+// false for a significand outside (a power of two, or a result in the next
+// binade, which would round in other units).
+__device__ __forceinline__ double from_significand(long long S, int e, bool& ok) {
+  const unsigned hi = (unsigned)(S >> 32), lo = (unsigned)S;
+  ok = ok & (hi - 0x100000u < 0x100000u) & (((hi ^ 0x100000u) | lo) != 0u);
+  return __hiloint2double((int)(hi + ((unsigned)(e + 1022) << 20)), (int)lo);
 }
 
-// The correctly rounded neighbour q0 + n ulp, unless that needs another
-// binade (the ulp used for n is q0's) or is a power of two.
-__device__ __forceinline__ long long step_ulps(long long qb, int n, bool& ok) {
-  const long long rb = qb + (long long)n;
-  ok = ok && (((rb ^ qb) >> 52) == 0) && ((rb & 0xFFFFFFFFFFFFFLL) != 0);
-  return rb;
-}
-
-// The correctly rounded 1/d from the bit pattern zb of an approximation
-// z0 within a few hundred ulps of it: the distance (1/d - z0) / ulp(z0) =
-// (1 - d z0) z0 / ulp(z0) (1 + O(2^-40)), z0 / ulp(z0) being its significand
-// in [1, 2) times 2^52.
-__device__ __forceinline__ long long rcp_from_approx(double d, long long zb, bool& ok) {
-  const double z0 = __longlong_as_double(zb);
-  const double er = __fma_rn(-d, z0, 1.0);
-  const unsigned hiZ = (unsigned)(zb >> 32);
-  const unsigned loZ = (unsigned)zb;
-  const float zh = __uint_as_float(0x3F800000u | ((hiZ & 0x000FFFFFu) << 3) | (loZ >> 29));
-  const float zl = __uint2float_rn(loZ & 0x1FFFFFFFu) * 2.220446049250313e-16f;  // 2^-52
-  float eh, el;
-  double_to_ff_scaled(er, 52, eh, el, ok);
-  const float ph = eh * zh;
-  const float pl = __fmaf_rn(eh, zh, -ph) + __fmaf_rn(eh, zl, el * zh);
-  return step_ulps(zb, round_ff(ph, pl, ok), ok);
+// The correctly rounded 1/d from an approximation Z 2^(ez - 52).  With D the
+// significand of d, 2^105 - D Z over D is its distance in units of Z; of the
+// product bits 32 to 95 are formed (the rest is known), their 32 from bit 33
+// on are the remainder where the distance is below 2^11.
+__device__ __forceinline__ double rcp_from_approx(double d, long long Z, int ez, bool& ok) {
+  const unsigned dh = (unsigned)__double2hiint(d), dl = (unsigned)__double2loint(d);
+  const unsigned Dh = (dh & 0xFFFFFu) | 0x100000u;
+  const unsigned Zl = (unsigned)Z, Zh = (unsigned)(Z >> 32);
+  const unsigned long long t1 = (unsigned long long)Dh * Zl + __umulhi(dl, Zl);
+  const unsigned long long t2 = (unsigned long long)dl * Zh + (unsigned)t1;
+  const unsigned t3 = Dh * Zh + (unsigned)(t1 >> 32) + (unsigned)(t2 >> 32);
+  const int v = -(int)__funnelshift_r((unsigned)t2, t3, 1);
+  // beyond 31 bits of remainder, or an approximation in the wrong binade
+  ok = ok & (t3 + 1u <= 1u) & ((int)(dh >> 20) - 1023 + ez == -1);
+  const int t = __mulhi(v, (int)(Z >> 22));  // v 2^33 / D = v Z 2^(33 - 105)
+  return from_significand(Z + (long long)round_distance<18>(t, ok), ez, ok);
 }
 
 }  // namespace solcr
@@ -130,7 +93,7 @@ __device__ __forceinline__ bool sol_ref_rinv3_fast(double a, double& rij, double
   const unsigned hiA = (unsigned)__double2hiint(a);
   const unsigned loA = (unsigned)__double2loint(a);
   const int E = (int)(hiA >> 20);  // the sign bit of a sum of squares is clear, NaN aside
-  bool ok = (E >= 1023 - 600) & (E <= 1023 + 600);
+  bool ok = (unsigned)(E - (1023 - 600)) <= 1200u;
   const int e2 = E - 1023;
   const int k = e2 >> 1;   // floor(e2 / 2)
   const int p = e2 - 2 * k;  // 0 or 1: m = a 4^-k in [1, 4)
@@ -163,25 +126,25 @@ __device__ __forceinline__ bool sol_ref_rinv3_fast(double a, double& rij, double
     ff_fast_two_sum(y3h, __fmaf_rn(y3h, c3, y3e), Rh, Rl);
   }
 
-  // ---- sqrt(a): q0 ~ m^1/2 2^k; distance = (a - q0^2) / (2 q0 ulp(q0)) ----
-  const long long qb = ff_to_double_bits(sh, sl, k);
-  const double q0 = __longlong_as_double(qb);
-  const double ea = __fma_rn(-q0, q0, a);
-  const int Eq = (int)(qb >> 52) - 1023;
-  // (a - q0^2) / (2 q0 2^(Eq-52)) = ea 2^(51-Eq-k) / (q0 2^-k) ~ ea 2^(51-Eq-k) m^-1/2
-  float eh, el;
-  double_to_ff_scaled(ea, 51 - Eq - k, eh, el, ok);
-  const float ph = eh * yh;
-  const float pl = __fmaf_rn(eh, yh, -ph) + __fmaf_rn(eh, yl, el * yh);
-  const long long rb = step_ulps(qb, round_ff(ph, pl, ok), ok);
-  const double r = __longlong_as_double(rb);
+  // ---- sqrt(a) = q 2^k: Q ~ m^1/2 2^52, (m 2^104 - Q^2) / (2 Q) ----
+  // (sh in [1, 2], its bits linear there, 2 included)
+  const long long Q = ff_significand(__float_as_uint(sh) - 0x3F000000u, sl, 4503599627370496.0f);
+  const unsigned Ql = (unsigned)Q, Qh = (unsigned)(Q >> 32);
+  const int R = (int)((loA << (20 + p)) - __umulhi(Ql, Ql) - (Qh << 1) * Ql);  // bits 32 to 63, |R| < 2^31
+  // m^-1/2 = yh + yl in units of 2^-31 (not for yh = 1: m within 2^-24 of 1)
+  ok = ok & (yh < 1.0f);
+  const int yi = (int)(((__float_as_uint(yh) & 0x7FFFFFu) | 0x800000u) << 7) +
+                 (__float_as_int(__fmaf_rn(yl, 2147483648.0f, 12582912.0f)) - 0x4B400000);
+  const int t = __mulhi(R, yi);  // R 2^32 / (2 Q) = R 2^-21 m^-1/2
+  const double r = from_significand(Q + (long long)round_distance<20>(t, ok), k, ok);
 
-  // ---- 1/d, d = RN(a r): z0 ~ m^-3/2 2^-3k ----
+  // ---- 1/d, d = RN(a r): Z ~ m^-3/2 2^-3k ----
   const double d = a * r;
-  const long long wb = rcp_from_approx(d, ff_to_double_bits(Rh, Rl, -3 * k), ok);
-
+  const unsigned Rb = __float_as_uint(Rh);
+  const long long Z = ff_significand((Rb & 0x7FFFFFu) | 0x800000u, Rl,
+                                     __uint_as_float(((127u + 52u + 127u) << 23) - (Rb & 0x7F800000u)));
   rij = r;
-  rijm3 = __longlong_as_double(wb);
+  rijm3 = rcp_from_approx(d, Z, (int)(Rb >> 23) - 127 - 3 * k, ok);
   return ok;
 }
 
@@ -297,16 +260,4 @@ __device__ __forceinline__ void sol_ref_terms(double gm, double rijm3, double dx
 // IEEE arithmetic for a pair the fast paths hand over: |d| and 1 / (|d|^2 |d|)
 static __device__ __noinline__ double2 sol_ref_pair_ieee(double dx, double dy, double dz) {
   return sol_ref_rinv3_ieee(dx * dx + dy * dy + dz * dz);
-}
-
-// Two independent pairs in one basic block (their dependency chains
-// interleave), the rare IEEE fallbacks after both.
-__device__ __forceinline__ void sol_ref_rinv3_x2(double a0, double a1, double& r0, double& w0, double& r1,
-                                                 double& w1) {
-  const bool ok0 = sol_ref_rinv3_fast(a0, r0, w0);
-  const bool ok1 = sol_ref_rinv3_fast(a1, r1, w1);
-  if (!(ok0 && ok1)) {
-    if (!ok0) sol_ref_rinv3_slow(a0, r0, w0);
-    if (!ok1) sol_ref_rinv3_slow(a1, r1, w1);
-  }
 }

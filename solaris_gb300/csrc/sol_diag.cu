@@ -364,8 +364,8 @@ __global__ void k_check_rinv3(int mode, long long n, unsigned long long seed, un
       }
       const double w = __ddiv_rn(1.0, d);
       const long long zb = __double_as_longlong(w) + ((long long)((h2 >> 20) % 601) - 300);
-      const long long wb = solcr::rcp_from_approx(d, zb, ok);
-      bad = ok && (wb != __double_as_longlong(w));
+      const double got = solcr::rcp_from_approx(d, (zb & 0xFFFFFFFFFFFFFll) | (1ll << 52), (int)(zb >> 52) - 1023, ok);
+      bad = ok && (__double_as_longlong(got) != __double_as_longlong(w));
     }
     if (!ok) atomicAdd(&counts[1], 1ull);
     if (bad) {

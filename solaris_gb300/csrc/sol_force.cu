@@ -425,18 +425,21 @@ __global__ void __launch_bounds__(kSinkBlock) k_gravity_ac(ForceCtx fc, const do
 // instructions, and a source costs each summing warp one more however few of
 // its lanes have a sink: the sums fill 30 of 32 lanes (10 sinks a summing
 // warp) where a warp per component would leave most of them empty, and the
-// squares of the displacement join the term multiplications on the integer
-// pipe: 11 FP64 instructions a pair instead of 14, beside ~430 integer ones
-// (333 before), which is where both pipes are about equally loaded.  (With
-// the product r^2 r moved there too the integer pipe leads: 1-3% slower.)  A
-// system of a few sinks per SM is bound by the sums' serial chain instead,
-// 64 cycles a source and ~80 measured, hence warps of their own for them
-// rather than a phase in which the producers wait.
+// squares of the displacement join the term multiplications and the
+// remainders of the root and the quotient (sol_crmath.cuh) on the integer
+// pipe: 9 FP64 instructions a pair beside its three sums, where both pipes are
+// about equally loaded.  (With the product r^2 r moved there too: 16,411
+// bodies 6.95 ms for 7.02, 2,049 160 us for 156.)  A system of a few sinks per
+// SM is bound by the sums' serial chain instead, 64 cycles a source alone and
+// ~105 beside the producers, hence warps of their own for them rather than a
+// phase in which the producers wait.  (Two half tiles interleaved in a
+// producing warp, 108 registers: 1,033 bodies 62.3 us for 64.1, 4,099 646 for
+// 509.)
 //
 // Measured (one evaluation, us; before: the two kernels this one replaces,
 // 4 sinks x 224 sources with 12 summing lanes, and 32 sinks alternating
-// between producing and summing): 300 bodies 37 -> 21, 1,033 94 -> 67, 2,049
-// 305 -> 168, 4,099 900 -> 565, 16,411 10,800 -> 7,970.
+// between producing and summing): 300 bodies 37 -> 25 (prepass included), 1,033
+// 94 -> 64, 2,049 305 -> 155, 4,099 900 -> 509, 16,411 10,800 -> 7,050.
 constexpr int kRefTile = 64;      // sources per round
 constexpr int kRefPerWarp = 10;   // sinks per summing warp: 30 of its 32 lanes
 constexpr int kRefMaxSinks = 21;  // of the two-warp form: 63 of 64 lanes
@@ -464,9 +467,11 @@ __device__ __forceinline__ void ref_pair(double xij, double yij, double zij, boo
   }
 }
 
-// 32 warps per SM (64 registers): four CTAs of the one-warp form, two of the other
+// 24 warps per SM (80 registers): three CTAs of the one-warp form, one of the
+// other.  With 32 (64 registers, a few spilled): 1,033 bodies 66.3 us for 64.1,
+// 4,099 521 for 509, 16,411 7.02 ms for 7.05.
 template <int SW, int PW>
-__global__ void __launch_bounds__((SW + PW) * 32, 32 / (SW + PW))
+__global__ void __launch_bounds__((SW + PW) * 32, 24 / (SW + PW))
     k_gravity_ac_ref(ForceCtx fc, const double* __restrict__ y, double* __restrict__ dydt, TimeSpec ts, uint32_t flags,
                      int spc) {
   extern __shared__ __align__(16) double ref_dyn[];
@@ -1468,8 +1473,7 @@ static FFPlan ff_plan(int device, int n, const Classes& cls, int npad) {
 // costs a source: spc sinks' pairs and the summing warps', which cost about
 // 1.9 sinks each (16 cycles of the FP64 pipe against ~9 a sink).  For each k
 // the fewest sinks that reach it; the cheapest of one summing warp (up to
-// kRefPerWarp sinks) and two.  Measured at 4,099 bodies (us): 9 sinks 575, 7
-// sinks 564, 14 sinks with two summing warps 569; at 16,411 18 with two 7,970.
+// kRefPerWarp sinks) and two.
 static void ref_shape(int nsink, int nsm, int& spc, int& sw) {
   double best = 1e300;
   spc = 1;
