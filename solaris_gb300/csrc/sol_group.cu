@@ -374,13 +374,14 @@ __device__ __noinline__ void last_evaluation(const GroupArgs& P, const View& V, 
 }
 
 // An item in two passes.  The first: rm3 of a body or d |d|^-3 and |d| of a
-// pair (GravityAC, Acceleration.cpp:259-261, :294-308).  IEEE square root and
-// reciprocal: latency counts here, and their ~1,240 cycles are fewer than
-// those of the integer-pipe forms that serve the throughput-bound kernels
-// (~2,000).  The second, once every first pass is done: the Kepler term
-// -mu rm3 r of a body (:281-283), G m_j (d |d|^-3 - r_j rm3_j) of a pair,
-// both as a fused multiply-add and a multiplication (x * 1 - y and x * y - 0
-// round once, as x - y and x * y do).
+// pair (GravityAC, Acceleration.cpp:259-261, :294-308), the root and the
+// reciprocal by sol_ref_rinv3: latency counts here, and its one FP64
+// instruction among FP32 and integer ones is a shorter chain than IEEE square
+// root and reciprocal (40 driver calls of 256 bodies: 1.56 ms for 1.86; four
+// of 8,193 in gas: 0.608 for 0.634).  The second, once every first pass is
+// done: the Kepler term -mu rm3 r of a body (:281-283), G m_j (d |d|^-3 -
+// r_j rm3_j) of a pair, both as a fused multiply-add and a multiplication
+// (x * 1 - y and x * y - 0 round once, as x - y and x * y do).
 __device__ __forceinline__ void first_pass(const View& V, const double* yt, int it, int ends) {
   const double* yi = yt + 6 * (ends & 0xFFFF);
   const double* yj = yt + 6 * (ends >> 16);
@@ -388,7 +389,8 @@ __device__ __forceinline__ void first_pass(const View& V, const double* yt, int 
   const double yij = yj[1] - yi[1];
   const double zij = yj[2] - yi[2];
   const double rij2 = xij * xij + yij * yij + zij * zij;
-  const double rij = __dsqrt_rn(rij2), rijm3 = __drcp_rn(rij2 * rij);
+  double rij, rijm3;
+  sol_ref_rinv3(rij2, rij, rijm3);
   double* p = V.p + it;
   p[0] = xij * rijm3;
   p[V.icap] = yij * rijm3;
@@ -434,7 +436,8 @@ __device__ __forceinline__ void work_by_component(const GroupArgs& P, const View
     const double qx = __shfl_sync(0xFFFFFFFFu, sq, 0, 4), qy = __shfl_sync(0xFFFFFFFFu, sq, 1, 4),
                  qz = __shfl_sync(0xFFFFFFFFu, sq, 2, 4);
     const double rij2 = qx + qy + qz;
-    const double rij = __dsqrt_rn(rij2), rijm3 = __drcp_rn(rij2 * rij);
+    double rij = 0.0, rijm3 = 0.0;
+    if (live) sol_ref_rinv3(rij2, rij, rijm3);
     const double pp = x * rijm3;
     if (live) {
       if (source) *xj = pp;
