@@ -26,7 +26,7 @@ namespace {
 constexpr int kBlock = 256;
 constexpr int kVjpThreads = 128;  // threads of k_vjp: one body's pairs
 constexpr int kVjpWarps = kVjpThreads / 32;
-constexpr int kPreBodies = 42;    // bodies per CTA of k_vjp_cotangent: 252 elements
+constexpr int kPreBodies = 32;    // bodies per CTA of k_vjp_cotangent, a lane each in its sums: 192 elements
 constexpr int kAdjStages = 11;  // stages 0..10 reach y_{n+1}
 
 // RKF78 tableau (RungeKuttaFehlberg78.cpp:41-56): a[j][k] and the weights b
@@ -65,40 +65,53 @@ __global__ void k_lincomb(int nv, double* __restrict__ out, const double* __rest
 }
 
 // The stage's cotangent w = h b_k lambda + h sum_j a_jk nu_j (L, scaled by h),
-// the structure-of-arrays view of (state, cotangent) that k_vjp streams -- x,
-// y, z, m, wx, wy, wz -- and this CTA's sums of the cotangent's velocity part
-// over its bodies: [0..2] those with index >= 1, [3..5] those below nm.  One
-// thread per element, kPreBodies bodies per CTA.
+// the structure-of-arrays view of (state, cotangent) that the pair kernels
+// stream -- x, y, z, m, wx, wy, wz -- and this CTA's sums of the cotangent's
+// velocity part over its bodies: [0..2] those with index >= 1, [3..5] those
+// below nm.  One thread per element, kPreBodies bodies per CTA; sw: 6 kPreBodies words.
+__device__ __forceinline__ void cotangent(int n, int nm, const double* __restrict__ Y, const double* __restrict__ mass,
+                                          double h, const Lin& L, double* __restrict__ w, double* __restrict__ soa,
+                                          double* __restrict__ wsum, double* sw) {
+  const int i0 = blockIdx.x * kPreBodies;
+  const int b = threadIdx.x / 6, k = threadIdx.x - 6 * b;
+  const int i = i0 + b;
+  if (b < kPreBodies) {
+    double acc = 0.0;
+    if (i < n) {
+      const size_t e = 6 * (size_t)i + k;
+      double v[kAdjStages + 1];  // every load in flight before the first product
+#pragma unroll
+      for (int q = 0; q <= kAdjStages; ++q) v[q] = q < L.k ? L.v[q][e] : 0.0;
+#pragma unroll
+      for (int q = 0; q <= kAdjStages; ++q)
+        if (q < L.k) acc = __fma_rn(L.c[q], v[q], acc);
+      acc = h * acc;
+      w[e] = acc;
+      if (k < 3) {
+        soa[(size_t)k * n + i] = Y[e];
+        if (k == 0) soa[(size_t)3 * n + i] = mass[i];
+      } else {
+        soa[(size_t)(k + 1) * n + i] = acc;
+      }
+    }
+    sw[threadIdx.x] = acc;
+  }
+  __syncthreads();
+  const int sum = threadIdx.x >> 5, lane = threadIdx.x & 31;  // a warp per sum
+  if (sum < 6) {
+    const int j = i0 + lane;
+    double t = j >= 1 && j < (sum < 3 ? n : nm) ? sw[6 * lane + 3 + sum % 3] : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) wsum[6 * (size_t)blockIdx.x + sum] = t;
+  }
+}
 __global__ void __launch_bounds__(6 * kPreBodies) k_vjp_cotangent(int n, int nm, const double* __restrict__ Y,
                                                                   const double* __restrict__ mass, double h, Lin L,
                                                                   double* __restrict__ w, double* __restrict__ soa,
                                                                   double* __restrict__ wsum) {
   __shared__ double sw[6 * kPreBodies];
-  const int i0 = blockIdx.x * kPreBodies;
-  const int b = threadIdx.x / 6, k = threadIdx.x - 6 * b;
-  const int i = i0 + b;
-  double acc = 0.0;
-  if (i < n) {
-    const size_t e = 6 * (size_t)i + k;
-    for (int q = 0; q < L.k; ++q) acc = __fma_rn(L.c[q], L.v[q][e], acc);
-    acc = h * acc;
-    w[e] = acc;
-    if (k < 3) {
-      soa[(size_t)k * n + i] = Y[e];
-      if (k == 0) soa[(size_t)3 * n + i] = mass[i];
-    } else {
-      soa[(size_t)(k + 1) * n + i] = acc;
-    }
-  }
-  sw[threadIdx.x] = acc;
-  __syncthreads();
-  if (threadIdx.x < 6) {
-    const int c = 3 + threadIdx.x % 3;
-    const int hi = min(i0 + kPreBodies, threadIdx.x < 3 ? n : nm);
-    double t = 0.0;
-    for (int j = max(i0, 1); j < hi; ++j) t += sw[6 * (j - i0) + c];
-    wsum[6 * (size_t)blockIdx.x + threadIdx.x] = t;
-  }
+  cotangent(n, nm, Y, mass, h, L, w, soa, wsum, sw);
 }
 
 // r^-3 and r^-2 of r^2: the FP32 seed y of 1/r, its square (exact) and cube
@@ -144,14 +157,36 @@ __device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
   return v[0];
 }
 
-__device__ __forceinline__ void tensor_apply(double dx, double dy, double dz, double rm3, double rm5, double vx,
-                                             double vy, double vz, double& ox, double& oy, double& oz) {
-  // T(d) v = v / r^3 - 3 d (d . v) / r^5
-  const double dv = __fma_rn(dx, vx, __fma_rn(dy, vy, dz * vz));
-  const double s = 3.0 * rm5 * dv;
-  ox = __fma_rn(vx, rm3, -s * dx);
-  oy = __fma_rn(vy, rm3, -s * dy);
-  oz = __fma_rn(vz, rm3, -s * dz);
+// Body k's part of nu, dm and d/d m_0 from its sums over the other bodies (tot)
+// and over the cotangents of its sinks (Wv), r, w_v of the body in x and wk:
+// part 0 to 2, a component of nu; 3, the masses.
+__device__ __forceinline__ void vjp_finish_body(int part, int k, const double* x, const double* wk, double mk, double m0,
+                                                const double* tot, const double* Wv, const double* w, double* nu,
+                                                double* __restrict__ dm, double* __restrict__ m0_part) {
+  const double G = SOL_GAUSS2;
+  const double r2 = __fma_rn(x[0], x[0], __fma_rn(x[1], x[1], x[2] * x[2]));
+  double rm3, rm2;
+  rinv32(r2, rm3, rm2);
+  if (part < 3) {
+    const double xc = part == 0 ? x[0] : part == 1 ? x[1] : x[2], wc = part == 0 ? wk[0] : part == 1 ? wk[1] : wk[2];
+    const double tc = part == 0 ? tot[0] : part == 1 ? tot[1] : tot[2], sc = part == 0 ? tot[4] : part == 1 ? tot[5] : tot[6];
+    const double g = __fma_rn(mk, tc, __fma_rn(-wc, tot[3], -3.0 * sc));
+    // Kepler term -G (m0 + m_k) r_k / |r_k|^3 and indirect term -G m_k r_k / |r_k|^3 (for the sinks of k):
+    // T(r) v = v / r^3 - 3 r (r . v) / r^5
+    const double mu = -(m0 + mk);
+    const double vx = __fma_rn(mu, wk[0], -mk * Wv[0]), vy = __fma_rn(mu, wk[1], -mk * Wv[1]),
+                 vz = __fma_rn(mu, wk[2], -mk * Wv[2]);
+    const double dv = __fma_rn(x[0], vx, __fma_rn(x[1], vy, x[2] * vz));
+    const double s = 3.0 * (rm3 * rm2) * dv;
+    const double t = __fma_rn(part == 0 ? vx : part == 1 ? vy : vz, rm3, -s * xc);
+    nu[6 * (size_t)k + part] = G * (g + t);
+    nu[6 * (size_t)k + 3 + part] = w[6 * (size_t)k + part];  // d(position)/dt = velocity
+  } else {
+    const double rk_w = __fma_rn(x[0], wk[0], __fma_rn(x[1], wk[1], x[2] * wk[2])) * rm3;  // w_k . r_k / |r_k|^3
+    const double rk_W = __fma_rn(x[0], Wv[0], __fma_rn(x[1], Wv[1], x[2] * Wv[2])) * rm3;
+    dm[k] += G * (tot[7] - rk_w - rk_W);
+    m0_part[k] -= G * rk_w;
+  }
 }
 
 // nu = J(Y)^T w for the heliocentric gravity with Kepler and indirect terms:
@@ -238,30 +273,192 @@ __global__ void __launch_bounds__(kVjpThreads) k_vjp(int n, int nm, int nspl, co
     tot[threadIdx.x] = t;
   }
   __syncwarp();
-  if (threadIdx.x != 0) return;
-  const double G = SOL_GAUSS2;
-  const double gx = __fma_rn(mk, tot[0], __fma_rn(-wkx, tot[3], -3.0 * tot[4]));
-  const double gy = __fma_rn(mk, tot[1], __fma_rn(-wky, tot[3], -3.0 * tot[5]));
-  const double gz = __fma_rn(mk, tot[2], __fma_rn(-wkz, tot[3], -3.0 * tot[6]));
-  // Kepler term -G (m0 + m_k) r_k / |r_k|^3 and indirect term -G m_k r_k / |r_k|^3 (for the sinks of k)
-  const double r2 = __fma_rn(xk, xk, __fma_rn(yk, yk, zk * zk));
-  double rm3, rm2;
-  rinv32(r2, rm3, rm2);
-  const double mu = -(M[0] + mk);
-  const double Wx = W[0], Wy = W[1], Wz = W[2];  // 0 when k is no source
-  double kx, ky, kz;
-  tensor_apply(xk, yk, zk, rm3, rm3 * rm2, __fma_rn(mu, wkx, -mk * Wx), __fma_rn(mu, wky, -mk * Wy),
-               __fma_rn(mu, wkz, -mk * Wz), kx, ky, kz);
-  nu[6 * (size_t)k + 0] = G * (gx + kx);
-  nu[6 * (size_t)k + 1] = G * (gy + ky);
-  nu[6 * (size_t)k + 2] = G * (gz + kz);
-  nu[6 * (size_t)k + 3] = w[6 * (size_t)k + 0];  // d(position)/dt = velocity
-  nu[6 * (size_t)k + 4] = w[6 * (size_t)k + 1];
-  nu[6 * (size_t)k + 5] = w[6 * (size_t)k + 2];
-  const double rk_w = __fma_rn(xk, wkx, __fma_rn(yk, wky, zk * wkz)) * rm3;  // w_k . r_k / |r_k|^3
-  const double rk_W = __fma_rn(xk, Wx, __fma_rn(yk, Wy, zk * Wz)) * rm3;
-  dm[k] += G * (tot[7] - rk_w - rk_W);
-  m0_part[k] -= G * rk_w;
+  if (threadIdx.x >= 4) return;
+  const double x[3] = {xk, yk, zk}, wk[3] = {wkx, wky, wkz};
+  vjp_finish_body(threadIdx.x, k, x, wk, mk, M[0], tot, W, w, nu, dm, m0_part);
+}
+
+// ---- block pairs: every unordered pair once --------------------------------------
+// Seen from j, d changes its sign and p = d . w_j and q = d . w_k change places,
+// so r^-3, p, q and s = (m_k p - m_j q) / r^5 serve both bodies: 20 FP64
+// instructions shared and 8 a side, 36 an unordered pair where k_vjp takes 56.
+// Bodies in blocks of 32.  A CTA has one pair of blocks (I, J), I <= J, its four
+// warps eight of the 32 steps each: lane l of a warp holds body k = 32 I + l
+// with its sums, and at step t takes body 32 J + (l + t) mod 32 from shared
+// memory, whose sums pass from lane to lane by shuffles.  (I = J: steps 1 to 16,
+// the last by half of the lanes.)  The warps' sums are added in shared memory
+// and written, k's and j's sides, to part[pair][side][8][32]; k_vjp_finish adds
+// a body's partials.  Blocks that lie beyond the sources attract nothing: only
+// pairs with I below nsb = ceil(sources / 32).
+//
+// FP64 pipe: 18 instructions a pair and body, 16.5 cycles each: 34 us at 1,033
+// bodies (561 CTAs, 3.7 an SM).  Measured, the product with its cotangent:
+// 1,033 bodies 82 -> 61 us, 4,000 460 -> 285, 16,384 7.1 -> 4.4 ms.
+constexpr int kPairBodies = 32;
+constexpr int kPairWarps = 4;
+constexpr int kPairSteps = 32 / kPairWarps;
+constexpr int kFinishWarps = 16;
+// Bodies for which it is used: below kPairMin k_vjp's one launch is shorter (a
+// product with its cotangent, us: 300 bodies 19 and 26, 500 33 and 29, 700 49 and
+// 38), beyond kPairMax the partials, 4 KB a block pair, would pass 0.54 GB.
+constexpr int kPairMin = 448, kPairMax = 16384;
+
+__host__ __device__ __forceinline__ size_t vjp_pair(int I, int J, int nb) {
+  return (size_t)I * nb - (size_t)I * (I - 1) / 2 + (J - I);
+}
+
+__global__ void __launch_bounds__(32 * kPairWarps, 4)
+    k_vjp_pairs(int n, int nm, int nspl, int nb, const double* __restrict__ soa, double* __restrict__ part) {
+  __shared__ double sj[7][kPairBodies];
+  __shared__ double red[2][kPairWarps][8][32];
+  int I = 0, J = blockIdx.x;  // row I has nb - I pairs
+  {
+    const float t = 2.0f * nb + 1.0f;
+    I = max(0, min(nb - 1, (int)(0.5f * (t - sqrtf(fmaxf(0.0f, t * t - 8.0f * (float)J))))));
+    while (I > 0 && (long long)vjp_pair(I, I, nb) > (long long)blockIdx.x) --I;
+    while (I + 1 < nb && (long long)vjp_pair(I + 1, I + 1, nb) <= (long long)blockIdx.x) ++I;
+    J = I + (int)(blockIdx.x - vjp_pair(I, I, nb));
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // a body beyond the system: apart from all others, no pair of it counts
+  for (int q = threadIdx.x; q < 7 * kPairBodies; q += 32 * kPairWarps) {
+    const int row = q / kPairBodies, j = J * kPairBodies + q % kPairBodies;
+    sj[row][q % kPairBodies] = j < n ? soa[(size_t)row * n + j] : (row == 0 ? 1.0e6 * (1 + q % kPairBodies) : 0.0);
+  }
+  const int k = I * kPairBodies + lane;
+  const bool livek = k >= 1 && k < n;
+  const double xk = k < n ? soa[k] : -1.0e6, yk = k < n ? soa[n + k] : 0.0, zk = k < n ? soa[2 * (size_t)n + k] : 0.0;
+  const double mk = livek ? soa[3 * (size_t)n + k] : 0.0;
+  const double wkx = livek ? soa[4 * (size_t)n + k] : 0.0, wky = livek ? soa[5 * (size_t)n + k] : 0.0,
+               wkz = livek ? soa[6 * (size_t)n + k] : 0.0;
+  const bool diag = I == J;
+  const int steps = diag ? kPairSteps / 2 : kPairSteps;
+  const int t0 = diag ? 1 + warp * steps : warp * steps;
+  double v[8] = {0, 0, 0, 0, 0, 0, 0, 0}, u[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  __syncthreads();
+#pragma unroll 1
+  for (int t = t0;; ++t) {
+    const int q = (lane + t) & 31, j = J * kPairBodies + q;
+    const bool live = livek && j >= 1 && j < n && !(diag && t == 16 && lane >= 16);
+    const bool ks = live && (k < nm || (k < nm + nspl && j < nm));  // k attracts j
+    const bool js = live && (j < nm || (j < nm + nspl && k < nm));  // j attracts k
+    const double dx = sj[0][q] - xk, dy = sj[1][q] - yk, dz = sj[2][q] - zk;
+    const double wjx = ks ? sj[4][q] : 0.0, wjy = ks ? sj[5][q] : 0.0, wjz = ks ? sj[6][q] : 0.0;
+    const double vkx = js ? wkx : 0.0, vky = js ? wky : 0.0, vkz = js ? wkz : 0.0;
+    const double mj = js ? sj[3][q] : 0.0, mi = ks ? mk : 0.0;
+    if (ks | js) {
+      const double r2 = __fma_rn(dx, dx, __fma_rn(dy, dy, dz * dz));
+      double rm3, rm2;
+      rinv32(r2, rm3, rm2);
+      const double p = __fma_rn(dx, wjx, __fma_rn(dy, wjy, dz * wjz));
+      const double g = __fma_rn(dx, vkx, __fma_rn(dy, vky, dz * vkz));
+      const double s = (__fma_rn(mi, p, -mj * g) * rm2) * rm3;
+      v[0] = __fma_rn(rm3, wjx, v[0]);
+      v[1] = __fma_rn(rm3, wjy, v[1]);
+      v[2] = __fma_rn(rm3, wjz, v[2]);
+      v[3] = __fma_rn(rm3, mj, v[3]);
+      v[4] = __fma_rn(s, dx, v[4]);
+      v[5] = __fma_rn(s, dy, v[5]);
+      v[6] = __fma_rn(s, dz, v[6]);
+      v[7] = __fma_rn(-rm3, p, v[7]);
+      u[0] = __fma_rn(rm3, vkx, u[0]);
+      u[1] = __fma_rn(rm3, vky, u[1]);
+      u[2] = __fma_rn(rm3, vkz, u[2]);
+      u[3] = __fma_rn(rm3, mi, u[3]);
+      u[4] = __fma_rn(-s, dx, u[4]);
+      u[5] = __fma_rn(-s, dy, u[5]);
+      u[6] = __fma_rn(-s, dz, u[6]);
+      u[7] = __fma_rn(rm3, g, u[7]);
+    }
+    if (t == t0 + steps - 1) {
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        red[0][warp][c][lane] = v[c];
+        red[1][warp][c][q] = u[c];
+      }
+      break;
+    }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) u[c] = __shfl_sync(0xffffffffu, u[c], (lane + 1) & 31);
+  }
+  __syncthreads();
+  double* out = part + (size_t)blockIdx.x * 16 * 32;
+  for (int x = threadIdx.x; x < 8 * 32; x += 32 * kPairWarps) {
+    const int c = x >> 5, l = x & 31;
+    const double a = (red[0][0][c][l] + red[0][1][c][l]) + (red[0][2][c][l] + red[0][3][c][l]);
+    const double b = (red[1][0][c][l] + red[1][1][c][l]) + (red[1][2][c][l] + red[1][3][c][l]);
+    out[x] = diag ? a + b : a;
+    out[8 * 32 + x] = diag ? 0.0 : b;
+  }
+}
+
+// A block's bodies: the partials in block order, the body's own terms (nu, dm,
+// m0_part), at a step's last stage (lam_out not null) lambda + sum nu (S), and
+// the cotangent of the next stage (L.k > 0; wsum_next is not wsum, which other
+// CTAs may still read).  Bounded by the latency of the partials' loads.
+__global__ void __launch_bounds__(32 * kFinishWarps) k_vjp_finish(
+    int n, int nm, int nspl, int nb, int nsb, double* __restrict__ soa, const double* __restrict__ part,
+    const double* __restrict__ wsum, double* __restrict__ w, double* nu, double* __restrict__ dm,
+    double* __restrict__ m0_part, const double* __restrict__ lam, double* lam_out, Lin S,
+    const double* __restrict__ Ynext, const double* __restrict__ mass, double h, Lin L,
+    double* __restrict__ wsum_next) {
+  __shared__ double tot[kFinishWarps / 8][8][32];
+  __shared__ double W[6];
+  __shared__ double sw[6 * kPreBodies];
+  static_assert(kPreBodies == kPairBodies, "a CTA finishes a block and prepares it");
+  const int B = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  {
+    // partial q of the block, q < nq: from row q as the column B, then the row's own
+    const int c = warp & 7, nq = B < nsb ? nb : nsb;
+    double t = 0.0;
+    constexpr int kStep = kFinishWarps / 8;
+#pragma unroll 4
+    for (int q = warp >> 3; q < nq; q += kStep) {
+      const size_t at = q < B ? vjp_pair(q, B, nb) * 2 + 1 : vjp_pair(B, q, nb) * 2;
+      t += part[at * 256 + 32 * c + lane];
+    }
+    tot[warp >> 3][c][lane] = t;
+  }
+  if (warp < 6) {
+    double t = 0.0;
+    for (int b = lane; b < nb; b += 32) t += wsum[6 * (size_t)b + warp];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) W[warp] = t;
+  }
+  __syncthreads();
+  const int k = B * kPairBodies + lane;
+  if (warp < 4 && k < n) {
+    if (k == 0) {
+      if (warp < 3) nu[warp] = nu[3 + warp] = 0.0;
+    } else {
+      const double x[3] = {soa[k], soa[n + k], soa[2 * (size_t)n + k]};
+      const double wk[3] = {soa[4 * (size_t)n + k], soa[5 * (size_t)n + k], soa[6 * (size_t)n + k]};
+      // the sum of w over the sinks of k: every other body, the massive ones, none
+      const bool massive = k < nm, source = k < nm + nspl;
+      double mine[8], Wv[3];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) Wv[q] = massive ? W[q] - wk[q] : source ? W[3 + q] : 0.0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        mine[q] = tot[0][q][lane];
+#pragma unroll
+        for (int u = 1; u < kFinishWarps / 8; ++u) mine[q] += tot[u][q][lane];
+      }
+      vjp_finish_body(warp, k, x, wk, soa[3 * (size_t)n + k], mass[0], mine, Wv, w, nu, dm, m0_part);
+    }
+  }
+  __syncthreads();
+  if (lam_out) {
+    const size_t e = 6 * (size_t)B * kPairBodies + threadIdx.x;
+    if (threadIdx.x < 6 * kPairBodies && e < 6 * (size_t)n) {
+      double acc = 0.0;
+      for (int q = 0; q < S.k; ++q) acc = __fma_rn(S.c[q], S.v[q][e], acc);
+      lam_out[e] = __fma_rn(1.0, acc, lam[e]);
+    }
+    __syncthreads();
+  }
+  if (L.k > 0) cotangent(n, nm, Ynext, mass, h, L, w, soa, wsum_next, sw);
 }
 
 // dm[0] += sum of the per-body parts, one block, fixed order
@@ -298,10 +495,12 @@ struct sol_adjoint_state {
   double* d_cp = nullptr;     // checkpoints, (n_cp) x 6N
   double* d_stages = nullptr; // every x 11 x 6N stage states of one segment
   double* d_nu = nullptr;     // 11 x 6N stage adjoints
-  double* d_lam = nullptr;    // 6N
+  double* d_lam = nullptr;    // 6N, and the next step's
+  double* d_lam2 = nullptr;
   double* d_w = nullptr;      // 6N
   double* d_soa = nullptr;    // 7N
-  double* d_wsum = nullptr;   // 6 per CTA of k_vjp_cotangent
+  double* d_wsum = nullptr;   // two of 6 per CTA of k_vjp_cotangent
+  double* d_part = nullptr;   // partials of k_vjp_pairs, or null: k_vjp
   double* d_dm = nullptr;     // N
   double* d_m0p = nullptr;    // N
   double* d_tmp = nullptr;    // 6N
@@ -309,7 +508,8 @@ struct sol_adjoint_state {
 
 void sol_adjoint_free(sol_adjoint_state* a) {
   if (!a) return;
-  double* p[] = {a->d_cp, a->d_stages, a->d_nu, a->d_lam, a->d_w, a->d_soa, a->d_wsum, a->d_dm, a->d_m0p, a->d_tmp};
+  double* p[] = {a->d_cp, a->d_stages, a->d_nu, a->d_lam, a->d_lam2, a->d_w, a->d_soa, a->d_wsum, a->d_part, a->d_dm, a->d_m0p,
+                a->d_tmp};
   for (double* q : p)
     if (q) cudaFree(q);
   delete a;
@@ -324,6 +524,20 @@ int set_fixed_h(sol_ctx* c, double h) {
   hc.eps = c->eps;
   SOL_CUDA(cudaMemcpyAsync(c->d_ctrl, &hc, sizeof(hc), cudaMemcpyHostToDevice, c->stream));
   return SOL_OK;
+}
+
+// w_k / h: kB[k] lambda + sum_{j > k} a_jk nu_j
+Lin stage_cotangent(const sol_adjoint_state* a, const double* lam, int k, size_t nv) {
+  Lin L;
+  memset(&L, 0, sizeof(L));
+  L.v[L.k] = lam;
+  L.c[L.k++] = kB[k];
+  for (int j = k + 1; j < kAdjStages; ++j)
+    if (kA[j][k] != 0.0) {
+      L.v[L.k] = a->d_nu + (size_t)j * nv;
+      L.c[L.k++] = kA[j][k];
+    }
+  return L;
 }
 
 // nu = J(Y)^T w of the cotangent w = h sum_i L.c[i] L.v[i]
@@ -402,9 +616,18 @@ extern "C" int sol_adjoint_backward(sol_ctx* c, const double* dl_dy_final, doubl
   RET(alloc(&a->d_stages, (size_t)a->every * kAdjStages * nv));
   RET(alloc(&a->d_nu, (size_t)kAdjStages * nv));
   RET(alloc(&a->d_lam, nv));
+  RET(alloc(&a->d_lam2, nv));
   RET(alloc(&a->d_w, nv));
   RET(alloc(&a->d_soa, 7 * (size_t)n));
-  RET(alloc(&a->d_wsum, 6 * (size_t)((n + kPreBodies - 1) / kPreBodies)));
+  const int nb = (n + kPairBodies - 1) / kPairBodies;
+  const int ns = c->cls.nm + c->cls.n_spl, nsb = (ns + kPairBodies - 1) / kPairBodies;
+  const size_t npairs = vjp_pair(nsb, nsb, nb);
+  RET(alloc(&a->d_wsum, 12 * (size_t)nb));
+  if (n >= kPairMin && n <= kPairMax && !a->d_part &&
+      cudaMalloc((void**)&a->d_part, sizeof(double) * npairs * 16 * 32) != cudaSuccess) {
+    cudaGetLastError();  // no room for the partials: k_vjp needs none
+    a->d_part = nullptr;
+  }
   RET(alloc(&a->d_dm, n));
   RET(alloc(&a->d_m0p, n));
   RET(alloc(&a->d_tmp, nv));
@@ -428,29 +651,56 @@ extern "C" int sol_adjoint_backward(sol_ctx* c, const double* dl_dy_final, doubl
       RET(sol_rkf78_stages(c, outs[0], a->d_tmp, outs));
     }
     // backward through the segment's steps
+    int buf = 0;
     for (int s = s1 - 1; s >= s0; --s) {
       const double* Ys = a->d_stages + (size_t)(s - s0) * kAdjStages * nv;
-      for (int k = kAdjStages - 1; k >= 0; --k) {
-        Lin L;
-        memset(&L, 0, sizeof(L));
-        L.v[L.k] = a->d_lam;
-        L.c[L.k++] = kB[k];
-        for (int j = k + 1; j < kAdjStages; ++j)
-          if (kA[j][k] != 0.0) {
-            L.v[L.k] = a->d_nu + (size_t)j * nv;
-            L.c[L.k++] = kA[j][k];
-          }
-        RET(vjp(c, a, Ys + (size_t)k * nv, h, L, a->d_nu + (size_t)k * nv));
-      }
-      Lin L;
-      memset(&L, 0, sizeof(L));
+      // lambda + sum nu, once the step's stages are done
+      Lin S;
+      memset(&S, 0, sizeof(S));
       for (int k = 0; k < kAdjStages; ++k) {
-        L.v[L.k] = a->d_nu + (size_t)k * nv;
-        L.c[L.k++] = 1.0;
+        S.v[S.k] = a->d_nu + (size_t)k * nv;
+        S.c[S.k++] = 1.0;
       }
-      k_lincomb<<<g, kBlock, 0, c->stream>>>((int)nv, a->d_w, a->d_lam, 1.0, L);
-      SOL_LAUNCHED();
-      std::swap(a->d_w, a->d_lam);
+      for (int k = kAdjStages - 1; k >= 0; --k) {
+        double* nu = a->d_nu + (size_t)k * nv;
+        const bool first = s == s1 - 1 && k == kAdjStages - 1;
+        if (!a->d_part) {
+          RET(vjp(c, a, Ys + (size_t)k * nv, h, stage_cotangent(a, a->d_lam, k, nv), nu));
+          continue;
+        }
+        double* wsum = a->d_wsum + (size_t)buf * 6 * nb;
+        if (first) {
+          k_vjp_cotangent<<<nb, 6 * kPreBodies, 0, c->stream>>>(n, c->cls.nm, Ys + (size_t)k * nv, c->d_mass, h,
+                                                                stage_cotangent(a, a->d_lam, k, nv), a->d_w, a->d_soa,
+                                                                wsum);
+          SOL_LAUNCHED();
+        }
+        k_vjp_pairs<<<(unsigned)npairs, 32 * kPairWarps, 0, c->stream>>>(n, c->cls.nm, c->cls.n_spl, nb, a->d_soa,
+                                                                         a->d_part);
+        SOL_LAUNCHED();
+        // the next stage: this step's, or the last one of the step before (none at the segment's start)
+        const bool end = k == 0;
+        Lin next;
+        memset(&next, 0, sizeof(next));
+        const double* Yn = nullptr;
+        if (!end) {
+          next = stage_cotangent(a, a->d_lam, k - 1, nv);
+          Yn = Ys + (size_t)(k - 1) * nv;
+        } else if (s > s0) {
+          next = stage_cotangent(a, a->d_lam2, kAdjStages - 1, nv);
+          Yn = Ys - nv;  // stage 10 of the step before
+        }
+        k_vjp_finish<<<nb, 32 * kFinishWarps, 0, c->stream>>>(n, c->cls.nm, c->cls.n_spl, nb, nsb, a->d_soa, a->d_part, wsum, a->d_w,
+                                                nu, a->d_dm, a->d_m0p, a->d_lam, end ? a->d_lam2 : nullptr, S, Yn,
+                                                c->d_mass, h, next, a->d_wsum + (size_t)(1 - buf) * 6 * nb);
+        SOL_LAUNCHED();
+        buf = 1 - buf;
+      }
+      if (!a->d_part) {
+        k_lincomb<<<g, kBlock, 0, c->stream>>>((int)nv, a->d_lam2, a->d_lam, 1.0, S);
+        SOL_LAUNCHED();
+      }
+      std::swap(a->d_lam2, a->d_lam);
     }
   }
   k_sum_m0<<<1, kBlock, 0, c->stream>>>(n, a->d_m0p, a->d_dm);

@@ -1,8 +1,8 @@
 """The vector-Jacobian product (sol_adjoint.cu) over every pairing of body
 classes -- massive bodies see the super-planetesimals, lighter ones do not, light
-ones attract nothing -- and sizes around its blocks, against the oracle's
-tangent-linear model.  Bound: as the adjoint's other tests, 1e-6 of the
-directional derivative."""
+ones attract nothing -- sizes around the blocks of 32 bodies and where the form
+over block pairs begins (448 bodies), against the oracle's tangent-linear model.
+Bound: as the adjoint's other tests, 1e-6 of the directional derivative."""
 import numpy as np
 import pytest
 
@@ -31,7 +31,9 @@ def _system(n_massive, n_spl, n_pl, n_tp):
 
 
 @pytest.mark.parametrize("sizes", [(1, 0, 0, 0), (5, 3, 4, 2), (31, 0, 0, 0), (32, 0, 0, 0), (33, 7, 0, 30), (20, 11, 1, 1),
-                                   (60, 5, 64, 3), (127, 0, 0, 0), (1, 0, 130, 0)])
+                                   (60, 5, 64, 3), (127, 0, 0, 0), (1, 0, 130, 0),
+                                   (446, 0, 0, 0), (447, 0, 0, 0), (448, 0, 0, 0), (511, 0, 0, 0), (300, 40, 150, 30),
+                                   (31, 480, 0, 0), (3, 9, 500, 0), (40, 24, 0, 455)])
 def test_adjoint_of_mixed_classes_matches_the_tangent_linear_model(sizes):
     s = _system(*sizes)
     h, n_steps, every = s.h0, 3, 2
