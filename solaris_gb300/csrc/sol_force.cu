@@ -443,8 +443,6 @@ __global__ void __launch_bounds__(kSinkBlock) k_gravity_ac(ForceCtx fc, const do
 constexpr int kRefTile = 64;      // sources per round
 constexpr int kRefPerWarp = 10;   // sinks per summing warp: 30 of its 32 lanes
 constexpr int kRefMaxSinks = 21;  // of the two-warp form: 63 of 64 lanes
-// at least this many sources per sink (fewer: one thread per sink is cheaper)
-constexpr int kRefMinSources = 224;
 constexpr int kMaxDevices = 64;
 
 constexpr size_t ref_smem(int sw, int spc) {
@@ -1493,6 +1491,20 @@ static void ref_shape(int nsink, int nsm, int& spc, int& sw) {
   }
 }
 
+// Whether k_gravity_ac_ref is the faster one for ns sources (k_gravity_ac: a
+// thread a sink).  The thread's chain is 0.92 us a source until the sinks fill
+// the FP64 pipe (0.041 ns a pair); the other takes 4.2 us a tile of 64 sources
+// and, per sink, 1.7 ns a tile and 1.5 besides, whether the tile is full or not.
+// Measured (an evaluation, us, thread / tiles): 12 sources and 1,000 sinks 20 /
+// 16, 5,000 sinks 23 / 33; 64 and 20,000 110 / 88; 128 and 200 sinks 126 / 17,
+// 100,000 sinks 612 / 425; 3 sources and 256 sinks 11 / 14.
+static bool ref_pays(int ns, int nsink) {
+  const double tiles = (ns + kRefTile - 1) / kRefTile;
+  const double by_thread = 9.0 + ns * std::max(0.92, 0.6 + 4.1e-5 * nsink);
+  const double by_tiles = 8.0 + 4.2 * tiles + 1.0e-3 * nsink * (1.5 + 1.7 * tiles);
+  return ns >= 224 || by_thread > 1.15 * by_tiles;
+}
+
 static int launch_ref(sol_ctx* c, const ForceCtx& fc, const double* d_y, double* d_dydt, TimeSpec ts, uint32_t flags,
                       int nsink) {
   // per device: the SM count, once the kernels' shared-memory sizes are
@@ -1560,7 +1572,7 @@ static int force_launch(sol_ctx* c, const ForceCtx& fc, const double* d_y, doubl
     SOL_LAUNCHED();
     return SOL_OK;
   }
-  if (!split && c->cls.nm + c->cls.n_spl >= kRefMinSources) return launch_ref(c, fc, d_y, d_dydt, ts, flags, nsink);
+  if (!split && ref_pays(c->cls.nm + c->cls.n_spl, nsink)) return launch_ref(c, fc, d_y, d_dydt, ts, flags, nsink);
   if (split && !sol_force_uses_chunk_partials(c, c->precision)) {
     const int grid = (nsink + kFewSplitWarps - 1) / kFewSplitWarps;
     if (c->precision == SOL_PRECISION_SPLIT_FF)
