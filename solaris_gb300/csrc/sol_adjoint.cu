@@ -3,10 +3,11 @@
 // Solaris/RungeKuttaFehlberg78.cpp:147-250) with GravityAC forces
 // (Solaris/Acceleration.cpp:248-329).
 //
-// Forward: n fixed steps on the device, the state stored every K steps.
-// Backward, one segment of K steps at a time from the last: the segment is
-// recomputed from its checkpoint with every stage state Y_k (k = 0..10) of
-// every step kept; then, step by step from the last, the stage adjoints
+// Forward: n fixed steps on the device, the state stored every K steps, and of
+// the last K (or fewer) steps, where the backward pass begins, every stage
+// state Y_k (k = 0..10).  Backward, one segment of K steps at a time from the
+// last: the segment (but for the last one) is recomputed from its checkpoint
+// with its stage states kept; then, step by step from the last, the stage adjoints
 //   w_k = h b_k lambda + h sum_{j>k} a_jk nu_j,   nu_k = J(Y_k)^T w_k
 // and lambda_n = lambda_{n+1} + sum_k nu_k, with the mass gradient
 // accumulated from the same w_k.  Stages 11 and 12 only enter the error
@@ -494,6 +495,7 @@ struct sol_adjoint_state {
   double h = 0.0;
   double* d_cp = nullptr;     // checkpoints, (n_cp) x 6N
   double* d_stages = nullptr; // every x 11 x 6N stage states of one segment
+  int stages_of = -1;         // which segment's they are (-1: none that still holds)
   double* d_nu = nullptr;     // 11 x 6N stage adjoints
   double* d_lam = nullptr;    // 6N, and the next step's
   double* d_lam2 = nullptr;
@@ -515,6 +517,12 @@ void sol_adjoint_free(sol_adjoint_state* a) {
   delete a;
 }
 
+// The masses or the precision changed: stage states of the forward pass no
+// longer are what recomputing their segment gives.
+void sol_adjoint_model_changed(sol_ctx* c) {
+  if (c->adj) c->adj->stages_of = -1;
+}
+
 namespace {
 int set_fixed_h(sol_ctx* c, double h) {
   sol_ctrl hc;
@@ -523,6 +531,22 @@ int set_fixed_h(sol_ctx* c, double h) {
   hc.h_next = h;
   hc.eps = c->eps;
   SOL_CUDA(cudaMemcpyAsync(c->d_ctrl, &hc, sizeof(hc), cudaMemcpyHostToDevice, c->stream));
+  return SOL_OK;
+}
+
+size_t stage_doubles(const sol_adjoint_state* a, size_t nv) {
+  return (size_t)std::min(a->every, a->n_steps) * kAdjStages * nv;
+}
+
+// One step from `from` to `to` (which may be the same), its stage states to
+// step `slot` of the segment's
+int step_keeping_stages(sol_ctx* c, sol_adjoint_state* a, int slot, const double* from, double* to) {
+  const size_t nv = c->nv;
+  double* base = a->d_stages + (size_t)slot * kAdjStages * nv;
+  double* outs[13];
+  for (int k = 0; k < 13; ++k) outs[k] = k < kAdjStages ? base + (size_t)k * nv : nullptr;
+  SOL_CUDA(cudaMemcpyAsync(outs[0], from, sizeof(double) * nv, cudaMemcpyDeviceToDevice, c->stream));
+  RET(sol_rkf78_stages(c, outs[0], to, outs));
   return SOL_OK;
 }
 
@@ -581,15 +605,25 @@ extern "C" int sol_adjoint_forward(sol_ctx* c, double h, int32_t n_steps, int32_
     return SOL_OK;
   };
   RET(alloc(&a->d_cp, (size_t)a->n_cp * nv));
+  // the last segment's stage states, if there is room for them now
+  const int last = a->n_cp - 1;
+  if (cudaMalloc((void**)&a->d_stages, sizeof(double) * stage_doubles(a, nv)) != cudaSuccess) {
+    cudaGetLastError();
+    a->d_stages = nullptr;
+  }
   SOL_CUDA(cudaMemcpyAsync(c->d_y0, y0, sizeof(double) * nv, cudaMemcpyHostToDevice, c->stream));
   RET(set_fixed_h(c, h));
   for (int s = 0; s < n_steps; ++s) {
     if (s % every == 0)
       SOL_CUDA(cudaMemcpyAsync(a->d_cp + (size_t)(s / every) * nv, c->d_y0, sizeof(double) * nv,
                                cudaMemcpyDeviceToDevice, c->stream));
-    RET(sol_rkf78_stages(c, c->d_y0, c->d_y, nullptr));
+    if (a->d_stages && s >= last * every)
+      RET(step_keeping_stages(c, a, s - last * every, c->d_y0, c->d_y));
+    else
+      RET(sol_rkf78_stages(c, c->d_y0, c->d_y, nullptr));
     SOL_CUDA(cudaMemcpyAsync(c->d_y0, c->d_y, sizeof(double) * nv, cudaMemcpyDeviceToDevice, c->stream));
   }
+  if (a->d_stages) a->stages_of = last;
   c->state_valid = 1;
   if (y_final) SOL_CUDA(cudaMemcpyAsync(y_final, c->d_y0, sizeof(double) * nv, cudaMemcpyDeviceToHost, c->stream));
   SOL_CUDA(cudaStreamSynchronize(c->stream));
@@ -613,7 +647,7 @@ extern "C" int sol_adjoint_backward(sol_ctx* c, const double* dl_dy_final, doubl
     }
     return SOL_OK;
   };
-  RET(alloc(&a->d_stages, (size_t)a->every * kAdjStages * nv));
+  RET(alloc(&a->d_stages, stage_doubles(a, nv)));
   RET(alloc(&a->d_nu, (size_t)kAdjStages * nv));
   RET(alloc(&a->d_lam, nv));
   RET(alloc(&a->d_lam2, nv));
@@ -641,14 +675,12 @@ extern "C" int sol_adjoint_backward(sol_ctx* c, const double* dl_dy_final, doubl
     const int s0 = seg * a->every;
     const int s1 = std::min(a->n_steps, s0 + a->every);
     // recompute the segment, keeping the stage states Y_0..Y_10 of every step
-    SOL_CUDA(cudaMemcpyAsync(a->d_tmp, a->d_cp + (size_t)seg * nv, sizeof(double) * nv, cudaMemcpyDeviceToDevice,
-                             c->stream));
-    for (int s = s0; s < s1; ++s) {
-      double* base = a->d_stages + (size_t)(s - s0) * kAdjStages * nv;
-      double* outs[13];
-      for (int k = 0; k < 13; ++k) outs[k] = k < kAdjStages ? base + (size_t)k * nv : nullptr;
-      SOL_CUDA(cudaMemcpyAsync(outs[0], a->d_tmp, sizeof(double) * nv, cudaMemcpyDeviceToDevice, c->stream));
-      RET(sol_rkf78_stages(c, outs[0], a->d_tmp, outs));
+    if (a->stages_of != seg) {
+      a->stages_of = -1;
+      SOL_CUDA(cudaMemcpyAsync(a->d_tmp, a->d_cp + (size_t)seg * nv, sizeof(double) * nv, cudaMemcpyDeviceToDevice,
+                               c->stream));
+      for (int s = s0; s < s1; ++s) RET(step_keeping_stages(c, a, s - s0, a->d_tmp, a->d_tmp));
+      a->stages_of = seg;
     }
     // backward through the segment's steps
     int buf = 0;
@@ -716,6 +748,7 @@ extern "C" int sol_set_masses(sol_ctx* c, const double* mass) {
   SOL_CUDA(cudaSetDevice(c->device));
   SOL_CUDA(cudaMemcpyAsync(c->d_mass, mass, sizeof(double) * c->n, cudaMemcpyHostToDevice, c->stream));
   SOL_CUDA(cudaStreamSynchronize(c->stream));
+  sol_adjoint_model_changed(c);
   // captured driver graphs read masses from device memory: nothing to rebuild
   return SOL_OK;
 }

@@ -413,6 +413,7 @@ int sol_set_precision(sol_ctx* c, int32_t p) {
     RET(set_device(c));
     RET(dev_alloc(&c->d_part, (size_t)sol_force_part_doubles(c)));
   }
+  if (c->precision != p) sol_adjoint_model_changed(c);
   c->precision = p;
   c->fc.precision = p;
   return SOL_OK;

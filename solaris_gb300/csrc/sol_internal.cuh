@@ -138,6 +138,7 @@ long long sol_capture_count();
 
 struct sol_adjoint_state;
 void sol_adjoint_free(sol_adjoint_state* a);
+void sol_adjoint_model_changed(sol_ctx* c);
 
 struct sol_ctx {
   int device;
