@@ -138,26 +138,6 @@ __device__ __forceinline__ void rinv32(double r2, double& rm3, double& rm2) {
   }
 }
 
-// Eight sums over the warp in 9 additions a lane (40 for eight shuffle
-// trees): at the first three steps a lane hands half of its sums to its
-// partner and takes the other half.  Lane l ends with sum
-// 4 (l >> 4 & 1) + 2 (l >> 3 & 1) + (l >> 2 & 1).
-__device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
-#pragma unroll
-  for (int half = 4, off = 16; half >= 1; half >>= 1, off >>= 1) {
-    const bool up = (lane & off) != 0;
-#pragma unroll
-    for (int q = 0; q < half; ++q) {
-      const double send = up ? v[q] : v[q + half];
-      const double keep = up ? v[q + half] : v[q];
-      v[q] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-    }
-  }
-  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
-  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-  return v[0];
-}
-
 // Body k's part of nu, dm and d/d m_0 from its sums over the other bodies (tot)
 // and over the cotangents of its sinks (Wv), r, w_v of the body in x and wk:
 // part 0 to 2, a component of nu; 3, the masses.

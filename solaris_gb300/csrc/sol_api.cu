@@ -313,7 +313,7 @@ int sol_create(const sol_body_data* b, const sol_gas_component* gas, int32_t bar
       (rc = dev_alloc(&c->d_drag, 3 * (size_t)(cl.n_spl + cl.n_pl))) ||
       (rc = dev_alloc(&c->d_mig1, 3 * (size_t)(cl.n_rocky + cl.n_proto))) ||
       (rc = dev_alloc(&c->d_mig2, 3 * (size_t)cl.n_giant)) ||
-      (rc = dev_alloc(&c->d_ind_part, 6 * (size_t)sol_force_prepass_blocks(c->npad))) ||
+      (rc = dev_alloc(&c->d_ind_part, 7 * (size_t)sol_force_prepass_blocks(c->npad))) ||
       (rc = dev_alloc(&c->d_ind_sum, 8)) || (rc = dev_alloc(&c->d_y0, NV)) || (rc = dev_alloc(&c->d_y, NV)) ||
       (rc = dev_alloc(&c->d_accel, NV)) || (rc = dev_alloc(&c->d_yscale, NV)) || (rc = dev_alloc(&c->d_err, NV)) ||
       (rc = dev_alloc(&c->d_ytmp, NV)) || (rc = dev_alloc(&c->d_io_in, NV)))

@@ -7,7 +7,8 @@
 //                 GravityAC computes it (:256-264), and the structure-of-arrays
 //                 source table {x, y, z, G m, x rm3, y rm3, z rm3} that the pair
 //                 kernel streams; per-block partial sums of the indirect term.
-//   k_ind_reduce  one block: the indirect-term totals (SPLIT only).
+//   k_ind_reduce  one block: the indirect-term totals (split forms; k_split_table
+//                 does it where it runs).
 //   k_gravity_*   one thread per sink body; source tiles of TJ bodies are
 //                 staged in shared memory by bulk copies (cp.async.bulk, the
 //                 TMA engine) completing on an mbarrier, double buffered.  The
@@ -36,9 +37,8 @@ enum SrcArray { SX = 0, SY, SZ, SGM, SPX, SPY, SPZ, SGF, SRC_ARRAYS = 8 };  // S
 // G m as (hi, lo), one float array each (two sources load as one float2).
 enum FTab { FAX = 0, FBX, FCX, FAY, FBY, FCY, FAZ, FBZ, FCZ, FGH, FGL, FTAB_USED = 11, FTAB_ARRAYS = 12 };
 constexpr int kSrcDoubles = SRC_ARRAYS + FTAB_ARRAYS / 2;  // doubles per padded body in the source table
-// ind_sum slots: [0..5] the indirect sums, [6] the grid G1 of the float table,
-// [7] (low word) the running maximum |coordinate| as FP32 bits (atomicMax)
-constexpr int kIndGrid = 6, kIndMaxWord = 7;
+// ind_sum slots: [0..5] the indirect sums, [6] the grid G1 of the float table
+constexpr int kIndGrid = 6;
 
 constexpr int kChunkTiles = 16;             // sources per work unit of the 2-D pair kernel
 constexpr int kChunk = kChunkTiles * kTile;  // 4,096
@@ -111,78 +111,90 @@ __global__ void k_prepass(ForceCtx fc, const double* __restrict__ y, int split, 
       mbits = __float_as_uint(__double2float_ru(m));
     }
   }
-  if (ff) {
-    const unsigned wmax = __reduce_max_sync(0xFFFFFFFFu, mbits);
-    if ((threadIdx.x & 31) == 0 && wmax) atomicMax(reinterpret_cast<unsigned*>(fc.ind_sum + kIndMaxWord), wmax);
-  }
   if (!split) return;
-  // fixed-order block tree reduction of the indirect contributions
-  __shared__ double red[6][kPrepassBlock];
-  for (int k = 0; k < 6; ++k) red[k][threadIdx.x] = q[k];
+  // the block's sums of the indirect contributions, in a fixed order, and its largest |coordinate|
+  __shared__ double red[kPrepassBlock / 32][8];
+  __shared__ unsigned far[kPrepassBlock / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double v[8] = {q[0], q[1], q[2], q[3], q[4], q[5], 0.0, 0.0};
+  const double mine = warp_sum8(v, lane);
+  if ((lane & 3) == 0) red[warp][4 * (lane >> 4 & 1) + 2 * (lane >> 3 & 1) + (lane >> 2 & 1)] = mine;
+  const unsigned wmax = __reduce_max_sync(0xFFFFFFFFu, mbits);
+  if (lane == 0) far[warp] = wmax;
   __syncthreads();
-  for (int w = kPrepassBlock / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w)
-      for (int k = 0; k < 6; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + w];
-    __syncthreads();
+  if (threadIdx.x < 6) {
+    double t = red[0][threadIdx.x];
+    for (int w = 1; w < kPrepassBlock / 32; ++w) t += red[w][threadIdx.x];
+    fc.ind_part[6 * blockIdx.x + threadIdx.x] = t;
   }
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 6; ++k) fc.ind_part[6 * blockIdx.x + k] = red[k][0];
+  if (ff && threadIdx.x == 6) {
+    unsigned m = far[0];
+    for (int w = 1; w < kPrepassBlock / 32; ++w) m = max(m, far[w]);
+    fc.ind_part[6 * fc.n_ind_blocks + blockIdx.x] = __hiloint2double(0, (int)m);
+  }
 }
 
-__global__ void k_ind_reduce(ForceCtx fc) {
-  // one block of 256 threads: strided partial sums then a fixed tree.
-  __shared__ double red[6][256];
-  double a[6] = {0, 0, 0, 0, 0, 0};
-  for (int b = threadIdx.x; b < fc.n_ind_blocks; b += blockDim.x)
-    for (int k = 0; k < 6; ++k) a[k] += fc.ind_part[6 * b + k];
-  for (int k = 0; k < 6; ++k) red[k][threadIdx.x] = a[k];
+// The indirect-term totals from the blocks' sums, a warp each, by a block of 256
+// threads: [0..2] over [1, nm); [3..5] over [1, nm + n_spl).
+__device__ __forceinline__ void ind_totals(const ForceCtx& fc) {
+  __shared__ double tot[6];
+  const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (k < 6) {
+    double t = 0.0;
+    for (int b = lane; b < fc.n_ind_blocks; b += 32) t += fc.ind_part[6 * b + k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xFFFFFFFFu, t, o);
+    if (lane == 0) tot[k] = t;
+  }
   __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if (threadIdx.x < w)
-      for (int k = 0; k < 6; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    // [0..2]: sum over [1, nm); [3..5]: sum over [1, nm + n_spl)
-    for (int k = 0; k < 3; ++k) {
-      fc.ind_sum[k] = red[k][0];
-      fc.ind_sum[3 + k] = red[k][0] + red[3 + k][0];
-    }
-    // the float table's grid: G1 = 2^(E - 23) with every |coordinate| < 2^E
-    // (then read and cleared for the next evaluation's maximum)
-    unsigned* word = reinterpret_cast<unsigned*>(fc.ind_sum + kIndMaxWord);
-    const unsigned mb = *word;
-    const int E = mb ? (int)((mb >> 23) & 0xFFu) - 127 + 1 : 0;
-    fc.ind_sum[kIndGrid] = ldexp(1.0, max(E, -90) - 23);
-    *word = 0u;
-  }
+  if (threadIdx.x < 6) fc.ind_sum[threadIdx.x] = threadIdx.x < 3 ? tot[threadIdx.x] : tot[threadIdx.x - 3] + tot[threadIdx.x];
 }
+__global__ void __launch_bounds__(256) k_ind_reduce(ForceCtx fc) { ind_totals(fc); }
 
 // Grid triples of every coordinate (f2_grid_disp): a = G1 rint(x / G1),
 // b = G2 rint((x - a) / G2), c = float(x - a - b); a and b are exact floats
 // (at most 2^23 of their grid), x - a and x - a - b exact doubles.  Padding
 // bodies (no mass) are set apart from the others and from each other, so that
 // k_pairs_sym, which does not mask them, meets no close pair among them.
-__global__ void k_split_table(ForceCtx fc, const double* __restrict__ y, float* __restrict__ bound) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= fc.npad) return;
-  const double G1 = fc.ind_sum[kIndGrid];
-  const double G2 = G1 * 0x1.0p-24;
-  const double iG1 = 1.0 / G1, iG2 = 1.0 / G2;  // powers of two: exact
+// The grid G1 = 2^(E - 23), every |coordinate| < 2^E, each block takes from the
+// prepass blocks' maxima; block 0 also does k_ind_reduce's sums (a launch of its
+// own cost 5 us).
+__global__ void __launch_bounds__(kPrepassBlock) k_split_table(ForceCtx fc, const double* __restrict__ y,
+                                                               float* __restrict__ bound) {
+  __shared__ unsigned far[kPrepassBlock / 32];
+  const int j = blockIdx.x * kPrepassBlock + threadIdx.x;  // < npad, a whole number of blocks
+  double x[3] = {0.0, 0.0, 0.0};
+  if (j < fc.cls.n)
+    for (int k = 0; k < 3; ++k) x[k] = y[6 * j + k];
+  unsigned mb = 0;
+  for (int b = threadIdx.x; b < fc.n_ind_blocks; b += kPrepassBlock)
+    mb = max(mb, (unsigned)__double2loint(fc.ind_part[6 * fc.n_ind_blocks + b]));
+  mb = __reduce_max_sync(0xFFFFFFFFu, mb);
+  if ((threadIdx.x & 31) == 0) far[threadIdx.x >> 5] = mb;
+  __syncthreads();
+  for (int w = 0; w < kPrepassBlock / 32; ++w) mb = max(mb, far[w]);
+  const int E = max(mb ? (int)(mb >> 23) - 127 + 1 : 0, -90) - 23;
+  const double G1 = __hiloint2double((1023 + E) << 20, 0);
+  // adding and subtracting 1.5 2^52 G rounds to the grid G
+  const double M1 = __hiloint2double(((1023 + E + 52) << 20) | 0x80000, 0);
+  const double M2 = __hiloint2double(((1023 + E + 28) << 20) | 0x80000, 0);
   float* T = ftab(fc);
   const int np = fc.npad;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const double x = j < fc.cls.n ? y[6 * j + k] : 0.0;
-    const double a = rint(x * iG1) * G1;
-    const double r = x - a;
-    const double b = rint(r * iG2) * G2;
+    const double a = (x[k] + M1) - M1;
+    const double r = x[k] - a;
+    const double b = (r + M2) - M2;
     T[(size_t)(FAX + 3 * k) * np + j] = (float)a;
     T[(size_t)(FBX + 3 * k) * np + j] = (float)b;
     T[(size_t)(FCX + 3 * k) * np + j] = __double2float_rn(r - b);
   }
   if (bound) bound[j] = 3.0e38f;  // for k_near_bound
   if (j >= fc.cls.n) T[(size_t)FAX * np + j] = (float)((4194304.0 + 1024.0 * (j - fc.cls.n)) * G1);
+  if (blockIdx.x == 0) {
+    if (threadIdx.x == 0) fc.ind_sum[kIndGrid] = G1;
+    ind_totals(fc);
+  }
 }
 
 // ---- tile pipeline -----------------------------------------------------------
@@ -1060,12 +1072,12 @@ __global__ void __launch_bounds__(kSinkBlock, 3) k_pairs_ff(ForceCtx fc, const d
 #include "sol_pairs_sym.cuh"
 
 // Where the partials of an evaluation lie in the context's d_part (offsets in
-// doubles): of the block pairs of k_pairs_sym (bodies [0, 256 nb)), sources'
+// doubles): of the block pairs of k_pairs_sym (bodies [0, nb block)), sources'
 // and sinks' sides, and of k_pairs_ff on what is left: r1, every sink and the
 // sources from `from` on; r2, the sinks from there on and the sources before.
 struct FFPlan {
-  int nb = 0, per = 1, chunks = 0;  // k_pairs_sym
-  int from = 0;                                  // 256 nb
+  int block = kTile, nb = 0, per = 1, chunks = 0;  // k_pairs_sym
+  int from = 0;                                    // nb block
   int n1 = 0, chunk1 = kTile, n2 = 0, chunk2 = kTile;
   size_t o_j = 0, o_i = 0, o_1 = 0, o_2 = 0, o_bound = 0, doubles = 0;
 };
@@ -1075,24 +1087,28 @@ struct FFPlan {
 // distanceOfNN recomputed in the reference's FP64 arithmetic for the chosen
 // neighbour, the Kepler and indirect terms, and the gas terms.
 // Bounded by the latency of the partials' loads (a few tens to some hundreds a
-// sink, far apart): a CTA's warps share its sinks' partials, eight loaded at a
-// time, and the first warp adds the warps' sums and finishes (10,007 bodies:
-// 21 us for 65 with one thread a sink).
-constexpr int kCombineSinks = 32, kCombineWarps = 4;
+// sink, far apart) and by FP64: a CTA's warps share its sinks' partials, four
+// loaded at a time, a warp a component adds the warps' sums, and the first warp
+// finishes.  Block pairs' partials are few terms each and add up plainly (3 FP64
+// instructions a partial; their float-float sums carry 2^-46), the chunks of up
+// to 4,096 sources compensated (21).  10,007 bodies 18 us
+// (one thread a sink 65), 65,536 138 (213).
+constexpr int kCombineSinks = 32, kCombineWarps = 8, kCombineLoads = 4;
 
-__global__ void __launch_bounds__(kCombineSinks* kCombineWarps)
+__global__ void __launch_bounds__(kCombineSinks* kCombineWarps, 4)
     k_combine(ForceCtx fc, const double* __restrict__ y, double* __restrict__ dydt, const double* __restrict__ part,
               FFPlan pl, TimeSpec ts, uint32_t flags) {
   static_assert(kCombineSinks == 32, "a warp finishes");
   __shared__ double sh_s[kCombineWarps][6][32];
   __shared__ long long sh_r2[kCombineWarps][32];
   __shared__ int sh_nn[kCombineWarps][32];
+  __shared__ double sh_tot[3][32];
   const Classes& c = fc.cls;
   const int n = sol_sink_hi(fc);  // sinks [sink_lo, n)
   const int np = fc.npad;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int i = fc.sink_lo + blockIdx.x * kCombineSinks + lane;
-  double sx = 0.0, sy = 0.0, sz = 0.0, ex = 0.0, ey = 0.0, ez = 0.0;
+  double s[3] = {0.0, 0.0, 0.0}, e[3] = {0.0, 0.0, 0.0};
   long long best = __double_as_longlong(1.0e300);  // r^2 >= 0: the order of doubles is that of their bits
   int nn = -1;
   auto near = [&](long long r2, int j) {
@@ -1102,44 +1118,35 @@ __global__ void __launch_bounds__(kCombineSinks* kCombineWarps)
     }
   };
   // partials [0, count), at(k) the first word of partial k and `stride` its
-  // words' distance, loaded eight at a time; their plain sum is compensated
-  // (of_blocks: one block's terms each) or every one (a chunk's, up to 4,096)
+  // words' distance; of_blocks: of block pairs
   auto add = [&](int count, size_t stride, bool of_blocks, auto at) {
-    for (int g = 8 * warp; g < count; g += 8 * kCombineWarps) {
-      double v[8][PART_SLOTS];
+    for (int g = kCombineLoads * warp; g < count; g += kCombineLoads * kCombineWarps) {
+      double v[kCombineLoads][PART_SLOTS];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
+      for (int u = 0; u < kCombineLoads; ++u) {
         const double* p = at(min(g + u, count - 1));
 #pragma unroll
         for (int k = 0; k < PART_SLOTS; ++k) v[u][k] = p[k * stride];
       }
-      double t[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
+      for (int u = 0; u < kCombineLoads; ++u) {
         if (g + u >= count) break;
-        if (of_blocks) {
-          t[0] += v[u][PAX];
-          t[1] += v[u][PAY];
-          t[2] += v[u][PAZ];
-        } else {
-          two_sum(sx, ex, v[u][PAX]);
-          two_sum(sy, ey, v[u][PAY]);
-          two_sum(sz, ez, v[u][PAZ]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          if (of_blocks)
+            s[k] += v[u][PAX + k];
+          else
+            two_sum(s[k], e[k], v[u][PAX + k]);
         }
         near(__double_as_longlong(v[u][PR2]), (int)__double_as_longlong(v[u][PIDX]));
-      }
-      if (of_blocks) {
-        two_sum(sx, ex, t[0]);
-        two_sum(sy, ey, t[1]);
-        two_sum(sz, ez, t[2]);
       }
     }
   };
   if (i < n && i > 0) {
-    const int B = i / kSymBlock;
+    const int B = i / pl.block;
     if (B < pl.nb) {
-      const double* pj = part + pl.o_j + (i - B * kSymBlock);  // as a source of the blocks below
-      add(B, kSymBlock, true, [&](int I) { return pj + sym_pair_index(I, B, pl.nb) * PART_SLOTS * kSymBlock; });
+      const double* pj = part + pl.o_j + (i - B * pl.block);  // as a source of the blocks below
+      add(B, pl.block, true, [&](int I) { return pj + sym_pair_index(I, B, pl.nb) * PART_SLOTS * pl.block; });
       const int first = B / pl.per;  // as a sink of its own block's chunks
       const double* pi = part + pl.o_i + (size_t)first * PART_SLOTS * np + i;
       add(pl.chunks - first, np, true, [&](int k) { return pi + (size_t)k * PART_SLOTS * np; });
@@ -1148,14 +1155,23 @@ __global__ void __launch_bounds__(kCombineSinks* kCombineWarps)
     }
     add(pl.n1, np, false, [&](int k) { return part + pl.o_1 + (size_t)k * PART_SLOTS * np + i; });
   }
-  sh_s[warp][0][lane] = sx;
-  sh_s[warp][1][lane] = sy;
-  sh_s[warp][2][lane] = sz;
-  sh_s[warp][3][lane] = ex;
-  sh_s[warp][4][lane] = ey;
-  sh_s[warp][5][lane] = ez;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    sh_s[warp][k][lane] = s[k];
+    sh_s[warp][3 + k][lane] = e[k];
+  }
   sh_r2[warp][lane] = best;
   sh_nn[warp][lane] = nn;
+  __syncthreads();
+  if (warp < 3) {
+    double t = sh_s[0][warp][lane], l = sh_s[0][3 + warp][lane];
+#pragma unroll
+    for (int w = 1; w < kCombineWarps; ++w) {
+      two_sum(t, l, sh_s[w][warp][lane]);
+      l += sh_s[w][3 + warp][lane];
+    }
+    sh_tot[warp][lane] = t + l;
+  }
   __syncthreads();
   if (warp > 0 || i >= n) return;
   double* out = dydt + 6 * i;
@@ -1166,15 +1182,7 @@ __global__ void __launch_bounds__(kCombineSinks* kCombineWarps)
     return;
   }
 #pragma unroll
-  for (int w = 1; w < kCombineWarps; ++w) {
-    two_sum(sx, ex, sh_s[w][0][lane]);
-    two_sum(sy, ey, sh_s[w][1][lane]);
-    two_sum(sz, ez, sh_s[w][2][lane]);
-    ex += sh_s[w][3][lane];
-    ey += sh_s[w][4][lane];
-    ez += sh_s[w][5][lane];
-    near(sh_r2[w][lane], sh_nn[w][lane]);
-  }
+  for (int w = 1; w < kCombineWarps; ++w) near(sh_r2[w][lane], sh_nn[w][lane]);
   const double* yv = y + 6 * i;
   const int ns = (fc.type[i] <= SOL_PROTO_PLANET) ? c.nm + c.n_spl : c.nm;
   const double mu = SOL_GAUSS2 * (fc.mass[0] + fc.mass[i]);
@@ -1185,17 +1193,17 @@ __global__ void __launch_bounds__(kCombineSinks* kCombineWarps)
   a[1] = -mu * rm3i * yi;
   a[2] = -mu * rm3i * zi;
   const double* S = fc.ind_sum + ((fc.type[i] <= SOL_PROTO_PLANET) ? 3 : 0);
-  const double* s = fc.src;
+  const double* tab = fc.src;
   double own[3] = {0.0, 0.0, 0.0};
   if (i < ns) {
-    const double gmi = s[SGM * np + i];
-    own[0] = gmi * s[SPX * np + i];
-    own[1] = gmi * s[SPY * np + i];
-    own[2] = gmi * s[SPZ * np + i];
+    const double gmi = tab[SGM * np + i];
+    own[0] = gmi * tab[SPX * np + i];
+    own[1] = gmi * tab[SPY * np + i];
+    own[2] = gmi * tab[SPZ * np + i];
   }
-  a[0] += (sx + ex) - (S[0] - own[0]);
-  a[1] += (sy + ey) - (S[1] - own[1]);
-  a[2] += (sz + ez) - (S[2] - own[2]);
+  a[0] += sh_tot[0][lane] - (S[0] - own[0]);
+  a[1] += sh_tot[1][lane] - (S[1] - own[1]);
+  a[2] += sh_tot[2][lane] - (S[2] - own[2]);
   if (nn >= 0) {
     // the reference's rij for this j (Acceleration.cpp:301-305), bit for bit
     const double xij = y[6 * nn + 0] - xi, yij = y[6 * nn + 1] - yi, zij = y[6 * nn + 2] - zi;
@@ -1232,7 +1240,7 @@ __global__ void __launch_bounds__(kCombineSinks* kCombineWarps)
 // and is charged per warp instruction.
 constexpr int kFewSplitWarps = 8;
 constexpr int kFewSplitMax = 16384;  // SPLIT: the warp-per-sink kernel up to here
-constexpr int kFfMinBodies = 4096;   // SPLIT_FF: k_pairs_ff from here (below, the warp-per-sink kernel)
+constexpr int kFfMinBodies = 4096;   // SPLIT_FF: k_pairs_ff from here (below, the warp-per-sink kernel or k_pairs_sym)
 constexpr int kFoldRounds = 64;
 
 __device__ __forceinline__ void warp_two_sum(double& s, double& c) {
@@ -1413,31 +1421,44 @@ static int ff_chunk(int device, long nsink, long nsrc) {
 
 // How a SPLIT_FF evaluation is divided.  k_pairs_sym takes the massive bodies
 // (which attract each other) in whole blocks, the last one padded where every
-// body is massive; k_pairs_ff the rest.  From kSymMin bodies on, where the
-// block pairs fill the GPU (us an evaluation with it and without: 5,000 bodies
-// 188 and 144, 6,400 232 and 205, 7,168 232 and 256, 7,500 283 and 262, 7,936
-// 282 and 288, 9,000 341 and 378), up to kSymMax, beyond which the block pairs'
-// partials (10 KB each) would pass 1.4 GB.  One block of sources a CTA up to
-// kSymSingle blocks; above, two and then four halve the sinks' partials (336 MB
-// at 65,536 bodies) for much the same time (24,000 bodies: 1.61 ms with one,
-// 1.65 with two; 45,000: 5.36 and 5.41; 65,536: 11.17 and 11.19).
-constexpr int kSymMin = 7936, kSymMax = 131072, kSymSingle = 192;
+// body is massive; k_pairs_ff the rest.  From kSymMin bodies on (us an
+// evaluation with it and without: 1,025 bodies 65 and 52, 1,250 61 and 71, 2,049
+// 65 and 99, 3,100 85 and 145, 4,096 98 and 108, 7,000 191 and 236), kSymMinMixed
+// where others are left to k_pairs_ff (two launches more: 100 light bodies beside
+// 6,200 massive 204 and 192, beside 8,300 295 and 340), up to kSymMax, beyond
+// which the block pairs' partials (10 KB each) would pass 1.4 GB.  Small blocks are many and
+// short tasks, large ones have fewer partials (us with 64, 128 and 256 bodies:
+// 2,049 65, 90, 141; 10,007 339, 345, 383; 12,288 480, 459, 479; 16,384 808, 772,
+// 783; 24,000 1,679, 1,605, 1,583).  One block of sources a CTA up to kSymSingle
+// blocks; above, two and then four halve the sinks' partials (336 MB at 65,536
+// bodies) for much the same time (24,000 bodies: 1.61 ms with one, 1.65 with
+// two; 45,000: 5.36 and 5.41; 65,536: 11.17 and 11.19).
+constexpr int kSymMin = 1152, kSymMinMixed = 7168, kSymMax = 131072, kSymSingle = 192;
 
-static void sym_shape(FFPlan& p, int nb) {
+static int sym_block(int massive) { return massive < 11000 ? 64 : massive < 20000 ? 128 : 256; }
+// the bodies k_pairs_sym takes
+static int sym_bodies(int n, const Classes& cls) {
+  // every body massive: the last block padded; else whole tiles (k_pairs_ff goes on from one)
+  const int massive = cls.nm == n ? n : cls.nm / kTile * kTile;
+  return massive >= (cls.nm == n ? kSymMin : kSymMinMixed) && massive <= kSymMax ? massive : 0;
+}
+static void sym_shape(FFPlan& p, int block, int nb) {
+  p.block = block;
   p.nb = nb;
-  p.per = nb <= kSymSingle ? 1 : (nb <= 256 ? 2 : 4);
+  p.per = block < 256 || nb <= kSymSingle ? 1 : (nb <= 256 ? 2 : 4);
   p.chunks = (nb + p.per - 1) / p.per;
 }
 static size_t sym_doubles(const FFPlan& p, int npad) {
-  return ((size_t)p.nb * (p.nb - 1) / 2 * kSymBlock + (size_t)p.chunks * npad) * PART_SLOTS + npad;
+  return ((size_t)p.nb * (p.nb - 1) / 2 * p.block + (size_t)p.chunks * npad) * PART_SLOTS + npad;
 }
 
 static FFPlan ff_plan(int device, int n, const Classes& cls, int npad) {
   FFPlan p;
-  const int nb = (cls.nm == n ? n + kSymBlock - 1 : cls.nm) / kSymBlock;
-  if (nb >= kSymMin / kSymBlock && nb <= kSymMax / kSymBlock) {
-    sym_shape(p, nb);
-    p.from = nb * kSymBlock;
+  const int massive = sym_bodies(n, cls);
+  if (massive > 0) {
+    const int block = sym_block(massive);
+    sym_shape(p, block, (massive + block - 1) / block);
+    p.from = p.nb * block;
   }
   const int sources = cls.nm + cls.n_spl;
   if (p.nb == 0) {
@@ -1457,13 +1478,29 @@ static FFPlan ff_plan(int device, int n, const Classes& cls, int npad) {
     o += doubles;
     return at;
   };
-  p.o_j = take((size_t)p.nb * (p.nb > 0 ? p.nb - 1 : 0) / 2 * kSymBlock * PART_SLOTS);
+  p.o_j = take((size_t)p.nb * (p.nb > 0 ? p.nb - 1 : 0) / 2 * p.block * PART_SLOTS);
   p.o_i = take((size_t)p.chunks * PART_SLOTS * npad);
   p.o_1 = take((size_t)p.n1 * PART_SLOTS * npad);
   p.o_2 = take((size_t)p.n2 * PART_SLOTS * npad);
   p.o_bound = take(p.nb > 0 ? npad : 0);
   p.doubles = o;
   return p;
+}
+
+template <int BLOCK>
+static int launch_sym(sol_ctx* c, const ForceCtx& fc, const double* d_y, const FFPlan& p, const float* bound) {
+  static std::atomic<int> ready[kMaxDevices];  // the kernel's shared-memory size is allowed
+  const int dev = (c->device >= 0 && c->device < kMaxDevices) ? c->device : 0;
+  if (!ready[dev].load(std::memory_order_acquire)) {
+    SOL_CUDA(cudaFuncSetAttribute(k_pairs_sym<BLOCK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)sizeof(SymShared<BLOCK>)));
+    ready[dev].store(1, std::memory_order_release);
+  }
+  const int tasks = sym_tasks_above(p.chunks, p.per) + p.nb;
+  k_pairs_sym<BLOCK><<<tasks, sym_threads(BLOCK), sizeof(SymShared<BLOCK>), c->stream>>>(
+      fc, d_y, c->d_part + p.o_i, c->d_part + p.o_j, bound, p.nb, p.per);
+  SOL_LAUNCHED();
+  return SOL_OK;
 }
 
 // Sinks per CTA and summing warps of k_gravity_ac_ref: the CTAs spread over
@@ -1556,7 +1593,7 @@ static int force_launch(sol_ctx* c, const ForceCtx& fc, const double* d_y, doubl
     const int nb_pre = (fc.npad + kPrepassBlock - 1) / kPrepassBlock;
     k_prepass<<<nb_pre, kPrepassBlock, 0, c->stream>>>(fc, d_y, split, ff2d, d_clear);
     SOL_LAUNCHED();
-    if (split && !c->barycentric) {
+    if (split && !c->barycentric && !ff2d) {
       k_ind_reduce<<<1, 256, 0, c->stream>>>(fc);
       SOL_LAUNCHED();
     }
@@ -1586,20 +1623,14 @@ static int force_launch(sol_ctx* c, const ForceCtx& fc, const double* d_y, doubl
     int* status = &c->d_ctrl->dev_status;
     if (c->precision == SOL_PRECISION_SPLIT_FF) {
       if (plan.nb > 0) {
-        static std::atomic<int> sym_ready[kMaxDevices];
-        const int dev = (c->device >= 0 && c->device < kMaxDevices) ? c->device : 0;
-        if (!sym_ready[dev].load(std::memory_order_acquire)) {
-          SOL_CUDA(cudaFuncSetAttribute(k_pairs_sym, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)sizeof(SymShared)));
-          sym_ready[dev].store(1, std::memory_order_release);
-        }
-        k_near_bound<<<dim3(plan.nb, plan.nb < kBoundBlocks ? plan.nb : kBoundBlocks), kSymBlock, 0, c->stream>>>(
-            fc, bound, plan.nb);
+        const int tiles = (plan.from + kTile - 1) / kTile;
+        k_near_bound<<<dim3(tiles, (tiles < kBoundBlocks ? tiles : kBoundBlocks) * kBoundParts), kTile, 0, c->stream>>>(fc, bound,
+                                                                                                       tiles);
         SOL_LAUNCHED();
-        const int tasks = sym_tasks_above(plan.chunks, plan.per) + plan.nb;
-        k_pairs_sym<<<tasks, kSymThreads, sizeof(SymShared), c->stream>>>(
-            fc, d_y, c->d_part + plan.o_i, c->d_part + plan.o_j, bound, plan.nb, plan.per);
-        SOL_LAUNCHED();
+        const int r = plan.block == 64    ? launch_sym<64>(c, fc, d_y, plan, bound)
+                      : plan.block == 128 ? launch_sym<128>(c, fc, d_y, plan, bound)
+                                          : launch_sym<256>(c, fc, d_y, plan, bound);
+        if (r != SOL_OK) return r;
       }
       if (plan.n1 > 0) {
         k_pairs_ff<<<dim3(nb, plan.n1), kSinkBlock, 0, c->stream>>>(fc, d_y, c->d_part + plan.o_1, status,
@@ -1664,22 +1695,24 @@ size_t sol_force_part_doubles(const sol_ctx* c) {
     const size_t d = (size_t)((n + ch - 1) / ch) * PART_SLOTS * np;
     if (d > most) most = d;
   }
-  const int top = (c->cls.nm + kSymBlock - 1) / kSymBlock;
   size_t sym = 0;
-  for (int nb = kSymMin / kSymBlock; nb <= top && nb <= kSymMax / kSymBlock; ++nb) {
-    FFPlan p;
-    sym_shape(p, nb);
-    const size_t d = sym_doubles(p, c->npad);
-    if (d > sym) sym = d;
-  }
+  for (int m = 64; m <= c->cls.nm + 255 && m <= kSymMax + 255; m += 64)
+    for (int block = 64; block <= 256; block *= 2)
+      if (m % block == 0 && m >= kSymMin && (sym_block(m) == block || sym_block(m - block + 1) == block)) {
+        FFPlan p;
+        sym_shape(p, block, m / block);
+        const size_t d = sym_doubles(p, c->npad);
+        if (d > sym) sym = d;
+      }
   if (sym > 0 && c->cls.nm < c->n)  // k_pairs_ff on the rest, in chunks of one tile at the least
-    sym += ((size_t)(kSymBlock + c->cls.n_spl + kTile - 1) / kTile + top) * PART_SLOTS * np;
+    sym += ((size_t)(kTile + c->cls.n_spl + kTile - 1) / kTile + (c->cls.nm + kTile - 1) / kTile) * PART_SLOTS * np;
   return sym > most ? sym : most;
 }
 // whether the split forms of this system run the 2-D kernel (and need its
 // chunk partials); the same test as the dispatch in sol_force_launch_parts
 int sol_force_uses_chunk_partials(const sol_ctx* c, int precision) {
   const int few_max = precision == SOL_PRECISION_SPLIT_FF ? kFfMinBodies - 1 : kFewSplitMax;
+  if (precision == SOL_PRECISION_SPLIT_FF && sym_bodies(c->n, c->cls) > 0) return 1;
   return !(c->n <= few_max && c->cls.nm + c->cls.n_spl >= kTile);
 }
 int sol_force_prepass_blocks(int npad) { return (npad + kPrepassBlock - 1) / kPrepassBlock; }
@@ -1699,7 +1732,7 @@ constexpr int kNoAllocPrepassBlocks = kNoAllocMaxBodies / kPrepassBlock;
 constexpr size_t kNoAllocSrc = (size_t)SRC_ARRAYS * kNoAllocMaxBodies;
 constexpr size_t kNoAllocPart = 6 * (size_t)kNoAllocPrepassBlocks;
 constexpr size_t kNoAllocDoubles = kNoAllocSrc + kNoAllocPart + 8 /* sums */ + 8 /* status */;
-static_assert(kSymBlock == kTile && kTile % kSinkBlock == 0, "blocks of sources are whole tiles, tiles whole sink blocks");
+static_assert(kTile == 256 && kTile % kSinkBlock == 0, "tiles are whole blocks of every size, and whole sink blocks");
 static_assert(kNoAllocMaxBodies % kTile == 0, "scratch must hold whole tiles");
 }  // namespace
 

@@ -50,6 +50,26 @@ __device__ __forceinline__ void ff_from_double(double d, float& h, float& l) {
   l = __uint_as_float(__float_as_uint(m) | sign);
 }
 
+// Eight sums over the warp in 9 additions a lane (40 for eight shuffle
+// trees): at the first three steps a lane hands half of its sums to its
+// partner and takes the other half.  Lane l ends with sum
+// 4 (l >> 4 & 1) + 2 (l >> 3 & 1) + (l >> 2 & 1).
+__device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
+#pragma unroll
+  for (int half = 4, off = 16; half >= 1; half >>= 1, off >>= 1) {
+    const bool up = (lane & off) != 0;
+#pragma unroll
+    for (int q = 0; q < half; ++q) {
+      const double send = up ? v[q] : v[q + half];
+      const double keep = up ? v[q + half] : v[q];
+      v[q] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    }
+  }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+  return v[0];
+}
+
 // Float-float pair: FP64 displacement (3 DADD, the only FP64 instructions),
 // r^2 with exact squares and sums, FP32 rsqrt seed and one Newton correction
 // r^-3 = y^3 (1 + 3/2 e + 15/8 e^2) with e = 1 - r^2 y^2 evaluated from exact

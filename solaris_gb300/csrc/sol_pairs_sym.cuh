@@ -7,7 +7,7 @@
 // pair costs 62 FP32 operations shared by its two terms and 42 for each term,
 // 73 a term instead of 106.5.
 //
-// Bodies are taken in blocks of 256.  A CTA has a block I of sinks, two a
+// Bodies are taken in blocks of 64, 128 or 256.  A CTA has a block I of sinks, two a
 // thread (the two lanes of its paired FP32 instructions: a warp's 64 sinks),
 // and runs over the source blocks J >= I of a chunk.  Within a warp the 32
 // lanes work on 32 different sources at a time; a source's sums travel from
@@ -25,8 +25,8 @@
 // sol_accel_sinks_device): what is computed keeps its order and so its bits.
 //
 // Bounded by the FP32 pipe: 73 operations a term are 7.8 ms at 65,536 bodies;
-// the kernel takes 10.7 (73 %), an evaluation 11.2 for 13.9 before, of 10,007
-// bodies 398 us for 455, of 16,384 0.80 ms for 0.99.  Its error against the
+// the kernel takes 10.7 (73 %), an evaluation 11.1 for 13.9 before, of 16,384
+// bodies 0.77 ms for 0.99, of 10,007 339 us for 455, of 2,049 65 for 99.  Its error against the
 // reference form is no larger: bodies of comparable pull on each other as from
 // the centre, 8,000 to 16,384 of them, 24 systems: median of the largest 1.5e-13
 // for 2.0e-13, rms 9.4e-15 for 1.0e-14.
@@ -35,25 +35,26 @@
 // sink takes the FP64 term at once, the source's side is marked and evaluated
 // after the block pair by a pass over it in source order (sym_close_pass).
 
-constexpr int kSymBlock = 256;                   // bodies per block, and sources per tile
-constexpr int kSymWarps = kSymBlock / 64;        // two sinks a thread
-constexpr int kSymThreads = 32 * kSymWarps;
+// Bodies per block (and sources per tile): BLOCK, 64 to 256; a thread has two sinks.
+__host__ __device__ constexpr int sym_threads(int block) { return block / 2; }
 // Four CTAs an SM (128 registers): measured at 65,536 bodies 10.7 ms against
 // 11.3 with three (144 registers), and 11.3 against 12.1 before the bounds of
 // k_near_bound; one source at a time a warp -- two interleaved take 160
 // registers and three CTAs -- 12.0.
-constexpr int kSymCtas = 4;
+__host__ __device__ constexpr int sym_ctas(int block) { return 1024 / block; }
 
 // A source's table entries, each twice (both lanes of a paired operand), two
 // to a 16-byte load.
 constexpr int kSymRows = (kFF + 1) / 2;
+template <int BLOCK>
 struct SymTile {
-  float4 v[kSymRows][kSymBlock];
+  float4 v[kSymRows][BLOCK];
 };
 struct SymSource {
   float2 v[2 * kSymRows];
 };
-__device__ __forceinline__ SymSource sym_load(const SymTile& T, int q) {
+template <int BLOCK>
+__device__ __forceinline__ SymSource sym_load(const SymTile<BLOCK>& T, int q) {
   SymSource s;
 #pragma unroll
   for (int k = 0; k < kSymRows; ++k) {
@@ -63,15 +64,16 @@ __device__ __forceinline__ SymSource sym_load(const SymTile& T, int q) {
   }
   return s;
 }
+template <int BLOCK>
 struct SymShared {
-  SymTile tile;
-  double js[3][kSymBlock];  // sums of the sources of J
-  float jmh[kSymBlock], jml[kSymBlock];  // their nearest sink of I
-  int jnn[kSymBlock];
+  SymTile<BLOCK> tile;
+  double js[3][BLOCK];  // sums of the sources of J
+  float jmh[BLOCK], jml[BLOCK];  // their nearest sink of I
+  int jnn[BLOCK];
   int close;
   // a thread's FP64 sums of its two sinks: totals, compensation, close pairs
   // (here, not in registers: they change every 128 sources only)
-  double sums[3][6][kSymThreads];
+  double sums[3][6][sym_threads(BLOCK)];
 };
 
 // Nearest neighbour of one body: the smallest r^2 (hi, then lo), ties to the lower index.
@@ -116,7 +118,8 @@ __device__ __forceinline__ void sym_displacement(const SymSource& J, const SymSi
 
 // A source's nearest sink in the CTA's shared arrays: read always, written
 // when a sink is nearer (about ln N times)
-__device__ __forceinline__ void sym_near_source(SymShared& sm, int q, const SymSinks& S, int ns, float2 r2h,
+template <int BLOCK>
+__device__ __forceinline__ void sym_near_source(SymShared<BLOCK>& sm, int q, const SymSinks& S, int ns, float2 r2h,
                                                 float2 r2l) {
   SymNear m = {sm.jmh[q], sm.jml[q], sm.jnn[q]};
   sym_near(m, r2h.x, r2l.x, (S.i0 >= 1) & (S.i0 < ns), S.i0);
@@ -155,8 +158,8 @@ __device__ __forceinline__ void sym_terms(const float2* h, const float2* l, floa
   }
 }
 
-template <bool DI, bool DJ, bool SECOND>
-__device__ __forceinline__ void sym_step(SymShared& sm, const ForceCtx& fc, const double* __restrict__ y, int q,
+template <bool DI, bool DJ, bool SECOND, int BLOCK>
+__device__ __forceinline__ void sym_step(SymShared<BLOCK>& sm, const ForceCtx& fc, const double* __restrict__ y, int q,
                                          int from, int j0, int ns, float thr, const SymSinks& S, SymSums& A,
                                          SymNear& n0, SymNear& n1, SymSums& B) {
   float2 h[3], l[3], r2h, r2l;
@@ -206,8 +209,8 @@ __device__ __forceinline__ void sym_step(SymShared& sm, const ForceCtx& fc, cons
 
 // 32 steps of a warp: its 64 sinks past the 32 sources of part `sub` of the
 // tile.  DI / DJ: the sinks' / the sources' sums.
-template <bool DI, bool DJ>
-__device__ __forceinline__ void sym_part(SymShared& sm, const ForceCtx& fc, const double* __restrict__ y, int sub,
+template <bool DI, bool DJ, int BLOCK>
+__device__ __forceinline__ void sym_part(SymShared<BLOCK>& sm, const ForceCtx& fc, const double* __restrict__ y, int sub,
                                          int lane, int j0, int ns, float thr, const SymSinks& S, SymSums& A,
                                          SymNear& n0, SymNear& n1, SymSums& B) {
   const int from = (lane + 1) & 31;
@@ -220,17 +223,18 @@ __device__ __forceinline__ void sym_part(SymShared& sm, const ForceCtx& fc, cons
 }
 
 // The source side of the close pairs of a block pair, in sink order.
-__device__ __noinline__ void sym_close_pass(SymShared& sm, const ForceCtx& fc, const double* __restrict__ y, int i0,
+template <int BLOCK>
+__device__ __noinline__ void sym_close_pass(SymShared<BLOCK>& sm, const ForceCtx& fc, const double* __restrict__ y, int i0,
                                             int j0, int ns, float thr) {
   const float* T = ftab(fc);
   const int np = fc.npad;
-  for (int q = threadIdx.x; q < kSymBlock; q += kSymThreads) {
+  for (int q = threadIdx.x; q < BLOCK; q += sym_threads(BLOCK)) {
     const int j = j0 + q;
     if (j >= ns) continue;
     const double* p = y + 6 * (size_t)j;
     const SymSource J = sym_load(sm.tile, q);
     double f[3] = {0.0, 0.0, 0.0};
-    for (int i = i0; i < min(i0 + kSymBlock, ns); ++i) {
+    for (int i = i0; i < min(i0 + BLOCK, ns); ++i) {
       float2 h[3], l[3], r2h, r2l;
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
@@ -257,22 +261,25 @@ __device__ __noinline__ void sym_close_pass(SymShared& sm, const ForceCtx& fc, c
 // there, so that a new minimum is rare (without it every block pair begins
 // with ~5 updates a body, and hardly a step of a warp has none).
 constexpr int kBoundBlocks = 4;
-__global__ void __launch_bounds__(kSymBlock) k_near_bound(ForceCtx fc, float* __restrict__ bound, int nb) {
-  __shared__ float2 sx[kSymBlock], sy[kSymBlock], sz[kSymBlock];
+constexpr int kBoundParts = 4, kBoundSources = kTile / kBoundParts;  // a block in quarters: a shorter chain
+__global__ void __launch_bounds__(kTile) k_near_bound(ForceCtx fc, float* __restrict__ bound, int nb) {
+  __shared__ float2 sx[kBoundSources], sy[kBoundSources], sz[kBoundSources];
   const float* T = ftab(fc);
   const int np = fc.npad, ns = fc.cls.nm;
-  const int i = blockIdx.x * kSymBlock + threadIdx.x;
-  const int j0 = ((blockIdx.x + blockIdx.y) % nb) * kSymBlock;
+  const int i = blockIdx.x * kTile + threadIdx.x;
+  const int j0 = ((blockIdx.x + blockIdx.y / kBoundParts) % nb) * kTile + blockIdx.y % kBoundParts * kBoundSources;
   auto at = [&](int k, int j) {
     return make_float2(T[(size_t)(FAX + 3 * k) * np + j], T[(size_t)(FBX + 3 * k) * np + j]);
   };
   const float2 x = at(0, i), yy = at(1, i), z = at(2, i);
-  sx[threadIdx.x] = at(0, j0 + threadIdx.x);
-  sy[threadIdx.x] = at(1, j0 + threadIdx.x);
-  sz[threadIdx.x] = at(2, j0 + threadIdx.x);
+  if (threadIdx.x < kBoundSources) {
+    sx[threadIdx.x] = at(0, j0 + threadIdx.x);
+    sy[threadIdx.x] = at(1, j0 + threadIdx.x);
+    sz[threadIdx.x] = at(2, j0 + threadIdx.x);
+  }
   __syncthreads();
   float m = 3.0e38f;
-  const int q1 = min(kSymBlock, ns - j0);
+  const int q1 = min(kBoundSources, ns - j0);
 #pragma unroll 8
   for (int q = j0 == 0 ? 1 : 0; q < q1; ++q) {
     const float dx = (sx[q].x - x.x) + (sx[q].y - x.y), dy = (sy[q].x - yy.x) + (sy[q].y - yy.y),
@@ -285,7 +292,7 @@ __global__ void __launch_bounds__(kSymBlock) k_near_bound(ForceCtx fc, float* __
 }
 
 // part_i: [chunk][PART_SLOTS][npad] as k_pairs_ff's; part_j: per block pair
-// I < J, packed by I, [PART_SLOTS][kSymBlock].
+// I < J, packed by I, [PART_SLOTS][BLOCK].
 __device__ __forceinline__ size_t sym_pair_index(int I, int J, int nb) {
   return (size_t)I * (nb - 1) - (size_t)I * (I - 1) / 2 + (J - I - 1);
 }
@@ -294,11 +301,13 @@ __device__ __forceinline__ size_t sym_pair_index(int I, int J, int nb) {
 // has per c of them.
 __host__ __device__ __forceinline__ int sym_tasks_above(int C, int per) { return per * (C * (C - 1) / 2); }
 
-__global__ void __launch_bounds__(kSymThreads, kSymCtas)
+template <int BLOCK>
+__global__ void __launch_bounds__(sym_threads(BLOCK), sym_ctas(BLOCK))
     k_pairs_sym(ForceCtx fc, const double* __restrict__ y, double* __restrict__ part_i, double* __restrict__ part_j,
                 const float* __restrict__ bound, int nb, int per) {
   extern __shared__ __align__(16) unsigned char sym_dyn[];
-  SymShared& sm = *reinterpret_cast<SymShared*>(sym_dyn);
+  SymShared<BLOCK>& sm = *reinterpret_cast<SymShared<BLOCK>*>(sym_dyn);
+  constexpr int kThreads = sym_threads(BLOCK), kParts = BLOCK / 32;
   // The CTA's block of sinks I and its chunk C of `per` blocks of sources: first
   // the chunks above I's own, by chunk, then the nb of I's own, whose diagonal
   // block takes less, so that the last to start are short.  No CTA is launched
@@ -320,12 +329,12 @@ __global__ void __launch_bounds__(kSymThreads, kSymCtas)
   const int Jlo = max(I, C * per), Jhi = min(nb, (C + 1) * per);
   const int np = fc.npad, ns = fc.cls.nm;
   const int lo = fc.sink_lo, hi = sol_sink_hi(fc);
-  auto wanted = [&](int B) { return B * kSymBlock < hi && (B + 1) * kSymBlock > lo; };
+  auto wanted = [&](int B) { return B * BLOCK < hi && (B + 1) * BLOCK > lo; };
   const bool want_i = wanted(I);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float* T = ftab(fc);
   SymSinks S;
-  S.i0 = I * kSymBlock + warp * 64 + lane;
+  S.i0 = I * BLOCK + warp * 64 + lane;
   S.i1 = S.i0 + 32;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
@@ -342,16 +351,16 @@ __global__ void __launch_bounds__(kSymThreads, kSymCtas)
   for (int J = Jlo; J < Jhi; ++J) {
     const bool want_j = J != I && wanted(J);
     if (!want_i && !want_j) continue;
-    const int j0 = J * kSymBlock;
+    const int j0 = J * BLOCK;
     __syncthreads();
 #pragma unroll 1
     for (int k = 0; k < kSymRows; ++k)
-      for (int q = threadIdx.x; q < kSymBlock; q += kSymThreads) {
+      for (int q = threadIdx.x; q < BLOCK; q += kThreads) {
         const float v = T[(size_t)(2 * k) * np + j0 + q];
         const float w = 2 * k + 1 < kFF ? T[(size_t)(2 * k + 1) * np + j0 + q] : 0.0f;
         sm.tile.v[k][q] = make_float4(v, v, w, w);
       }
-    for (int q = threadIdx.x; q < kSymBlock; q += kSymThreads) {
+    for (int q = threadIdx.x; q < BLOCK; q += kThreads) {
       sm.js[0][q] = sm.js[1][q] = sm.js[2][q] = 0.0;
       sm.jmh[q] = bound[j0 + q];
       sm.jml[q] = 3.0e38f;
@@ -363,8 +372,8 @@ __global__ void __launch_bounds__(kSymThreads, kSymCtas)
 #pragma unroll
     for (int k = 0; k < 3; ++k) A.h[k] = A.l[k] = make_float2(0.0f, 0.0f);
 #pragma unroll 1
-    for (int p = 0; p < 8; ++p) {
-      const int sub = (p + 2 * warp) & 7;  // a part of its own for every warp
+    for (int p = 0; p < kParts; ++p) {
+      const int sub = (p + 2 * warp) & (kParts - 1);  // a part of its own for every warp
       const int q = sub * 32 + lane;
       SymSums B;
 #pragma unroll
@@ -380,13 +389,13 @@ __global__ void __launch_bounds__(kSymThreads, kSymCtas)
         for (int k = 0; k < 3; ++k)
           sm.js[k][q] += ((double)B.h[k].x + (double)B.l[k].x) + ((double)B.h[k].y + (double)B.l[k].y);
       }
-      if (want_i && (p & 3) == 3) {  // the sinks' float-float sums of 128 sources into FP64
+      if (want_i && ((p & 3) == 3 || p == kParts - 1)) {  // the sinks' float-float sums of 128 sources into FP64
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
           double* t = &sm.sums[0][k][threadIdx.x];
           double* c = &sm.sums[1][k][threadIdx.x];
           two_sum(t[0], c[0], (double)A.h[k].x + (double)A.l[k].x);
-          two_sum(t[3 * kSymThreads], c[3 * kSymThreads], (double)A.h[k].y + (double)A.l[k].y);
+          two_sum(t[3 * kThreads], c[3 * kThreads], (double)A.h[k].y + (double)A.l[k].y);
           A.h[k] = A.l[k] = make_float2(0.0f, 0.0f);
         }
       }
@@ -394,16 +403,16 @@ __global__ void __launch_bounds__(kSymThreads, kSymCtas)
     }
     if (want_j) {
       if (sm.close) {
-        sym_close_pass(sm, fc, y, I * kSymBlock, j0, ns, thr);
+        sym_close_pass(sm, fc, y, I * BLOCK, j0, ns, thr);
         __syncthreads();
       }
-      double* out = part_j + sym_pair_index(I, J, nb) * PART_SLOTS * kSymBlock;
-      for (int q = threadIdx.x; q < kSymBlock; q += kSymThreads) {
-        out[PAX * kSymBlock + q] = sm.js[0][q];
-        out[PAY * kSymBlock + q] = sm.js[1][q];
-        out[PAZ * kSymBlock + q] = sm.js[2][q];
-        out[PR2 * kSymBlock + q] = sm.jnn[q] >= 0 ? (double)sm.jmh[q] + (double)sm.jml[q] : 1.0e300;
-        out[PIDX * kSymBlock + q] = __longlong_as_double((long long)sm.jnn[q]);
+      double* out = part_j + sym_pair_index(I, J, nb) * PART_SLOTS * BLOCK;
+      for (int q = threadIdx.x; q < BLOCK; q += kThreads) {
+        out[PAX * BLOCK + q] = sm.js[0][q];
+        out[PAY * BLOCK + q] = sm.js[1][q];
+        out[PAZ * BLOCK + q] = sm.js[2][q];
+        out[PR2 * BLOCK + q] = sm.jnn[q] >= 0 ? (double)sm.jmh[q] + (double)sm.jml[q] : 1.0e300;
+        out[PIDX * BLOCK + q] = __longlong_as_double((long long)sm.jnn[q]);
       }
     }
   }

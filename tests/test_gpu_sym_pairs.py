@@ -1,16 +1,18 @@
-"""The float-float kernel over pairs of blocks (k_pairs_sym, from 31 blocks of 256
-massive bodies) against the reference (FP64) form on the device.
+"""The float-float kernel over pairs of blocks (k_pairs_sym, from 1,152 massive
+bodies) against the reference (FP64) form on the device.
 
-Sizes: where the path begins, whole blocks of 256 bodies and one more or less
-(the last block is padded when every body is massive, left to k_pairs_ff when
-not), both sides of 192 and 256 blocks (one, two and four blocks of sources a
-CTA, with and without a remainder), beyond the path's end, and light bodies in
-numbers that leave the last massive block empty, nearly empty and nearly full.
-Pairs are planted closer than the grid step (FP64 arithmetic, on both bodies'
-sides) inside one block, in neighbouring blocks, in the first and last block,
-and across the end of the whole blocks.  Bound: 1e-12 relative acceleration error per body, as the
-form's other kernel's; nearest neighbours and their distances are equal.  A
-block of sinks alone gives the same bits as the whole evaluation."""
+Sizes: where the path begins (every body massive, or light bodies besides),
+whole blocks of 64, 128 and 256 bodies, the sizes at which the blocks grow, and
+one more or less (the last block is padded when every body is massive, left to
+k_pairs_ff when not), both sides of 192 and 256 blocks of 256 (one, two and four
+blocks of sources a CTA, with and without a remainder), beyond the path's end,
+and light bodies in numbers that leave the last massive block empty, nearly
+empty and nearly full.  Pairs are planted closer than the grid step (FP64
+arithmetic, on both bodies' sides) inside one block, in neighbouring blocks, in
+the first and last block, and across the end of the whole blocks.  Bound: 1e-12
+relative acceleration error per body, as the form's other kernel's; nearest
+neighbours and their distances are equal.  A block of sinks alone gives the same
+bits as the whole evaluation."""
 import numpy as np
 import pytest
 
@@ -47,9 +49,10 @@ def _system(n_massive, n_spl=0, n_light=0, seed=91):
     return scenarios._assemble("sym_pairs", groups), pairs
 
 
-@pytest.mark.parametrize("sizes", [(7680,), (7681,), (7935,), (7936,), (7937,), (10007,), (49152,), (49153,), (49409,),
-                                   (66000,), (131073,), (7935, 0, 5), (7936, 3, 0), (7937, 0, 700), (8191, 300, 1),
-                                   (49664, 1, 130)])
+@pytest.mark.parametrize("sizes", [(1151,), (1152,), (1153,), (1343,), (1344,), (2049,), (10007,), (10999,), (11000,), (11137,),
+                                   (19999,), (20000,), (20225,), (49152,), (49153,), (49409,), (66000,), (131073,),
+                                   (7167, 0, 5), (7168, 3, 0), (7423, 0, 700), (7424, 300, 1), (11008, 1, 130),
+                                   (11009, 40, 600), (20224, 0, 77), (49664, 1, 130)])
 def test_block_pairs_against_the_reference_form(sizes):
     s, pairs = _system(*sizes)
     with engine.Context(s, precision=abi.PRECISION_FP64) as ctx:
@@ -68,7 +71,7 @@ def test_block_pairs_against_the_reference_form(sizes):
     assert np.array_equal(again.view(np.uint64), dff.view(np.uint64))
 
 
-@pytest.mark.parametrize("sizes", [(9000,), (8198, 40, 900)])
+@pytest.mark.parametrize("sizes", [(1500,), (9000,), (8198, 40, 900)])
 def test_sink_blocks_of_block_pairs_equal_the_whole(sizes):
     torch = pytest.importorskip("torch")
     s, _ = _system(*sizes)
@@ -78,7 +81,7 @@ def test_sink_blocks_of_block_pairs_equal_the_whole(sizes):
         y = torch.from_numpy(s.y0.copy()).to(dev)
         out = torch.full((6 * s.n,), float("nan"), dtype=torch.float64, device=dev)
         torch.cuda.synchronize()
-        cuts = [0, 1, 255, 600, 8191, 8195, s.n]
+        cuts = [c for c in (0, 1, 255, 600, 8191, 8195) if c < s.n] + [s.n]
         for lo, hi in zip(cuts, cuts[1:]):
             abi.check(ctx.lib, ctx.lib.sol_accel_sinks_device(ctx.h, 0.0, y.data_ptr(), lo, hi, out.data_ptr()))
             assert np.array_equal(ctx.last_eval()[1][lo:hi], nn[lo:hi])
