@@ -192,7 +192,7 @@ def run_reference(args, rank, world):
     replicas.finalize()
 
 
-def profile_figures(names=("pair_kernels_65536.md", "k_pairs_ff_65536.md")):
+def profile_figures(names=("pair_kernels_65536.md", "k_pairs_sym_65536.md")):
     """`key: value` lines of the committed ncu summaries (DRAM bytes per
     launch, instructions per pair measured at the bench size); later files
     override earlier ones."""
@@ -217,7 +217,7 @@ def _figures(p):
     return out
 
 
-FF_FP32_OPS_PER_PAIR = 106.5
+FF_FP32_OPS_PER_PAIR = 71.5  # per ordered pair: 59 shared by the two terms of an unordered pair, 42 a term
 # The FP32 pipe completes 128 lane operations per SM cycle (4 sub-partitions x
 # 32 lanes; a paired FFMA2 instruction is two).
 FP32_LANES_PER_SM_CYCLE = 128.0
@@ -245,11 +245,11 @@ def roofline_entry(name, pps, fp64_ops, fp32_ops, peak64, info64, peak32, info32
     traffic = {"traffic": prof.get(f"{name}_dram_bytes_per_launch"),
                "traffic_note": "ncu dram__bytes_read.sum + dram__bytes_write.sum of the pair kernel and its "
                                "k_combine at 65,536 bodies (profiles/pair_kernels_65536.md, "
-                               "profiles/k_pairs_ff_65536.md; SPLIT_FF with the caches as the timed step "
+                               "profiles/k_pairs_sym_65536.md; SPLIT_FF with the caches as the timed step "
                                "leaves them, --cache-control none)",
                "kernel_ms_per_launch": ms}
     if name in fp32_ops:
-        return {"bound": "fp32", "kernel": "k_pairs_ff (SPLIT_FF pair kernel) + k_combine",
+        return {"bound": "fp32", "kernel": "k_pairs_sym (SPLIT_FF pair kernel) + k_combine",
                 "achieved": pps * fp32_ops[name] / 1e9, "peak": peak32 / 1e9, "unit": "Gop/s",
                 "frac": pps * fp32_ops[name] / peak32, **traffic, "fp32_ops_per_pair": fp32_ops[name],
                 "fp64_instructions_per_pair_ncu": prof.get(f"{name}_fp64_instructions_per_pair"),

@@ -4,8 +4,8 @@
 // A pair's displacement, r^2 and r^-3 are the same numbers seen from either
 // body (d changes its sign, exactly), and both bodies take a term from it:
 // G m_j r^-3 d on i, -G m_i r^-3 d on j.  k_pairs_ff forms them twice; here a
-// pair costs 62 FP32 operations shared by its two terms and 42 for each term,
-// 73 a term instead of 106.5.
+// pair costs 59 FP32 operations shared by its two terms and 42 for each term,
+// 71.5 a term instead of 103.5.
 //
 // Bodies are taken in blocks of 64, 128 or 256.  A CTA has a block I of sinks, two a
 // thread (the two lanes of its paired FP32 instructions: a warp's 64 sinks),
@@ -24,8 +24,8 @@
 // Either side of a block pair can be left out (a block of sinks alone,
 // sol_accel_sinks_device): what is computed keeps its order and so its bits.
 //
-// Bounded by the FP32 pipe: 73 operations a term are 7.8 ms at 65,536 bodies;
-// the kernel takes 10.7 (73 %), an evaluation 11.1 for 13.9 before, of 16,384
+// Bounded by the FP32 pipe: 71.5 operations a term are 7.6 ms at 65,536 bodies;
+// the kernel takes 10.6 (72 %), an evaluation 10.96 for 13.9 before, of 16,384
 // bodies 0.77 ms for 0.99, of 10,007 339 us for 455, of 2,049 65 for 99.  Its error against the
 // reference form is no larger: bodies of comparable pull on each other as from
 // the centre, 8,000 to 16,384 of them, 24 systems: median of the largest 1.5e-13
