@@ -25,11 +25,11 @@
 // sol_accel_sinks_device): what is computed keeps its order and so its bits.
 //
 // Bounded by the FP32 pipe: 71.5 operations a term are 7.6 ms at 65,536 bodies;
-// the kernel takes 10.6 (72 %), an evaluation 10.96 for 13.9 before, of 16,384
-// bodies 0.77 ms for 0.99, of 10,007 339 us for 455, of 2,049 65 for 99.  Its error against the
+// the kernel takes 10.5 (73 %), an evaluation 10.85 for 13.9 before, of 16,384
+// bodies 0.75 ms for 0.99, of 10,007 329 us for 455, of 2,049 64 for 99.  Its error against the
 // reference form is no larger: bodies of comparable pull on each other as from
-// the centre, 8,000 to 16,384 of them, 24 systems: median of the largest 1.5e-13
-// for 2.0e-13, rms 9.4e-15 for 1.0e-14.
+// the centre, 8,000 to 16,384 of them, 24 systems: median of the largest 1.6e-13
+// for 2.0e-13, rms 9.5e-15 for 1.0e-14.
 //
 // Pairs closer than the grid (ff_close_pair) leave their FP32 terms zero: the
 // sink takes the FP64 term at once, the source's side is marked and evaluated
@@ -71,9 +71,10 @@ struct SymShared {
   float jmh[BLOCK], jml[BLOCK];  // their nearest sink of I
   int jnn[BLOCK];
   int close;
-  // a thread's FP64 sums of its two sinks: totals, compensation, close pairs
-  // (here, not in registers: they change every 128 sources only)
-  double sums[3][6][sym_threads(BLOCK)];
+  // a thread's FP64 sums of its two sinks: totals (of a few float-float sums each,
+  // added plainly), close pairs (here, not in registers: they change every 128
+  // sources only)
+  double sums[2][6][sym_threads(BLOCK)];
 };
 
 // Nearest neighbour of one body: the smallest r^2 (hi, then lo), ties to the lower index.
@@ -176,7 +177,7 @@ __device__ __forceinline__ void sym_step(SymShared<BLOCK>& sm, const ForceCtx& f
       double f[3] = {0.0, 0.0, 0.0};
       if (S.i0 < ns && j < ns) ff_close_pair(fc, j, p[0], p[1], p[2], gh.x, gl.x, f[0], f[1], f[2], r2h.x, r2l.x);
       if (DI)
-        for (int k = 0; k < 3; ++k) sm.sums[2][k][threadIdx.x] += f[k];
+        for (int k = 0; k < 3; ++k) sm.sums[1][k][threadIdx.x] += f[k];
       gh.x = gl.x = mh.x = ml.x = ql.x = 0.0f;
       qh.x = 1.0f;
       sm.close = 1;
@@ -186,7 +187,7 @@ __device__ __forceinline__ void sym_step(SymShared<BLOCK>& sm, const ForceCtx& f
       double f[3] = {0.0, 0.0, 0.0};
       if (S.i1 < ns && j < ns) ff_close_pair(fc, j, p[0], p[1], p[2], gh.y, gl.y, f[0], f[1], f[2], r2h.y, r2l.y);
       if (DI)
-        for (int k = 0; k < 3; ++k) sm.sums[2][3 + k][threadIdx.x] += f[k];
+        for (int k = 0; k < 3; ++k) sm.sums[1][3 + k][threadIdx.x] += f[k];
       gh.y = gl.y = mh.y = ml.y = ql.y = 0.0f;
       qh.y = 1.0f;
       sm.close = 1;
@@ -346,7 +347,7 @@ __global__ void __launch_bounds__(sym_threads(BLOCK), sym_ctas(BLOCK))
   S.gl = make_float2(-T[(size_t)FGL * np + S.i0], -T[(size_t)FGL * np + S.i1]);
   const double G1 = fc.ind_sum[kIndGrid];
   const float thr = fmaxf((float)(G1 * G1), 7.888609052210118e-31f);  // as k_pairs_ff
-  for (int k = 0; k < 18; ++k) sm.sums[k / 6][k % 6][threadIdx.x] = 0.0;
+  for (int k = 0; k < 12; ++k) sm.sums[k / 6][k % 6][threadIdx.x] = 0.0;
   SymNear n0 = {bound[S.i0], 3.0e38f, -1}, n1 = {bound[S.i1], 3.0e38f, -1};
   for (int J = Jlo; J < Jhi; ++J) {
     const bool want_j = J != I && wanted(J);
@@ -386,16 +387,17 @@ __global__ void __launch_bounds__(sym_threads(BLOCK), sym_ctas(BLOCK))
         sym_part<false, true>(sm, fc, y, sub, lane, j0, ns, thr, S, A, n0, n1, B);
       if (want_j) {
 #pragma unroll
-        for (int k = 0; k < 3; ++k)
-          sm.js[k][q] += ((double)B.h[k].x + (double)B.l[k].x) + ((double)B.h[k].y + (double)B.l[k].y);
+        for (int k = 0; k < 3; ++k) {
+          float u, e;  // both lanes in FP32 first: a warp waits 64 cycles for an FP64 instruction
+          ff_two_sum(B.h[k].x, B.h[k].y, u, e);
+          sm.js[k][q] += (double)u + (double)(e + (B.l[k].x + B.l[k].y));
+        }
       }
       if (want_i && ((p & 3) == 3 || p == kParts - 1)) {  // the sinks' float-float sums of 128 sources into FP64
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-          double* t = &sm.sums[0][k][threadIdx.x];
-          double* c = &sm.sums[1][k][threadIdx.x];
-          two_sum(t[0], c[0], (double)A.h[k].x + (double)A.l[k].x);
-          two_sum(t[3 * kThreads], c[3 * kThreads], (double)A.h[k].y + (double)A.l[k].y);
+          sm.sums[0][k][threadIdx.x] += (double)A.h[k].x + (double)A.l[k].x;
+          sm.sums[0][3 + k][threadIdx.x] += (double)A.h[k].y + (double)A.l[k].y;
           A.h[k] = A.l[k] = make_float2(0.0f, 0.0f);
         }
       }
@@ -423,8 +425,7 @@ __global__ void __launch_bounds__(sym_threads(BLOCK), sym_ctas(BLOCK))
     double* out = part_i + (size_t)C * PART_SLOTS * np + (u ? S.i1 : S.i0);
 #pragma unroll
     for (int k = 0; k < 3; ++k)
-      out[(size_t)(PAX + k) * np] = (sm.sums[0][3 * u + k][threadIdx.x] + sm.sums[1][3 * u + k][threadIdx.x]) +
-                                    sm.sums[2][3 * u + k][threadIdx.x];
+      out[(size_t)(PAX + k) * np] = sm.sums[0][3 * u + k][threadIdx.x] + sm.sums[1][3 * u + k][threadIdx.x];
     out[(size_t)PR2 * np] = m.j >= 0 ? (double)m.h + (double)m.l : 1.0e300;
     out[(size_t)PIDX * np] = __longlong_as_double((long long)m.j);
   }
