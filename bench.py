@@ -688,14 +688,15 @@ def main():
     # pair runs on the FP32 pipe); SPLIT 12 (displacement 3, r^2 3, the Newton
     # residual 1, G m y^3 and its correction 2, the accumulation 3; the seed's
     # square and cube and the correction's t come from the integer pipe); the
-    # reference form 14 in the pair (correctly rounded sqrt and reciprocal by
-    # one FMA remainder each, the six term multiplies on the integer pipe) plus
-    # the 3 in-order additions
-    fp64_ops = {"split_ff": 0, "split": 12, "fp64": 17}
-    # SPLIT_FF's pair (k_pairs_ff) runs on the FP32 pipe: FP32 lane operations
-    # per pair of its float-float arithmetic (sol_pair.cuh): the displacement
-    # from the grid triples 21, r^2 23, G m r^-3 22, the accumulation 40.5
-    # (12 per component and step, a 3-operation renormalisation every second)
+    # reference form 9 in the pair (its multiplications and the remainders of
+    # the correctly rounded sqrt and reciprocal on the integer pipe) plus the 3
+    # in-order additions
+    fp64_ops = {"split_ff": 0, "split": 12, "fp64": 12}
+    # SPLIT_FF's pair (k_pairs_sym) runs on the FP32 pipe: FP32 lane operations
+    # of its float-float arithmetic (sol_pair.cuh), the unordered pair's shared
+    # ones -- the displacement from the grid triples 21, r^2 23, r^-3 15 -- and
+    # a term's: G m 4, the accumulation 37.5 (12 per component and step, a
+    # 3-operation renormalisation every second)
     fp32_ops = {"split_ff": FF_FP32_OPS_PER_PAIR}
     prof = profile_figures()
 

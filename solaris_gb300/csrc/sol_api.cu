@@ -11,7 +11,7 @@
 #include "sol_internal.cuh"
 
 int sol_force_tile();
-size_t sol_force_part_doubles(const sol_ctx* c);
+int sol_force_alloc_parts(sol_ctx* c);
 int sol_force_uses_chunk_partials(const sol_ctx* c, int precision);
 int sol_force_prepass_blocks(int npad);
 int sol_force_src_doubles();
@@ -411,7 +411,7 @@ int sol_set_precision(sol_ctx* c, int32_t p) {
   }
   if (p != SOL_PRECISION_FP64 && !c->barycentric && !c->d_part && sol_force_uses_chunk_partials(c, p)) {
     RET(set_device(c));
-    RET(dev_alloc(&c->d_part, (size_t)sol_force_part_doubles(c)));
+    RET(sol_force_alloc_parts(c));
   }
   if (c->precision != p) sol_adjoint_model_changed(c);
   c->precision = p;

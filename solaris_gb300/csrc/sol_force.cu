@@ -23,7 +23,6 @@
 #include "sol_pair.cuh"
 
 int sol_force_uses_chunk_partials(const sol_ctx* c, int precision);
-size_t sol_force_part_doubles(const sol_ctx* c);
 
 namespace {
 
@@ -1079,7 +1078,7 @@ struct FFPlan {
   int block = kTile, nb = 0, per = 1, chunks = 0;  // k_pairs_sym
   int from = 0;                                    // nb block
   int n1 = 0, chunk1 = kTile, n2 = 0, chunk2 = kTile;
-  size_t o_j = 0, o_i = 0, o_1 = 0, o_2 = 0, o_bound = 0, doubles = 0;
+  size_t o_j = 0, o_i = 0, o_1 = 0, o_2 = 0, o_bound = 0;
 };
 
 // Per sink: the partials in a fixed order, the nearest neighbour (the
@@ -1452,9 +1451,10 @@ static size_t sym_doubles(const FFPlan& p, int npad) {
   return ((size_t)p.nb * (p.nb - 1) / 2 * p.block + (size_t)p.chunks * npad) * PART_SLOTS + npad;
 }
 
-static FFPlan ff_plan(int device, int n, const Classes& cls, int npad) {
+// room: doubles of the partials' buffer (k_pairs_ff alone where the block pairs' do not fit)
+static FFPlan ff_plan(int device, int n, const Classes& cls, int npad, size_t room, bool blocks = true) {
   FFPlan p;
-  const int massive = sym_bodies(n, cls);
+  const int massive = blocks ? sym_bodies(n, cls) : 0;
   if (massive > 0) {
     const int block = sym_block(massive);
     sym_shape(p, block, (massive + block - 1) / block);
@@ -1483,7 +1483,7 @@ static FFPlan ff_plan(int device, int n, const Classes& cls, int npad) {
   p.o_1 = take((size_t)p.n1 * PART_SLOTS * npad);
   p.o_2 = take((size_t)p.n2 * PART_SLOTS * npad);
   p.o_bound = take(p.nb > 0 ? npad : 0);
-  p.doubles = o;
+  if (o > room && p.nb > 0) return ff_plan(device, n, cls, npad, room, false);
   return p;
 }
 
@@ -1585,7 +1585,7 @@ static int force_launch(sol_ctx* c, const ForceCtx& fc, const double* d_y, doubl
       return SOL_ERR_STATE;
     }
     if (ff2d) {
-      plan = ff_plan(c->device, c->n, c->cls, fc.npad);
+      plan = ff_plan(c->device, c->n, c->cls, fc.npad, c->part_doubles);
       if (plan.nb > 0) bound = reinterpret_cast<float*>(c->d_part + plan.o_bound);
     }
   }
@@ -1686,7 +1686,7 @@ int sol_force_src_doubles() { return kSrcDoubles; }
 // Partials for either split form's 2-D kernels, of this system and of every
 // smaller one it can become (removed bodies): fewer blocks can have more
 // chunks.
-size_t sol_force_part_doubles(const sol_ctx* c) {
+static size_t part_doubles(const sol_ctx* c, bool blocks) {
   const size_t np = c->npad;
   size_t most = (size_t)((c->n + kChunk - 1) / kChunk) * PART_SLOTS * np;  // SPLIT
   // k_pairs_ff alone: the number of chunks changes at whole sink blocks only
@@ -1695,6 +1695,7 @@ size_t sol_force_part_doubles(const sol_ctx* c) {
     const size_t d = (size_t)((n + ch - 1) / ch) * PART_SLOTS * np;
     if (d > most) most = d;
   }
+  if (!blocks) return most;
   size_t sym = 0;
   for (int m = 64; m <= c->cls.nm + 255 && m <= kSymMax + 255; m += 64)
     for (int block = 64; block <= 256; block *= 2)
@@ -1707,6 +1708,21 @@ size_t sol_force_part_doubles(const sol_ctx* c) {
   if (sym > 0 && c->cls.nm < c->n)  // k_pairs_ff on the rest, in chunks of one tile at the least
     sym += ((size_t)(kTile + c->cls.n_spl + kTile - 1) / kTile + (c->cls.nm + kTile - 1) / kTile) * PART_SLOTS * np;
   return sym > most ? sym : most;
+}
+// The partials' buffer (not cleared: what is read has been written): without
+// the block pairs' where they do not fit.
+int sol_force_alloc_parts(sol_ctx* c) {
+  for (bool blocks : {true, false}) {
+    const size_t doubles = part_doubles(c, blocks);
+    if (cudaMalloc((void**)&c->d_part, sizeof(double) * doubles) == cudaSuccess) {
+      c->part_doubles = doubles;
+      return SOL_OK;
+    }
+    c->d_part = nullptr;
+    cudaGetLastError();
+  }
+  sol_set_error("cudaMalloc of the split partials failed");
+  return SOL_ERR_NOMEM;
 }
 // whether the split forms of this system run the 2-D kernel (and need its
 // chunk partials); the same test as the dispatch in sol_force_launch_parts

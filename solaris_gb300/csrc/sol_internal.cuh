@@ -167,7 +167,8 @@ struct sol_ctx {
   char *d_slab, *h_slab;
   size_t slab_bytes, slab_from;
   double* d_partial;           // block partial maxima of the error norm
-  double* d_part;              // per-chunk partial sums of the split pair kernels
+  double* d_part;              // partial sums of the split pair kernels
+  size_t part_doubles;
   int n_partial;
   sol_ctrl* d_ctrl;
   sol_ctrl* h_ctrl;            // pinned mirror

@@ -3,14 +3,14 @@
     python tests/kernel_cases.py <case>
 
 Cases (each holds a few hundred MB of device memory at most):
-  fp64_few        k_gravity_ac_few: FP64 force, 2,048 self-gravitating bodies
-  fp64_wide       k_gravity_ac_wide: FP64 force, 16,384 self-gravitating bodies
-  fp64_wide_65536 k_gravity_ac_wide: FP64 force at the bench size, 65,536 bodies
+  fp64_few        k_gravity_ac_ref: FP64 force, 2,048 self-gravitating bodies
+  fp64_wide       k_gravity_ac_ref: FP64 force, 16,384 self-gravitating bodies
+  fp64_wide_65536 k_gravity_ac_ref: FP64 force at the bench size, 65,536 bodies
   split_65536     k_pairs<SPLIT> + k_combine: 65,536 bodies (bench size)
-  split_ff_65536  k_split_table + k_pairs_ff + k_combine: 65,536 bodies (bench size)
-  split_ff_warp   k_pairs_few<SPLIT_FF>: float-float force, one warp per sink,
-                  2,048 bodies (below the 4,096 where k_pairs_ff takes over)
-  split_ff_2d     k_pairs_ff + k_combine: float-float force, 32,768 bodies
+  split_ff_65536  k_split_table + k_near_bound + k_pairs_sym + k_combine: 65,536
+                  bodies (bench size)
+  split_ff_warp   k_pairs_sym in blocks of 64: float-float force, 2,048 bodies
+  split_ff_2d     k_pairs_sym + k_combine: float-float force, 32,768 bodies
   potential       k_potential_pairs: the integrals' potential energy, 65,536
                   bodies
   fp64_rate       k_fp64_rate<0,1,2>: the FP64 pipe throughput probe (DFMA,
@@ -20,8 +20,8 @@ Cases (each holds a few hundred MB of device memory at most):
   persistent      k_group_rkf78: 20 RKF78 driver calls of 1 star + 2 giants +
                   253 test particles in one cooperative launch
   ensemble        k_ensemble_rkf78: 2 driver calls of 512 small systems
-  adjoint         k_vjp: forward and backward of 20 fixed RKF78 steps,
-                  1 star + 8 planets + 1,024 planetesimals
+  adjoint         k_vjp_pairs + k_vjp_finish: forward and backward of 20 fixed
+                  RKF78 steps, 1 star + 8 planets + 1,024 planetesimals
   stages          k_stage / k_rkf78_final: the elementwise kernels of 2 RKF78
                   attempts over 1,048,576 bodies
 """
