@@ -422,10 +422,10 @@ __global__ void __launch_bounds__(kSinkBlock) k_gravity_ac(ForceCtx fc, const do
 }
 
 // ---- FP64 GravityAC for sinks with many sources -------------------------------
-// A CTA takes spc sinks.  Its PW producing warps compute the pair terms of a
+// A CTA takes spc sinks.  Its producing warps compute the pair terms of a
 // tile of kRefTile sources for all of them (the reference's arithmetic,
 // Acceleration.cpp:294-317; a warp takes one sink and half a tile at a time)
-// into one of two shared tiles, while its SW summing warps -- one lane per
+// into one of two shared tiles, while its summing warp -- one lane per
 // (sink, component) -- add the previous tile's terms in ascending source
 // order: the reference's sequential sums, bit for bit.
 //
@@ -450,14 +450,16 @@ __global__ void __launch_bounds__(kSinkBlock) k_gravity_ac(ForceCtx fc, const do
 // Measured (one evaluation, us; before: the two kernels this one replaces,
 // 4 sinks x 224 sources with 12 summing lanes, and 32 sinks alternating
 // between producing and summing): 300 bodies 37 -> 25 (prepass included), 1,033
-// 94 -> 64, 2,049 305 -> 155, 4,099 900 -> 509, 16,411 10,800 -> 7,050.
+// 94 -> 64, 2,049 305 -> 155, 4,099 900 -> 509, 16,411 10,800 -> 7,040, 65,536
+// 150,000 -> 106,400.
 constexpr int kRefTile = 64;      // sources per round
-constexpr int kRefPerWarp = 10;   // sinks per summing warp: 30 of its 32 lanes
-constexpr int kRefMaxSinks = 21;  // of the two-warp form: 63 of 64 lanes
+constexpr int kRefMaxSinks = 10;  // of a CTA: 30 of its summing warp's 32 lanes
+constexpr int kRefProducers = 7;  // its other warps
+constexpr int kRefRow = 33;       // doubles per row of terms (odd: conflict-free columns)
 constexpr int kMaxDevices = 64;
 
-constexpr size_t ref_smem(int sw, int spc) {
-  return sizeof(double) * (2 * 7 * kRefTile + 2 * (size_t)kRefTile * (32 * sw + 1)) +
+constexpr size_t ref_smem(int spc) {
+  return sizeof(double) * (2 * 7 * kRefTile + 2 * (size_t)kRefTile * kRefRow) +
          (sizeof(long long) + sizeof(int)) * (size_t)kRefTile * spc;
 }
 
@@ -476,23 +478,20 @@ __device__ __forceinline__ void ref_pair(double xij, double yij, double zij, boo
   }
 }
 
-// 24 warps per SM (80 registers): three CTAs of the one-warp form, one of the
-// other.  With 32 (64 registers, a few spilled): 1,033 bodies 66.3 us for 64.1,
-// 4,099 521 for 509, 16,411 7.02 ms for 7.05.
-template <int SW, int PW>
-__global__ void __launch_bounds__((SW + PW) * 32, 24 / (SW + PW))
+// Three CTAs an SM (80 registers).  With four (64 registers, a few spilled):
+// 1,033 bodies 66.3 us for 64.1, 4,099 521 for 509, 16,411 7.02 ms for 7.05.
+__global__ void __launch_bounds__((1 + kRefProducers) * 32, 3)
     k_gravity_ac_ref(ForceCtx fc, const double* __restrict__ y, double* __restrict__ dydt, TimeSpec ts, uint32_t flags,
                      int spc) {
   extern __shared__ __align__(16) double ref_dyn[];
   __shared__ double sink_pos[kRefMaxSinks][3];
   __shared__ int sink_ns[kRefMaxSinks];
-  __shared__ double acc[SW * 32];
+  __shared__ double acc[32];
   __shared__ double nn_d[kRefMaxSinks];
   __shared__ int nn_i[kRefMaxSinks];
-  constexpr int row = 32 * SW + 1;             // doubles per source row (odd: conflict-free columns)
   double* srct = ref_dyn;                      // [2][7][kRefTile] source tiles
-  double* terms = srct + 2 * 7 * kRefTile;     // [2][kRefTile][row]
-  long long* nn_r = reinterpret_cast<long long*>(terms + 2 * kRefTile * row);  // [2 spc][32] nearest so far
+  double* terms = srct + 2 * 7 * kRefTile;     // [2][kRefTile][kRefRow]
+  long long* nn_r = reinterpret_cast<long long*>(terms + 2 * kRefTile * kRefRow);  // [2 spc][32] nearest so far
   int* nn_j = reinterpret_cast<int*>(nn_r + kRefTile * spc);
   const Classes& c = fc.cls;
   const int n = sol_sink_hi(fc);  // sinks [sink_lo, n)
@@ -510,33 +509,33 @@ __global__ void __launch_bounds__((SW + PW) * 32, 24 / (SW + PW))
   }
   const double* src = fc.src;
   const int np = fc.npad;
-  constexpr int kLoads = (7 * kRefTile + PW * 32 - 1) / (PW * 32);
-  const int pt = (warp - SW) * 32 + lane;  // producing thread
-  if (warp >= SW)
-    for (int q = pt; q < 7 * kRefTile; q += PW * 32) srct[q] = src[(size_t)(q / kRefTile) * np + (q % kRefTile)];
+  constexpr int kLoads = (7 * kRefTile + kRefProducers * 32 - 1) / (kRefProducers * 32);
+  const int pt = (warp - 1) * 32 + lane;  // producing thread
+  if (warp >= 1)
+    for (int q = pt; q < 7 * kRefTile; q += kRefProducers * 32) srct[q] = src[(size_t)(q / kRefTile) * np + (q % kRefTile)];
   __syncthreads();
   int ns_cta = 0;
   for (int s = 0; s < spc; ++s) ns_cta = max(ns_cta, sink_ns[s]);
   const int rounds = (ns_cta + kRefTile - 1) / kRefTile;
   double a_sum = 0.0;
   // round r: the producers fill term tile r & 1 from source tile r & 1 and
-  // fetch the next sources; the summing warps add term tile (r - 1) & 1
+  // fetch the next sources; the summing warp adds term tile (r - 1) & 1
   for (int r = 0; r <= rounds; ++r) {
-    if (warp >= SW) {
+    if (warp >= 1) {
       if (r < rounds) {
         double pre[kLoads];
         const bool more = r + 1 < rounds;
 #pragma unroll
         for (int u = 0; u < kLoads; ++u) {
-          const int q = pt + u * PW * 32;
+          const int q = pt + u * kRefProducers * 32;
           pre[u] = (more && q < 7 * kRefTile)
                        ? src[(size_t)(q / kRefTile) * np + (r + 1) * kRefTile + (q % kRefTile)]
                        : 0.0;
         }
         const double* st = srct + (r & 1) * 7 * kRefTile;
-        double* out = terms + (size_t)(r & 1) * kRefTile * row;
+        double* out = terms + (size_t)(r & 1) * kRefTile * kRefRow;
 #pragma unroll 1
-        for (int item = warp - SW; item < 2 * spc; item += PW) {  // (sink, half of the tile)
+        for (int item = warp - 1; item < 2 * spc; item += kRefProducers) {  // (sink, half of the tile)
           const int s = item >> 1;
           const int p = (item & 1) * 32 + lane;
           const int j = r * kRefTile + p;
@@ -551,7 +550,7 @@ __global__ void __launch_bounds__((SW + PW) * 32, 24 / (SW + PW))
                         st[SPZ * kRefTile + p], tx, ty, tz);
           // a source the sink does not take adds +0, which changes no sum:
           // a sum that starts at +0 is never -0
-          double* o = out + (size_t)p * row + 3 * s;
+          double* o = out + (size_t)p * kRefRow + 3 * s;
           o[0] = tx;
           o[1] = ty;
           o[2] = tz;
@@ -565,24 +564,23 @@ __global__ void __launch_bounds__((SW + PW) * 32, 24 / (SW + PW))
         double* nx = srct + ((r + 1) & 1) * 7 * kRefTile;
 #pragma unroll
         for (int u = 0; u < kLoads; ++u) {
-          const int q = pt + u * PW * 32;
+          const int q = pt + u * kRefProducers * 32;
           if (q < 7 * kRefTile) nx[q] = pre[u];
         }
       }
     } else if (r > 0) {
-      const int L = warp * 32 + lane;  // 3 sink + component
-      if (L < 3 * spc) {
-        const double* col = terms + (size_t)((r - 1) & 1) * kRefTile * row + L;
+      if (lane < 3 * spc) {  // 3 sink + component
+        const double* col = terms + (size_t)((r - 1) & 1) * kRefTile * kRefRow + lane;
 #pragma unroll
-        for (int p = 0; p < kRefTile; ++p) a_sum += col[p * row];
+        for (int p = 0; p < kRefTile; ++p) a_sum += col[p * kRefRow];
       }
     }
     __syncthreads();
   }
-  if (warp < SW) acc[warp * 32 + lane] = a_sum;
+  if (warp == 0) acc[lane] = a_sum;
   // nearest neighbour of a sink: the smallest distance over its 64 columns,
   // ties to the lowest index (each column keeps its first minimum)
-  for (int s = warp; s < spc; s += SW + PW) {
+  for (int s = warp; s < spc; s += 1 + kRefProducers) {
     long long b = nn_r[(2 * s) * 32 + lane];
     int bj = nn_j[(2 * s) * 32 + lane];
     const long long b2 = nn_r[(2 * s + 1) * 32 + lane];
@@ -1503,29 +1501,26 @@ static int launch_sym(sol_ctx* c, const ForceCtx& fc, const double* d_y, const F
   return SOL_OK;
 }
 
-// Sinks per CTA and summing warps of k_gravity_ac_ref: the CTAs spread over
-// the SMs, so an SM's work is its CTAs (the busiest SM's, k) times what one
-// costs a source: spc sinks' pairs and the summing warps', which cost about
-// 1.9 sinks each (16 cycles of the FP64 pipe against ~9 a sink).  For each k
-// the fewest sinks that reach it; the cheapest of one summing warp (up to
-// kRefPerWarp sinks) and two.
-static void ref_shape(int nsink, int nsm, int& spc, int& sw) {
+// Sinks per CTA of k_gravity_ac_ref: the CTAs spread over the SMs, so an SM's
+// work is its CTAs (the busiest SM's, k) times what one costs a source: spc
+// sinks' pairs and the summing warp's, which cost about 1.9 sinks (16 cycles of
+// the FP64 pipe against ~9 a sink).  For each k the fewest sinks that reach it.
+// (21 sinks with two summing and 14 producing warps, one such CTA an SM at 80
+// registers: 10,007 bodies 3.28 ms for 2.79, 65,536 121 for 106; two at 64: 2.89
+// and 106.)
+static int ref_sinks(int nsink, int nsm) {
   double best = 1e300;
-  spc = 1;
-  sw = 1;
-  for (int w = 1; w <= 2; ++w) {
-    const int most = w == 1 ? kRefPerWarp : kRefMaxSinks;
-    const long k0 = ((long)nsink + (long)nsm * most - 1) / ((long)nsm * most);
-    for (long k = k0; k < k0 + 3; ++k) {
-      const int sp = (int)(((long)nsink + k * nsm - 1) / (k * nsm));
-      const double cost = (double)k * (sp + 1.9 * w);
-      if (cost < best) {
-        best = cost;
-        spc = sp;
-        sw = w;
-      }
+  int spc = 1;
+  const long k0 = ((long)nsink + (long)nsm * kRefMaxSinks - 1) / ((long)nsm * kRefMaxSinks);
+  for (long k = k0; k < k0 + 3; ++k) {
+    const int sp = (int)(((long)nsink + k * nsm - 1) / (k * nsm));
+    const double cost = (double)k * (sp + 1.9);
+    if (cost < best) {
+      best = cost;
+      spc = sp;
     }
   }
+  return spc;
 }
 
 // Whether k_gravity_ac_ref is the faster one for ns sources (k_gravity_ac: a
@@ -1544,7 +1539,7 @@ static bool ref_pays(int ns, int nsink) {
 
 static int launch_ref(sol_ctx* c, const ForceCtx& fc, const double* d_y, double* d_dydt, TimeSpec ts, uint32_t flags,
                       int nsink) {
-  // per device: the SM count, once the kernels' shared-memory sizes are
+  // per device: the SM count, once the kernel's shared-memory size is
   // allowed (contexts of several host threads may race to set it: the same
   // values, hence an atomic published after the attribute calls)
   static std::atomic<int> ref_sms[kMaxDevices];
@@ -1552,19 +1547,13 @@ static int launch_ref(sol_ctx* c, const ForceCtx& fc, const double* d_y, double*
   int nsm = ref_sms[dev].load(std::memory_order_acquire);
   if (nsm == 0) {
     SOL_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
-    SOL_CUDA(cudaFuncSetAttribute(k_gravity_ac_ref<1, 7>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)ref_smem(1, kRefPerWarp)));
-    SOL_CUDA(cudaFuncSetAttribute(k_gravity_ac_ref<2, 14>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)ref_smem(2, kRefMaxSinks)));
+    SOL_CUDA(cudaFuncSetAttribute(k_gravity_ac_ref, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)ref_smem(kRefMaxSinks)));
     ref_sms[dev].store(nsm, std::memory_order_release);
   }
-  int spc, sw;
-  ref_shape(nsink, nsm, spc, sw);
-  const int grid = (nsink + spc - 1) / spc;
-  if (sw == 1)
-    k_gravity_ac_ref<1, 7><<<grid, 8 * 32, ref_smem(1, spc), c->stream>>>(fc, d_y, d_dydt, ts, flags, spc);
-  else
-    k_gravity_ac_ref<2, 14><<<grid, 16 * 32, ref_smem(2, spc), c->stream>>>(fc, d_y, d_dydt, ts, flags, spc);
+  const int spc = ref_sinks(nsink, nsm);
+  k_gravity_ac_ref<<<(nsink + spc - 1) / spc, (1 + kRefProducers) * 32, ref_smem(spc), c->stream>>>(fc, d_y, d_dydt, ts,
+                                                                                                  flags, spc);
   SOL_LAUNCHED();
   return SOL_OK;
 }
