@@ -2,17 +2,22 @@
 // (Solaris/Acceleration.cpp:60-246) and its gravity, gas-drag and migration
 // terms.
 //
-// One evaluation is three launches:
+// One evaluation:
 //   k_prepass     one thread per body: rm3[j] = 1/|r_j|^3 exactly as
 //                 GravityAC computes it (:256-264), and the structure-of-arrays
 //                 source table {x, y, z, G m, x rm3, y rm3, z rm3} that the pair
 //                 kernel streams; per-block partial sums of the indirect term.
 //   k_ind_reduce  one block: the indirect-term totals (split forms; k_split_table
 //                 does it where it runs).
-//   k_gravity_*   one thread per sink body; source tiles of TJ bodies are
-//                 staged in shared memory by bulk copies (cp.async.bulk, the
-//                 TMA engine) completing on an mbarrier, double buffered.  The
-//                 epilogue adds gas drag and type-I/II migration for the sink.
+//   the pairs     FP64: k_gravity_ac_ref (tiles of 64 sources, the sums in
+//                 source order by a warp of their own) or k_gravity_ac (a thread
+//                 a sink, few sources); SPLIT_FF: k_split_table, then k_pairs_sym
+//                 (unordered pairs of massive bodies) and / or k_pairs_ff, or
+//                 k_pairs_few; SPLIT: k_pairs or k_pairs_few.  The 2-D kernels'
+//                 source tiles are staged in shared memory by bulk copies
+//                 (cp.async.bulk, the TMA engine) completing on an mbarrier,
+//                 double buffered; k_combine adds their partials.  The epilogue
+//                 adds gas drag and type-I/II migration for the sink.
 #include <cstdio>
 #include <cstring>
 #include <atomic>
