@@ -55,6 +55,41 @@ __device__ __forceinline__ double eval_time(const TimeSpec& ts) {
 // ---- prepass ----------------------------------------------------------------
 __device__ __forceinline__ float* ftab(const ForceCtx& fc) { return reinterpret_cast<float*>(fc.src + (size_t)SRC_ARRAYS * fc.npad); }
 
+// Body j's rm3 and its entries of the source table (zeros for padding bodies)
+struct SourceRow {
+  double gm, px, py, pz;
+};
+__device__ __forceinline__ SourceRow source_row(const ForceCtx& fc, int j, double x, double yy, double z) {
+  SourceRow r = {0.0, 0.0, 0.0, 0.0};
+  if (j < fc.cls.n) {
+    double rm3 = 0.0;
+    if (j >= 1) {
+      if (!fc.barycentric) {
+        // Acceleration.cpp:259-261
+        double r2 = x * x + yy * yy + z * z;
+        double d;
+        sol_ref_rinv3(r2, d, rm3);
+        fc.rm3[j] = rm3;
+      }
+      r.gm = SOL_GAUSS2 * fc.mass[j];
+    }
+    r.px = x * rm3;
+    r.py = yy * rm3;
+    r.pz = z * rm3;
+    if (fc.barycentric) r.gm = fc.mass[j];  // GravityBC uses m_j and scales by G at the end
+  }
+  double* s = fc.src;
+  const int np = fc.npad;
+  s[SX * np + j] = x;
+  s[SY * np + j] = yy;
+  s[SZ * np + j] = z;
+  s[SGM * np + j] = r.gm;
+  s[SPX * np + j] = r.px;
+  s[SPY * np + j] = r.py;
+  s[SPZ * np + j] = r.pz;
+  return r;
+}
+
 // prec: SOL_PRECISION_*.  The split forms also sum the indirect term; SPLIT_FF
 // (2-D kernel, ff = 1) also takes the largest |coordinate| and writes G m as
 // float (hi, lo) arrays of the float table.  clear: a status word to zero for
@@ -66,51 +101,28 @@ __global__ void k_prepass(ForceCtx fc, const double* __restrict__ y, int split, 
   double q[6] = {0, 0, 0, 0, 0, 0};  // indirect contributions: massive range, super-planetesimal range
   unsigned mbits = 0;                 // |coordinate| maximum as FP32 bits, rounded up
   if (j < fc.npad) {
-    double x = 0, yy = 0, z = 0, gm = 0, px = 0, py = 0, pz = 0;
+    double x = 0, yy = 0, z = 0;
     if (j < n) {
       x = y[6 * j + 0];
       yy = y[6 * j + 1];
       z = y[6 * j + 2];
-      double rm3 = 0.0;
-      if (j >= 1) {
-        if (!fc.barycentric) {
-          // Acceleration.cpp:259-261
-          double r2 = x * x + yy * yy + z * z;
-          double r;
-          sol_ref_rinv3(r2, r, rm3);
-          fc.rm3[j] = rm3;
-        }
-        gm = SOL_GAUSS2 * fc.mass[j];
-      }
-      px = x * rm3;
-      py = yy * rm3;
-      pz = z * rm3;
-      if (fc.barycentric) gm = fc.mass[j];  // GravityBC uses m_j and scales by G at the end
-      if (split && j >= 1) {
-        int slot = (j < fc.cls.nm) ? 0 : ((j < fc.cls.nm + fc.cls.n_spl) ? 3 : -1);
-        if (slot >= 0) {
-          q[slot + 0] = gm * px;
-          q[slot + 1] = gm * py;
-          q[slot + 2] = gm * pz;
-        }
+    }
+    const SourceRow r = source_row(fc, j, x, yy, z);
+    if (split && j < n && j >= 1) {
+      int slot = (j < fc.cls.nm) ? 0 : ((j < fc.cls.nm + fc.cls.n_spl) ? 3 : -1);
+      if (slot >= 0) {
+        q[slot + 0] = r.gm * r.px;
+        q[slot + 1] = r.gm * r.py;
+        q[slot + 2] = r.gm * r.pz;
       }
     }
-    double* s = fc.src;
-    const int np = fc.npad;
-    s[SX * np + j] = x;
-    s[SY * np + j] = yy;
-    s[SZ * np + j] = z;
-    s[SGM * np + j] = gm;
-    s[SPX * np + j] = px;
-    s[SPY * np + j] = py;
-    s[SPZ * np + j] = pz;
-    float gh = __double2float_rn(gm);
-    float gl = __double2float_rn(gm - (double)gh);
-    reinterpret_cast<float2*>(s + (size_t)SGF * np)[j] = make_float2(gh, gl);
+    float gh = __double2float_rn(r.gm);
+    float gl = __double2float_rn(r.gm - (double)gh);
+    reinterpret_cast<float2*>(fc.src + (size_t)SGF * fc.npad)[j] = make_float2(gh, gl);
     if (ff) {
       float* T = ftab(fc);
-      T[(size_t)FGH * np + j] = gh;
-      T[(size_t)FGL * np + j] = gl;
+      T[(size_t)FGH * fc.npad + j] = gh;
+      T[(size_t)FGL * fc.npad + j] = gl;
       const double m = fmax(fabs(x), fmax(fabs(yy), fabs(z)));
       mbits = __float_as_uint(__double2float_ru(m));
     }
@@ -154,6 +166,39 @@ __device__ __forceinline__ void ind_totals(const ForceCtx& fc) {
   if (threadIdx.x < 6) fc.ind_sum[threadIdx.x] = threadIdx.x < 3 ? tot[threadIdx.x] : tot[threadIdx.x - 3] + tot[threadIdx.x];
 }
 __global__ void __launch_bounds__(256) k_ind_reduce(ForceCtx fc) { ind_totals(fc); }
+
+// A stage's input y0 + h (a_0 f_0 + ...), summed left to right
+// (RungeKuttaFehlberg78.cpp:170-232, RungeKutta4.cpp:413-433), and what k_prepass
+// makes of it for the FP64 forms: a thread per element, then one per body.  Both
+// are a few dependent instructions, so a launch of its own was most of either
+// (a stage with its evaluation, in two launches and in one: 200 bodies 27.3 and
+// 23.8 us, 1,033 71.8 and 68.4, 4,000 509 and 505).
+constexpr int kStageBodies = 32;
+template <int K>
+__global__ void __launch_bounds__(6 * kStageBodies) k_stage_prepass(ForceCtx fc, const double* __restrict__ y0,
+                                                                    double* __restrict__ out, StageArgs s,
+                                                                    const sol_ctrl* ctrl) {
+  __shared__ double sv[6 * kStageBodies];
+  const double h = ctrl->h;
+  const int i = blockIdx.x * (6 * kStageBodies) + threadIdx.x;
+  double v = 0.0;
+  if (i < 6 * fc.cls.n) {
+    double f[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) f[k] = s.f[k][i];
+    double acc = s.a[0] * f[0];
+#pragma unroll
+    for (int k = 1; k < K; ++k) acc = acc + s.a[k] * f[k];
+    v = y0[i] + h * acc;
+    out[i] = v;
+  }
+  sv[threadIdx.x] = v;
+  __syncthreads();
+  if (threadIdx.x < kStageBodies) {
+    const int b = 6 * threadIdx.x;
+    source_row(fc, blockIdx.x * kStageBodies + threadIdx.x, sv[b], sv[b + 1], sv[b + 2]);
+  }
+}
 
 // Grid triples of every coordinate (f2_grid_disp): a = G1 rint(x / G1),
 // b = G2 rint((x - a) / G2), c = float(x - a - b); a and b are exact floats
@@ -1663,6 +1708,29 @@ int sol_force_launch_parts(sol_ctx* c, const double* d_y, double* d_dydt, TimeSp
 
 int sol_force_launch(sol_ctx* c, const double* d_y, double* d_dydt, TimeSpec ts, uint32_t flags) {
   return sol_force_launch_parts(c, d_y, d_dydt, ts, flags, 3);
+}
+
+// The FP64 forms, while a launch is a part of an evaluation (beyond, k_stage's grid
+// of whole warps of elements is as good).
+bool sol_force_takes_stage(const sol_ctx* c) {
+  return (c->precision == SOL_PRECISION_FP64 || c->barycentric) && c->n <= 16384;
+}
+int sol_force_launch_stage(sol_ctx* c, int k, const StageArgs& s, const double* y0, double* yt, double* d_dydt,
+                           TimeSpec ts, uint32_t flags) {
+  const int g = c->fc.npad / kStageBodies, b = 6 * kStageBodies;
+  switch (k) {
+    case 1: k_stage_prepass<1><<<g, b, 0, c->stream>>>(c->fc, y0, yt, s, c->d_ctrl); break;
+    case 2: k_stage_prepass<2><<<g, b, 0, c->stream>>>(c->fc, y0, yt, s, c->d_ctrl); break;
+    case 3: k_stage_prepass<3><<<g, b, 0, c->stream>>>(c->fc, y0, yt, s, c->d_ctrl); break;
+    case 4: k_stage_prepass<4><<<g, b, 0, c->stream>>>(c->fc, y0, yt, s, c->d_ctrl); break;
+    case 6: k_stage_prepass<6><<<g, b, 0, c->stream>>>(c->fc, y0, yt, s, c->d_ctrl); break;
+    case 7: k_stage_prepass<7><<<g, b, 0, c->stream>>>(c->fc, y0, yt, s, c->d_ctrl); break;
+    case 8: k_stage_prepass<8><<<g, b, 0, c->stream>>>(c->fc, y0, yt, s, c->d_ctrl); break;
+    case 9: k_stage_prepass<9><<<g, b, 0, c->stream>>>(c->fc, y0, yt, s, c->d_ctrl); break;
+    default: sol_set_error("stage with %d terms", k); return SOL_ERR_ARG;
+  }
+  SOL_LAUNCHED();
+  return sol_force_launch_parts(c, yt, d_dydt, ts, flags, 2);
 }
 
 // Sinks [lo, hi) only (heliocentric contexts): a rank's block of a

@@ -20,12 +20,6 @@
 namespace {
 
 constexpr int kBlock = 256;
-constexpr int kMaxTerms = 9;
-
-struct StageArgs {
-  const double* f[kMaxTerms];
-  double a[kMaxTerms];
-};
 
 inline int grid_for(int n) {
   int g = (n + kBlock - 1) / kBlock;
@@ -328,6 +322,14 @@ inline TimeSpec stage_time(sol_ctx* c, double coef) {
   return ts;
 }
 
+// A stage's input and its evaluation
+int stage_force(sol_ctx* c, int k, const StageArgs& s, const double* y0, double* yt, double* f, double coef,
+                uint32_t fl) {
+  if (sol_force_takes_stage(c)) return sol_force_launch_stage(c, k, s, y0, yt, f, stage_time(c, coef), fl);
+  RET(launch_stage(c, k, s, y0, yt));
+  return sol_force_launch(c, yt, f, stage_time(c, coef), fl);
+}
+
 // One RKF78 attempt (RungeKuttaFehlberg78::Step, :147-250): 12 stages, the
 // final sum, the error estimate and its norm.  The time of every stage is the
 // step's start time (:168, :173-234).
@@ -345,8 +347,7 @@ int rkf78_attempt(sol_ctx* c, const double* y0, double* y, double* err, uint32_t
       s.f[k] = fk[st[r].idx[k]];
       s.a[k] = st[r].a[k];
     }
-    RET(launch_stage(c, st[r].k, s, y0, c->d_ytmp));
-    RET(sol_force_launch(c, c->d_ytmp, fk[r], stage_time(c, 0.0), fl));
+    RET(stage_force(c, st[r].k, s, y0, c->d_ytmp, fk[r], 0.0, fl));
   }
   Rkf78FinalArgs fa;
   for (int k = 0; k < 13; ++k) fa.f[k] = fk[k];
@@ -411,16 +412,13 @@ int rk4_attempt(sol_ctx* c, const double* y0, double* y, uint32_t fl = SOL_EVAL_
   memset(&s, 0, sizeof(s));
   s.f[0] = c->d_accel;
   s.a[0] = a21;
-  RET(launch_stage(c, 1, s, y0, c->d_ytmp));
-  RET(sol_force_launch(c, c->d_ytmp, c->d_fk[1], stage_time(c, c2), fl));
+  RET(stage_force(c, 1, s, y0, c->d_ytmp, c->d_fk[1], c2, fl));
   s.f[0] = c->d_fk[1];
   s.a[0] = a32;
-  RET(launch_stage(c, 1, s, y0, c->d_ytmp));
-  RET(sol_force_launch(c, c->d_ytmp, c->d_fk[2], stage_time(c, c3), fl));
+  RET(stage_force(c, 1, s, y0, c->d_ytmp, c->d_fk[2], c3, fl));
   s.f[0] = c->d_fk[2];
   s.a[0] = a43;
-  RET(launch_stage(c, 1, s, y0, c->d_ytmp));
-  RET(sol_force_launch(c, c->d_ytmp, c->d_fk[3], stage_time(c, c4), fl));
+  RET(stage_force(c, 1, s, y0, c->d_ytmp, c->d_fk[3], c4, fl));
   StageArgs fs;
   memset(&fs, 0, sizeof(fs));
   fs.f[0] = c->d_accel;
@@ -840,8 +838,7 @@ int sol_rkf78_stages(sol_ctx* c, const double* d_y0, double* d_y, double* const*
     }
     if (r > 10) break;  // stages 11 and 12 enter only the error estimate
     double* out = (stage_out && stage_out[r]) ? stage_out[r] : c->d_ytmp;
-    RET(launch_stage(c, st[r].k, sa, d_y0, out));
-    RET(sol_force_launch(c, out, fk[r], stage_time(c, 0.0), SOL_EVAL_GAS_DRAG));
+    RET(stage_force(c, st[r].k, sa, d_y0, out, fk[r], 0.0, SOL_EVAL_GAS_DRAG));
   }
   Rkf78FinalArgs fa;
   for (int k = 0; k < 13; ++k) fa.f[k] = fk[k];

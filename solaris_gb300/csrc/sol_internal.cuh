@@ -192,6 +192,16 @@ struct sol_ctx {
 
 // ---- launch helpers (defined in sol_force.cu / sol_integrate.cu) --------------
 int sol_force_launch(sol_ctx* c, const double* d_y, double* d_dydt, TimeSpec ts, uint32_t flags);
+// A stage's terms: y0 + h (a_0 f_0 + a_1 f_1 + ...), and its evaluation with the
+// stage's input formed in the evaluation's first kernel (where that is taken).
+constexpr int kMaxTerms = 9;
+struct StageArgs {
+  const double* f[kMaxTerms];
+  double a[kMaxTerms];
+};
+bool sol_force_takes_stage(const sol_ctx* c);
+int sol_force_launch_stage(sol_ctx* c, int k, const StageArgs& s, const double* y0, double* yt, double* d_dydt,
+                           TimeSpec ts, uint32_t flags);
 int sol_force_launch_parts(sol_ctx* c, const double* d_y, double* d_dydt, TimeSpec ts, uint32_t flags, int parts,
                            int* d_clear = nullptr);
 int sol_integrator_run(sol_ctx* c, int integrator, int n_steps);
