@@ -1138,8 +1138,8 @@ struct FFPlan {
 // loaded at a time, a warp a component adds the warps' sums, and the first warp
 // finishes.  Block pairs' partials are few terms each and add up plainly (3 FP64
 // instructions a partial; their float-float sums carry 2^-46), the chunks of up
-// to 4,096 sources compensated (21).  10,007 bodies 18 us
-// (one thread a sink 65), 65,536 138 (213).
+// to 4,096 sources compensated (21).  10,007 bodies 18 us (one thread a sink 65),
+// 65,536 131 (213).
 constexpr int kCombineSinks = 32, kCombineWarps = 8, kCombineLoads = 4;
 
 __global__ void __launch_bounds__(kCombineSinks* kCombineWarps, 4)
@@ -1663,8 +1663,8 @@ static int force_launch(sol_ctx* c, const ForceCtx& fc, const double* d_y, doubl
     if (c->precision == SOL_PRECISION_SPLIT_FF) {
       if (plan.nb > 0) {
         const int tiles = (plan.from + kTile - 1) / kTile;
-        k_near_bound<<<dim3(tiles, (tiles < kBoundBlocks ? tiles : kBoundBlocks) * kBoundParts), kTile, 0, c->stream>>>(fc, bound,
-                                                                                                       tiles);
+        const dim3 grid_bound(tiles, (tiles < kBoundBlocks ? tiles : kBoundBlocks) * kBoundParts);
+        k_near_bound<<<grid_bound, kTile, 0, c->stream>>>(fc, bound, tiles);
         SOL_LAUNCHED();
         const int r = plan.block == 64    ? launch_sym<64>(c, fc, d_y, plan, bound)
                       : plan.block == 128 ? launch_sym<128>(c, fc, d_y, plan, bound)

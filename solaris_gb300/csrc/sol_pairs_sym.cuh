@@ -26,10 +26,10 @@
 //
 // Bounded by the FP32 pipe: 71.5 operations a term are 7.6 ms at 65,536 bodies;
 // the kernel takes 10.5 (73 %), an evaluation 10.85 for 13.9 before, of 16,384
-// bodies 0.75 ms for 0.99, of 10,007 329 us for 455, of 2,049 64 for 99.  Its error against the
-// reference form is no larger: bodies of comparable pull on each other as from
-// the centre, 8,000 to 16,384 of them, 24 systems: median of the largest 1.6e-13
-// for 2.0e-13, rms 9.5e-15 for 1.0e-14.
+// bodies 0.75 ms for 0.99, of 10,007 329 us for 455, of 2,049 64 for 99.  Its
+// error against the reference form is no larger: bodies of comparable pull on
+// each other as from the centre, 8,000 to 16,384 of them, 24 systems: median of
+// the largest 1.6e-13 for 2.0e-13, rms 9.5e-15 for 1.0e-14.
 //
 // Pairs closer than the grid (ff_close_pair) leave their FP32 terms zero: the
 // sink takes the FP64 term at once, the source's side is marked and evaluated

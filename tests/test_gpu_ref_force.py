@@ -1,9 +1,9 @@
 """k_gravity_ac_ref (the FP64 form of sinks with 224 sources or more) against
-the oracle, bit for bit: source counts around whole tiles of 64, systems of
-one summing warp per CTA and of two, sinks of different source ranges in one
-CTA (Acceleration.cpp:285-289), a planar system (every z displacement zero),
-and displacements whose x or y is exactly zero or far outside the integer
-multiply's range (the IEEE path)."""
+the oracle, bit for bit: source counts around whole tiles of 64, from two sinks a
+CTA to ten and many CTAs an SM, sinks of different source ranges in one CTA
+(Acceleration.cpp:285-289), a planar system (every z displacement zero), and
+displacements whose x or y is exactly zero or far outside the integer multiply's
+range (the IEEE path)."""
 import numpy as np
 import pytest
 
