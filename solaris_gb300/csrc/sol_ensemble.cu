@@ -448,17 +448,18 @@ int ens_run(sol_ensemble* e, int n_steps) {
 }
 }  // namespace
 
-// The launch shape until the caller sets one.  768 threads fill an SM
+// The launch shape until the caller sets one.  ~800 threads fill an SM
 // (registers), and a system's steps are a serial chain: with few systems an SM
 // the last ones decide, so each gets more threads; with many, small CTAs waste
-// the fewest lanes.  Measured (ms, four calls, FP64 / SPLIT_FF, against the 128
-// threads x 4 this rule replaces): 160 systems 8.15 / 5.08 -> 4.05 / 2.67; 512
-// 11.1 / 6.47 -> 6.49 / 3.86; 1,024 12.7 / 7.33 -> 9.63 / 5.96; 3,000 28.2 /
-// 17.4 -> 26.8 / 15.6.
+// the fewest lanes.  Measured (ms, four calls, FP64 / SPLIT_FF): 160 systems 3.61
+// / 2.27 with 640 threads (512: 3.66 / 2.58), 300 3.94 / 2.66 (4.72 / 2.85), 512
+// 5.77 / 3.67 with 384 x 2 (640: 6.29 / 4.33), 1,024 8.78 / 5.81 with 256 x 3
+// (384 x 2: 9.06 / 6.29), 2,000 15.4 / 10.3 with 192 x 4 (256 x 3: 15.6 / 10.7),
+// 3,000 26.8 / 15.6 with 128 x 6.
 static void default_shape(int n_systems, int n_sm, int& threads, int& per_sm) {
   const double s = (double)n_systems / n_sm;
-  threads = s <= 2 ? 512 : s <= 5 ? 384 : s <= 16 ? 256 : 128;
-  per_sm = s <= 5 ? 2 : s <= 16 ? 3 : 6;
+  threads = s <= 2 ? 640 : s <= 5 ? 384 : s <= 10 ? 256 : s <= 16 ? 192 : 128;
+  per_sm = s <= 2 ? 1 : s <= 5 ? 2 : s <= 10 ? 3 : s <= 16 ? 4 : 6;
 }
 
 extern "C" {

@@ -12,7 +12,7 @@ from solaris_gb300 import abi, engine, scenarios
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("count", [1, 5, 310, 800])
+@pytest.mark.parametrize("count", [1, 5, 310, 800, 1600])
 def test_default_shapes_and_out_of_range_components(count):
     base = [scenarios.config1(seed=60 + k, n_tp=k) for k in (0, 1, 29, 125, 253)]
     for s in base[2:]:  # planar and nearly planar bodies, and components that square to subnormals
