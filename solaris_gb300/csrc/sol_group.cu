@@ -430,7 +430,7 @@ __device__ __forceinline__ void work_by_component(const GroupArgs& P, const View
   for (;;) {
     __syncthreads();
     if (S.leave) return;
-    const int o = S.cur * V.stride;
+    const int o = S.cur * V.stride, last = S.last;  // (all of Ctl's between the two barriers: submit() writes the next)
     const double x = bj[o] - bi[o];
     const double sq = x * x;
     const double qx = __shfl_sync(0xFFFFFFFFu, sq, 0, 4), qy = __shfl_sync(0xFFFFFFFFu, sq, 1, 4),
@@ -450,7 +450,7 @@ __device__ __forceinline__ void work_by_component(const GroupArgs& P, const View
     const double t = second_pass(body, x, rijm3, pp, *xj, gm);
     if (live && c < 3) p[0] = t;
     __syncthreads();
-    if (S.last) last_evaluation(P, V, const_cast<int*>(&S.event), w * 32 + lane, nwork * 32);
+    if (last) last_evaluation(P, V, const_cast<int*>(&S.event), w * 32 + lane, nwork * 32);
   }
 }
 
@@ -473,6 +473,7 @@ __device__ __noinline__ void work(const GroupArgs& P, const View& V, const Ctl& 
     if (S.leave) return;
     const double* yt = V.yt + S.cur * V.stride;
     const uint32_t flags = S.flags;
+    const int last = S.last;  // (as above)
     const bool drag = ndrag > 0 && (flags & SOL_EVAL_GAS_DRAG);
     const bool mig = nmig > 0 && (flags & (SOL_EVAL_TYPE_I | SOL_EVAL_TYPE_II));
     const int u_drag = drag ? kRoles * w_role : 0;
@@ -518,14 +519,14 @@ __device__ __noinline__ void work(const GroupArgs& P, const View& V, const Ctl& 
         drag_finish(fc.gas, S.factor, S.m0pt, yt + 6 * sd, fc.radius[i], fc.density[i], fc.cd[i], fc.gamma_stokes[i],
                     fc.gamma_epstein[i], V.dv + d, V.cap, out);
         for (int k = 0; k < 3; ++k) V.gbuf[3 * sd + k] = out[k];
-        if (S.last && (sd >= P.ns || home)) {  // the buffers hold the last evaluation's drag
+        if (last && (sd >= P.ns || home)) {  // the buffers hold the last evaluation's drag
           double* gb = global_gas_buf(fc, i, 1);
           for (int k = 0; k < 3; ++k) gb[k] = out[k];
         }
       }
     }
     __syncthreads();
-    if (S.last) last_evaluation(P, V, const_cast<int*>(&S.event), w * 32 + lane, nwork * 32);
+    if (last) last_evaluation(P, V, const_cast<int*>(&S.event), w * 32 + lane, nwork * 32);
   }
 }
 

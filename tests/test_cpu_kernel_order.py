@@ -1,0 +1,36 @@
+"""Order of shared-memory accesses between warps, checked in the kernels' source.
+
+A missing order is a race that timing hides nearly always and that must not be
+provoked on a GPU, so these tests read the source."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "solaris_gb300", "csrc")
+
+
+def _body(name, function):
+    """The text between the braces of a function's definition, without comments."""
+    src = open(os.path.join(CSRC, name)).read()
+    src = re.sub(r"//[^\n]*", "", src)
+    at = src.index("{", re.search(r"\b%s\([^;{]*\)\s*(?=\{)" % function, src).start())
+    depth = 0
+    for end in range(at, len(src)):
+        depth += {"{": 1, "}": -1}.get(src[end], 0)
+        if depth == 0:
+            return src[at + 1:end]
+    raise AssertionError(function)
+
+
+def test_group_workers_read_the_evaluation_between_its_two_barriers():
+    """The state warps write the next evaluation's fields of Ctl (submit) after
+    the block barrier that ends the present one: a worker reads them between the
+    two barriers of its own evaluation only."""
+    written = re.findall(r"S\.(\w+) =", _body("sol_group.cu", r"submit = \[&\]"))
+    assert sorted(written) == ["cur", "factor", "flags", "last"]
+    for function in ("work_by_component", "work"):
+        body = _body("sol_group.cu", function)
+        loop = body[body.index("for (;;) {"):]
+        barriers = [m.end() for m in re.finditer(r"__syncthreads\(\);", loop)]
+        assert len(barriers) == 2
+        late = set(re.findall(r"\bS\.(\w+)", loop[barriers[1]:])) & set(written)
+        assert not late, f"{function} reads {late} after the evaluation's last barrier"
