@@ -218,6 +218,7 @@ __device__ __forceinline__ void sym_part(SymShared<BLOCK>& sm, const ForceCtx& f
 #pragma unroll 1
   for (int t = 0; t < 32; t += 2) {
     sym_step<DI, DJ, false>(sm, fc, y, sub * 32 + ((lane + t) & 31), from, j0, ns, thr, S, A, n0, n1, B);
+    __syncwarp();  // the next lane's source, whose nearest sink this one may just have written
     sym_step<DI, DJ, true>(sm, fc, y, sub * 32 + ((lane + t + 1) & 31), from, j0, ns, thr, S, A, n0, n1, B);
     __syncwarp();
   }

@@ -34,3 +34,13 @@ def test_group_workers_read_the_evaluation_between_its_two_barriers():
         assert len(barriers) == 2
         late = set(re.findall(r"\bS\.(\w+)", loop[barriers[1]:])) & set(written)
         assert not late, f"{function} reads {late} after the evaluation's last barrier"
+
+
+def test_source_minima_are_ordered_between_two_steps_of_a_warp():
+    """Two lanes of a warp take the same source in consecutive steps and both
+    update its nearest sink in shared memory; votes and shuffles order no memory,
+    so every step is followed by __syncwarp."""
+    body = _body("sol_pairs_sym.cuh", "sym_part")
+    steps = re.findall(r"sym_step<[^;]*;\s*(\w+)", body)
+    assert len(steps) == 2
+    assert steps == ["__syncwarp"] * 2
