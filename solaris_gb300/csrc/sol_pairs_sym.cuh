@@ -89,6 +89,12 @@ __device__ __forceinline__ void sym_near(SymNear& m, float h, float l, bool ok, 
   m.j = better ? j : m.j;
 }
 
+// r^2 below which a pair is close (ff_close_pair), as in k_pairs_ff: |d| < max(G1, 2^-50)
+__device__ __forceinline__ float sym_close_r2(const ForceCtx& fc) {
+  const double G1 = fc.ind_sum[kIndGrid];
+  return fmaxf((float)(G1 * G1), 7.888609052210118e-31f);
+}
+
 struct SymSinks {  // the thread's two sinks
   float2 a[3], b[3], c[3];  // grid triples
   float2 gh, gl;            // -G m
@@ -258,9 +264,11 @@ __device__ __noinline__ void sym_close_pass(SymShared<BLOCK>& sm, const ForceCtx
 
 // An upper bound of every body's squared distance to its nearest neighbour:
 // the smallest among the sources of its own block and the next ones
-// (kBoundBlocks in all), in FP32 from the grid triples' two leading parts
-// (relative error ~2^-22, covered by the factor).  A sink starts its search
-// there, so that a new minimum is rare (without it every block pair begins
+// (kBoundBlocks in all), in FP32 from the grid triples' two leading parts.  What
+// they leave out, up to 2^-24 G1 a component, is ~2^-23 of a distance of G1 or
+// more, which the factor covers, but of any size for a closer pair: such a
+// pair's r^2 is below sym_close_r2, and the bound is not.  A sink starts its
+// search there, so that a new minimum is rare (without it every block pair begins
 // with ~5 updates a body, and hardly a step of a warp has none).
 constexpr int kBoundBlocks = 4;
 constexpr int kBoundParts = 4, kBoundSources = kTile / kBoundParts;  // a block in quarters: a shorter chain
@@ -290,7 +298,8 @@ __global__ void __launch_bounds__(kTile) k_near_bound(ForceCtx fc, float* __rest
     m = (j0 + q != i && r2 < m) ? r2 : m;
   }
   // k_split_table set 3e38; the order of floats that are not negative is that of their bits
-  atomicMin(reinterpret_cast<int*>(bound) + i, __float_as_int(fminf(m * 1.0001f + 1.0e-37f, 3.0e38f)));
+  m = fmaxf(m, sym_close_r2(fc));
+  atomicMin(reinterpret_cast<int*>(bound) + i, __float_as_int(fminf(m * 1.0001f, 3.0e38f)));
 }
 
 // part_i: [chunk][PART_SLOTS][npad] as k_pairs_ff's; part_j: per block pair
@@ -346,8 +355,7 @@ __global__ void __launch_bounds__(sym_threads(BLOCK), sym_ctas(BLOCK))
   }
   S.gh = make_float2(-T[(size_t)FGH * np + S.i0], -T[(size_t)FGH * np + S.i1]);
   S.gl = make_float2(-T[(size_t)FGL * np + S.i0], -T[(size_t)FGL * np + S.i1]);
-  const double G1 = fc.ind_sum[kIndGrid];
-  const float thr = fmaxf((float)(G1 * G1), 7.888609052210118e-31f);  // as k_pairs_ff
+  const float thr = sym_close_r2(fc);
   for (int k = 0; k < 12; ++k) sm.sums[k / 6][k % 6][threadIdx.x] = 0.0;
   SymNear n0 = {bound[S.i0], 3.0e38f, -1}, n1 = {bound[S.i1], 3.0e38f, -1};
   for (int J = Jlo; J < Jhi; ++J) {
