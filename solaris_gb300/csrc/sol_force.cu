@@ -330,6 +330,15 @@ __device__ __forceinline__ void two_sum(double& s, double& c, double a) {
   c += err;
 }
 
+// two_sum's result, bit for bit, with three FP64 instructions less: the larger of s
+// and a by exponent (compared and selected on the integer pipe), then FastTwoSum.
+__device__ __forceinline__ void add_ordered(double& s, double& c, double a) {
+  const bool a_less = (__double2hiint(a) & 0x7FF00000) <= (__double2hiint(s) & 0x7FF00000);
+  const double big = a_less ? s : a, small = a_less ? a : s;
+  s = big + small;
+  c += small - (s - big);
+}
+
 // spin: the limit of every mbarrier wait; withhold >= 0: that tile is never
 // copied, so its wait runs out (failure-path tests only; -1 in production).
 template <int PREC>
@@ -1134,13 +1143,105 @@ struct FFPlan {
 // distanceOfNN recomputed in the reference's FP64 arithmetic for the chosen
 // neighbour, the Kepler and indirect terms, and the gas terms.
 // Bounded by the latency of the partials' loads (a few tens to some hundreds a
-// sink, far apart) and by FP64: a CTA's warps share its sinks' partials, four
-// loaded at a time, a warp a component adds the warps' sums, and the first warp
-// finishes.  Block pairs' partials are few terms each and add up plainly (3 FP64
-// instructions a partial; their float-float sums carry 2^-46), the chunks of up
-// to 4,096 sources compensated (21).  10,007 bodies 18 us (one thread a sink 65),
-// 65,536 131 (213).
+// sink, far apart): a CTA's warps share its sinks' partials, four loaded at a
+// time, a warp a component adds the warps' sums, and the first warp finishes.
+// The sums are 128-bit integers (FixSum), ~75 integer instructions a partial, as
+// accurate as compensated ones: those take 12 FP64 instructions a partial (21
+// with two_sum) of 16 cycles each.  An evaluation of 10,007 bodies 338 us for
+// 372, of 65,536 11.10 ms for 11.29; the kernel 30 and 131 us for 63 and 332
+// (27 and 131 with plain FP64 sums; one thread a sink 65 and 213).
 constexpr int kCombineSinks = 32, kCombineWarps = 8, kCombineLoads = 4;
+
+// A sum of doubles as a 128-bit integer A 2^(base - 1075), on the integer pipe.
+// A value of exponent field e is shifted left by e - base, 0 to 63 places; a
+// larger one raises the base so that it lies kFixPlace places up (fix_add_slow),
+// what lies below the last place is cut off: 2^-106 of the largest value, as a
+// compensated sum's second word.  2^11 values of the window's end fit.
+struct FixSum {
+  unsigned long long lo;
+  long long hi;
+  int base;
+};
+constexpr int kFixPlace = 54, kFixEmpty = -(1 << 20), kFixNan = 1 << 20;
+
+__device__ __forceinline__ void fix_add_shifted(FixSum& a, long long m, int sh) {
+  const unsigned r = sh & 31;
+  const unsigned w0 = (unsigned)m, w1 = (unsigned)(m >> 32), w2 = (unsigned)((int)w1 >> 31);
+  const unsigned s0 = w0 << r, s1 = __funnelshift_l(w0, w1, r), s2 = __funnelshift_l(w1, w2, r);
+  const bool word = sh >= 32;
+  const unsigned long long lo = word ? (unsigned long long)s0 << 32 : ((unsigned long long)s1 << 32 | s0);
+  const unsigned long long hi = word ? ((unsigned long long)s2 << 32 | s1) : ((unsigned long long)w2 << 32 | s2);
+  const unsigned long long t = a.lo + lo;
+  a.hi += (long long)(hi + (t < lo ? 1u : 0u));
+  a.lo = t;
+}
+static __device__ __noinline__ FixSum fix_add_slow(FixSum a, double v) {
+  const long long b = __double_as_longlong(v);
+  const int ef = (int)(b >> 52) & 0x7FF;
+  if (ef == 0x7FF || a.base == kFixNan) {  // as a compensated sum of an infinity gives
+    a.base = kFixNan;
+    return a;
+  }
+  long long m = (b & 0xFFFFFFFFFFFFFll) | (ef ? 1ll << 52 : 0ll);
+  if (b < 0) m = -m;
+  const int e = max(ef, 1);
+  int sh = e - a.base;
+  if (sh > 63) {
+    const int up = min(sh - kFixPlace, 127);
+    if (up >= 64) {
+      a.lo = (unsigned long long)(a.hi >> (up - 64));
+      a.hi >>= 63;
+    } else {
+      a.lo = (a.lo >> up) | ((unsigned long long)a.hi << (64 - up));
+      a.hi >>= up;
+    }
+    a.base = e - kFixPlace;
+    sh = kFixPlace;
+  }
+  if (sh < 0) {
+    m >>= min(-sh, 63);
+    sh = 0;
+  }
+  fix_add_shifted(a, m, sh);
+  return a;
+}
+__device__ __forceinline__ void fix_add(FixSum& a, double v) {
+  const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v);
+  const int ef = (int)(h >> 20) & 0x7FF;
+  const int sh = ef - a.base;
+  if ((unsigned)sh > 63u || ef == 0) {
+    if ((h << 1 | l) != 0u) a = fix_add_slow(a, v);
+    return;
+  }
+  const unsigned sg = (unsigned)((int)h >> 31);
+  const unsigned long long m = ((unsigned long long)((h & 0xFFFFFu) | 0x100000u) << 32) | l;
+  const unsigned long long sx = (unsigned long long)sg << 32 | sg;
+  fix_add_shifted(a, (long long)((m ^ sx) - sx), sh);
+}
+// The sum as a double and the rest
+static __device__ __noinline__ double2 fix_value(FixSum a) {
+  if (a.base == kFixNan) return make_double2(__longlong_as_double(0x7FF8000000000000LL), 0.0);
+  const bool neg = a.hi < 0;
+  unsigned long long hi = (unsigned long long)a.hi, lo = a.lo;
+  if (neg) {
+    lo = ~lo + 1;
+    hi = ~hi + (lo == 0 ? 1 : 0);
+  }
+  if ((hi | lo) == 0) return make_double2(0.0, 0.0);
+  int z = hi ? __clzll((long long)hi) : 64 + __clzll((long long)lo);
+  const int ex = 127 - z - 52 + a.base - 1075;  // of the leading 53 bits' last
+  if (z >= 64) {
+    hi = lo;
+    lo = 0;
+    z -= 64;
+  }
+  if (z) {
+    hi = hi << z | lo >> (64 - z);
+    lo <<= z;
+  }
+  const double top = ldexp((double)(hi >> 11), ex), rest = ldexp((double)((hi & 0x7FF) << 42 | lo >> 22), ex - 53);
+  return make_double2(neg ? -top : top, neg ? -rest : rest);
+}
 
 __global__ void __launch_bounds__(kCombineSinks* kCombineWarps, 4)
     k_combine(ForceCtx fc, const double* __restrict__ y, double* __restrict__ dydt, const double* __restrict__ part,
@@ -1155,7 +1256,7 @@ __global__ void __launch_bounds__(kCombineSinks* kCombineWarps, 4)
   const int np = fc.npad;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int i = fc.sink_lo + blockIdx.x * kCombineSinks + lane;
-  double s[3] = {0.0, 0.0, 0.0}, e[3] = {0.0, 0.0, 0.0};
+  FixSum s[3] = {{0, 0, kFixEmpty}, {0, 0, kFixEmpty}, {0, 0, kFixEmpty}};
   long long best = __double_as_longlong(1.0e300);  // r^2 >= 0: the order of doubles is that of their bits
   int nn = -1;
   auto near = [&](long long r2, int j) {
@@ -1165,8 +1266,8 @@ __global__ void __launch_bounds__(kCombineSinks* kCombineWarps, 4)
     }
   };
   // partials [0, count), at(k) the first word of partial k and `stride` its
-  // words' distance; of_blocks: of block pairs
-  auto add = [&](int count, size_t stride, bool of_blocks, auto at) {
+  // words' distance
+  auto add = [&](int count, size_t stride, auto at) {
     for (int g = kCombineLoads * warp; g < count; g += kCombineLoads * kCombineWarps) {
       double v[kCombineLoads][PART_SLOTS];
 #pragma unroll
@@ -1179,12 +1280,7 @@ __global__ void __launch_bounds__(kCombineSinks* kCombineWarps, 4)
       for (int u = 0; u < kCombineLoads; ++u) {
         if (g + u >= count) break;
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          if (of_blocks)
-            s[k] += v[u][PAX + k];
-          else
-            two_sum(s[k], e[k], v[u][PAX + k]);
-        }
+        for (int k = 0; k < 3; ++k) fix_add(s[k], v[u][PAX + k]);
         near(__double_as_longlong(v[u][PR2]), (int)__double_as_longlong(v[u][PIDX]));
       }
     }
@@ -1193,19 +1289,20 @@ __global__ void __launch_bounds__(kCombineSinks* kCombineWarps, 4)
     const int B = i / pl.block;
     if (B < pl.nb) {
       const double* pj = part + pl.o_j + (i - B * pl.block);  // as a source of the blocks below
-      add(B, pl.block, true, [&](int I) { return pj + sym_pair_index(I, B, pl.nb) * PART_SLOTS * pl.block; });
+      add(B, pl.block, [&](int I) { return pj + sym_pair_index(I, B, pl.nb) * PART_SLOTS * pl.block; });
       const int first = B / pl.per;  // as a sink of its own block's chunks
       const double* pi = part + pl.o_i + (size_t)first * PART_SLOTS * np + i;
-      add(pl.chunks - first, np, true, [&](int k) { return pi + (size_t)k * PART_SLOTS * np; });
+      add(pl.chunks - first, np, [&](int k) { return pi + (size_t)k * PART_SLOTS * np; });
     } else {
-      add(pl.n2, np, false, [&](int k) { return part + pl.o_2 + (size_t)k * PART_SLOTS * np + i; });
+      add(pl.n2, np, [&](int k) { return part + pl.o_2 + (size_t)k * PART_SLOTS * np + i; });
     }
-    add(pl.n1, np, false, [&](int k) { return part + pl.o_1 + (size_t)k * PART_SLOTS * np + i; });
+    add(pl.n1, np, [&](int k) { return part + pl.o_1 + (size_t)k * PART_SLOTS * np + i; });
   }
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    sh_s[warp][k][lane] = s[k];
-    sh_s[warp][3 + k][lane] = e[k];
+    const double2 d = fix_value(s[k]);
+    sh_s[warp][k][lane] = d.x;
+    sh_s[warp][3 + k][lane] = d.y;
   }
   sh_r2[warp][lane] = best;
   sh_nn[warp][lane] = nn;
@@ -1214,7 +1311,7 @@ __global__ void __launch_bounds__(kCombineSinks* kCombineWarps, 4)
     double t = sh_s[0][warp][lane], l = sh_s[0][3 + warp][lane];
 #pragma unroll
     for (int w = 1; w < kCombineWarps; ++w) {
-      two_sum(t, l, sh_s[w][warp][lane]);
+      add_ordered(t, l, sh_s[w][warp][lane]);
       l += sh_s[w][3 + warp][lane];
     }
     sh_tot[warp][lane] = t + l;

@@ -25,11 +25,14 @@
 // sol_accel_sinks_device): what is computed keeps its order and so its bits.
 //
 // Bounded by the FP32 pipe: 71.5 operations a term are 7.6 ms at 65,536 bodies;
-// the kernel takes 10.5 (73 %), an evaluation 10.85 for 13.9 before, of 16,384
-// bodies 0.75 ms for 0.99, of 10,007 329 us for 455, of 2,049 64 for 99.  Its
-// error against the reference form is no larger: bodies of comparable pull on
-// each other as from the centre, 8,000 to 16,384 of them, 24 systems: median of
-// the largest 1.6e-13 for 2.0e-13, rms 9.5e-15 for 1.0e-14.
+// the kernel takes 10.8 (70 %), an evaluation 11.06 for 13.9 before, of 16,384
+// bodies 0.77 ms for 0.99, of 10,007 335 us for 455, of 2,049 66 for 99.  Its
+// error is no larger: bodies of comparable pull on each other as from the centre,
+// 24 systems of 8,000 to 16,384, median of the largest against the reference form
+// 1.5e-13 for 2.0e-13; rms against long double (2,049 to 50,000 bodies) 9.2e-15
+// for 9.7e-15.  The FP64 sums are compensated as k_pairs_ff's are; without that
+// (and the two lanes' low words added in FP32) an evaluation takes 10.87 ms and
+// 331 us, and what a later sum cancels down to is lost.
 //
 // Pairs closer than the grid (ff_close_pair) leave their FP32 terms zero: the
 // sink takes the FP64 term at once, the source's side is marked and evaluated
@@ -67,13 +70,15 @@ __device__ __forceinline__ SymSource sym_load(const SymTile<BLOCK>& T, int q) {
 template <int BLOCK>
 struct SymShared {
   SymTile<BLOCK> tile;
-  double js[3][BLOCK];  // sums of the sources of J
+  // FP64 sums of the sources of J: totals and, where more than one warp adds to
+  // one, compensation
+  double js[BLOCK > 64 ? 2 : 1][3][BLOCK];
   float jmh[BLOCK], jml[BLOCK];  // their nearest sink of I
   int jnn[BLOCK];
   int close;
-  // a thread's FP64 sums of its two sinks: totals (of a few float-float sums each,
-  // added plainly), close pairs (here, not in registers: they change every 128
-  // sources only)
+  // a thread's FP64 sums of its two sinks (here, not in registers: they change
+  // every 128 sources only): totals and compensation; with blocks below 256, whose
+  // CTAs have one block of sources and one total of it, that total and the close pairs
   double sums[2][6][sym_threads(BLOCK)];
 };
 
@@ -93,6 +98,45 @@ __device__ __forceinline__ void sym_near(SymNear& m, float h, float l, bool ok, 
 __device__ __forceinline__ float sym_close_r2(const ForceCtx& fc) {
   const double G1 = fc.ind_sum[kIndGrid];
   return fmaxf((float)(G1 * G1), 7.888609052210118e-31f);
+}
+
+// The sum of two float-float numbers of one source (its two lanes'), to 2^-70 and
+// better, before its one rounding: the FP32 parts added exactly, so that two of
+// seven FP64 instructions (a conversion is one) go.
+__device__ __forceinline__ double sym_lanes(float2 h, float2 l) {
+  float u, e, v, w, f, g;
+  ff_two_sum(h.x, h.y, u, e);
+  ff_two_sum(l.x, l.y, v, w);
+  ff_two_sum(e, v, f, g);
+  return (double)u + ((double)f + (double)(g + w));
+}
+
+// v into component k of source q's sums; first: the first value of a block pair.
+// (With blocks of 64 bodies there is one, its only warp's, and the close pairs'.)
+template <int BLOCK>
+__device__ __forceinline__ void sym_add_source(SymShared<BLOCK>& sm, int k, int q, double v, bool first) {
+  if (BLOCK == 64 || first) {
+    sm.js[0][k][q] = v;
+    if constexpr (BLOCK > 64) sm.js[1][k][q] = 0.0;
+  } else if constexpr (BLOCK > 64) {
+    add_ordered(sm.js[0][k][q], sm.js[1][k][q], v);
+  }
+}
+
+// Component k's total of up to 128 sources, and a close pair, into the thread's sums
+template <int BLOCK>
+__device__ __forceinline__ void sym_add_sink(SymShared<BLOCK>& sm, int k, double v) {
+  if constexpr (BLOCK > 128)
+    add_ordered(sm.sums[0][k][threadIdx.x], sm.sums[1][k][threadIdx.x], v);
+  else
+    sm.sums[0][k][threadIdx.x] = v;
+}
+template <int BLOCK>
+__device__ __forceinline__ void sym_add_close(SymShared<BLOCK>& sm, int k, double v) {
+  if constexpr (BLOCK > 128)
+    add_ordered(sm.sums[0][k][threadIdx.x], sm.sums[1][k][threadIdx.x], v);
+  else
+    sm.sums[1][k][threadIdx.x] += v;
 }
 
 struct SymSinks {  // the thread's two sinks
@@ -183,7 +227,7 @@ __device__ __forceinline__ void sym_step(SymShared<BLOCK>& sm, const ForceCtx& f
       double f[3] = {0.0, 0.0, 0.0};
       if (S.i0 < ns && j < ns) ff_close_pair(fc, j, p[0], p[1], p[2], gh.x, gl.x, f[0], f[1], f[2], r2h.x, r2l.x);
       if (DI)
-        for (int k = 0; k < 3; ++k) sm.sums[1][k][threadIdx.x] += f[k];
+        for (int k = 0; k < 3; ++k) sym_add_close(sm, k, f[k]);
       gh.x = gl.x = mh.x = ml.x = ql.x = 0.0f;
       qh.x = 1.0f;
       sm.close = 1;
@@ -193,7 +237,7 @@ __device__ __forceinline__ void sym_step(SymShared<BLOCK>& sm, const ForceCtx& f
       double f[3] = {0.0, 0.0, 0.0};
       if (S.i1 < ns && j < ns) ff_close_pair(fc, j, p[0], p[1], p[2], gh.y, gl.y, f[0], f[1], f[2], r2h.y, r2l.y);
       if (DI)
-        for (int k = 0; k < 3; ++k) sm.sums[1][3 + k][threadIdx.x] += f[k];
+        for (int k = 0; k < 3; ++k) sym_add_close(sm, 3 + k, f[k]);
       gh.y = gl.y = mh.y = ml.y = ql.y = 0.0f;
       qh.y = 1.0f;
       sm.close = 1;
@@ -258,7 +302,12 @@ __device__ __noinline__ void sym_close_pass(SymShared<BLOCK>& sm, const ForceCtx
       float a, b;
       ff_close_pair(fc, i, p[0], p[1], p[2], T[(size_t)FGH * np + i], T[(size_t)FGL * np + i], f[0], f[1], f[2], a, b);
     }
-    for (int k = 0; k < 3; ++k) sm.js[k][q] += f[k];
+    for (int k = 0; k < 3; ++k) {
+      if constexpr (BLOCK > 64)
+        add_ordered(sm.js[0][k][q], sm.js[1][k][q], f[k]);
+      else
+        sm.js[0][k][q] += f[k];
+    }
   }
 }
 
@@ -371,7 +420,6 @@ __global__ void __launch_bounds__(sym_threads(BLOCK), sym_ctas(BLOCK))
         sm.tile.v[k][q] = make_float4(v, v, w, w);
       }
     for (int q = threadIdx.x; q < BLOCK; q += kThreads) {
-      sm.js[0][q] = sm.js[1][q] = sm.js[2][q] = 0.0;
       sm.jmh[q] = bound[j0 + q];
       sm.jml[q] = 3.0e38f;
       sm.jnn[q] = -1;
@@ -383,7 +431,7 @@ __global__ void __launch_bounds__(sym_threads(BLOCK), sym_ctas(BLOCK))
     for (int k = 0; k < 3; ++k) A.h[k] = A.l[k] = make_float2(0.0f, 0.0f);
 #pragma unroll 1
     for (int p = 0; p < kParts; ++p) {
-      const int sub = (p + 2 * warp) & (kParts - 1);  // a part of its own for every warp
+      const int sub = (p + 2 * warp) & (kParts - 1);  // a part of its own for every warp, its first for p = 0 and 1
       const int q = sub * 32 + lane;
       SymSums B;
 #pragma unroll
@@ -396,17 +444,14 @@ __global__ void __launch_bounds__(sym_threads(BLOCK), sym_ctas(BLOCK))
         sym_part<false, true>(sm, fc, y, sub, lane, j0, ns, thr, S, A, n0, n1, B);
       if (want_j) {
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          float u, e;  // both lanes in FP32 first: a warp waits 64 cycles for an FP64 instruction
-          ff_two_sum(B.h[k].x, B.h[k].y, u, e);
-          sm.js[k][q] += (double)u + (double)(e + (B.l[k].x + B.l[k].y));
-        }
+        for (int k = 0; k < 3; ++k)
+          sym_add_source(sm, k, q, sym_lanes(B.h[k], B.l[k]), p < 2);
       }
       if (want_i && ((p & 3) == 3 || p == kParts - 1)) {  // the sinks' float-float sums of 128 sources into FP64
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-          sm.sums[0][k][threadIdx.x] += (double)A.h[k].x + (double)A.l[k].x;
-          sm.sums[0][3 + k][threadIdx.x] += (double)A.h[k].y + (double)A.l[k].y;
+          sym_add_sink(sm, k, (double)A.h[k].x + (double)A.l[k].x);
+          sym_add_sink(sm, 3 + k, (double)A.h[k].y + (double)A.l[k].y);
           A.h[k] = A.l[k] = make_float2(0.0f, 0.0f);
         }
       }
@@ -419,9 +464,12 @@ __global__ void __launch_bounds__(sym_threads(BLOCK), sym_ctas(BLOCK))
       }
       double* out = part_j + sym_pair_index(I, J, nb) * PART_SLOTS * BLOCK;
       for (int q = threadIdx.x; q < BLOCK; q += kThreads) {
-        out[PAX * BLOCK + q] = sm.js[0][q];
-        out[PAY * BLOCK + q] = sm.js[1][q];
-        out[PAZ * BLOCK + q] = sm.js[2][q];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          double v = sm.js[0][k][q];
+          if constexpr (BLOCK > 64) v += sm.js[1][k][q];
+          out[(PAX + k) * BLOCK + q] = v;
+        }
         out[PR2 * BLOCK + q] = sm.jnn[q] >= 0 ? (double)sm.jmh[q] + (double)sm.jml[q] : 1.0e300;
         out[PIDX * BLOCK + q] = __longlong_as_double((long long)sm.jnn[q]);
       }
