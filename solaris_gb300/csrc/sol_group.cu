@@ -494,13 +494,6 @@ __device__ __noinline__ void work(const GroupArgs& P, const View& V, const Ctl& 
         if (m < nmig) {
           const int s = V.mlist[m], i = body_of(P, V, s), kind = V.kind[s];
           mig_compute(fc, i, kind, yt + 6 * s, S.factor, flags, V.gbuf + 3 * s, V.mig + s);
-          if (s >= P.ns || home) {
-            double* gb = global_gas_buf(fc, i, kind);
-            gb[0] = V.gbuf[3 * s + 0];
-            gb[1] = V.gbuf[3 * s + 1];
-            gb[2] = V.gbuf[3 * s + 2];
-            fc.mig_type[i] = V.mig[s];
-          }
         }
       }
     }
@@ -685,7 +678,8 @@ __global__ void __launch_bounds__(MAXT) k_group_rkf78(GroupArgs P) {
     V.mig[s] = fc.mig_type[i];
     const int kind = gas_kind(fc, i);
     V.kind[s] = kind;
-    for (int k = 0; k < 3; ++k) V.gbuf[3 * s + k] = kind ? global_gas_buf(fc, i, kind)[k] : 0.0;
+    // (the drag's is formed anew by the first evaluation)
+    for (int k = 0; k < 3; ++k) V.gbuf[3 * s + k] = kind >= 2 ? global_gas_buf(fc, i, kind)[k] : 0.0;
     const int nsrc = (fc.type[i] <= SOL_PROTO_PLANET) ? ns : fc.cls.nm;
     // items of sinks i >= 1: the origin, sources 1 <= j < nsrc, j != i
     V.base[s] = i == 0 ? 0 : nsrc - ((i < nsrc) ? 1 : 0);
@@ -917,6 +911,16 @@ __global__ void __launch_bounds__(MAXT) k_group_rkf78(GroupArgs P) {
       y0 = S.flush && fabs(yn) < 1.0e-50 ? 0.0 : yn;
     }
   }
+  // A block may start late: what it reads at its start (the state, the control
+  // record, the migration's state and buffers) is written from here on, when every
+  // block has exchanged a word with the others.  (RK4 calls outside the step loop
+  // have had no exchange yet.)
+  if (ran && P.rk4 && !P.sim && gridDim.x > 1 && !S.abort) {
+    if (warp == 0) {
+      __threadfence();
+      if (!exchange(P, k, 0, 0).ok) S.abort = 1;
+    }
+  }
   if (threadIdx.x == 0) {
     if (pending) grow(S);
     S.leave = 1;
@@ -934,6 +938,13 @@ __global__ void __launch_bounds__(MAXT) k_group_rkf78(GroupArgs P) {
       P.err[ge] = err;
     }
   }
+  if (ran && home)  // migrating bodies are sources
+    for (int q = threadIdx.x; q < S.nmig; q += nstate) {
+      const int s = V.mlist[q], i = body_of(P, V, s);
+      double* gb = global_gas_buf(fc, i, V.kind[s]);
+      for (int c = 0; c < 3; ++c) gb[c] = V.gbuf[3 * s + c];
+      fc.mig_type[i] = V.mig[s];
+    }
   if (home && threadIdx.x == 0) {
     sol_ctrl* c = P.ctrl;
     c->t = S.t;

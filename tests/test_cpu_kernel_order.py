@@ -44,3 +44,18 @@ def test_source_minima_are_ordered_between_two_steps_of_a_warp():
     steps = re.findall(r"sym_step<[^;]*;\s*(\w+)", body)
     assert len(steps) == 2
     assert steps == ["__syncwarp"] * 2
+
+
+def test_group_launch_keeps_what_a_late_block_still_reads():
+    """Every block of the group driver reads the start state, the control record
+    and the migration state of the sources at its start, which may be late: the
+    home block writes them at the launch's end only, and there (also in RK4
+    calls outside the step loop, which exchange nothing) after an exchange."""
+    work = _body("sol_group.cu", "work")
+    migration = work[work.index("mig_compute("):work.index("part_sync(1")]
+    assert "global_gas_buf" not in migration and "fc.mig_type" not in migration
+    kernel = _body("sol_group.cu", "k_group_rkf78")
+    end = kernel[kernel.index("pending = !P.rk4"):]
+    guard = end.index("if (ran && P.rk4 && !P.sim && gridDim.x > 1 && !S.abort)")
+    assert guard < end.index("exchange(P, k") < end.index("if (S.abort) return;") < end.index("P.y0[ge] = y0")
+    assert end.index("if (S.abort) return;") < end.index("fc.mig_type[")
