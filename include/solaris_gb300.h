@@ -464,7 +464,8 @@ int sol_ensemble_set_state(sol_ensemble* ens, const double* y0_all, const sol_ti
 int sol_ensemble_get_state(sol_ensemble* ens, double* y0_all, sol_time_line* time_lines, int32_t* status);
 /* n_steps driver calls for every system */
 int sol_ensemble_advance(sol_ensemble* ens, int32_t n_steps, sol_step_stats* stats);
-/* launch shape: threads per system (multiple of 32) and resident systems per SM */
+/* launch shape: threads per system (a multiple of 32 in [32, 736]) and resident
+ * systems per SM (1 to 32); SOL_ERR_ARG for any other */
 int sol_ensemble_configure(sol_ensemble* ens, int32_t threads_per_system, int32_t systems_per_sm);
 /* times `steps` driver calls for each candidate launch shape on a copy of the
  * state, restores the state and keeps the fastest shape */

@@ -36,7 +36,7 @@ struct EnsCtrl {
   long long n_acc, n_rej;
 };
 
-constexpr int kMaxThreads = 736;  // 88 registers; the largest launch shape sol_ensemble_configure takes effect with
+constexpr int kMaxThreads = 736;  // of 88 registers: the largest launch shape sol_ensemble_configure takes
 constexpr int kVecs = 17;  // f0..f12, yscale, ytmp, y, error
 enum { V_YSCALE = 13, V_YTMP = 14, V_Y = 15, V_ERR = 16 };
 
@@ -653,9 +653,9 @@ int sol_ensemble_advance(sol_ensemble* e, int32_t n_steps, sol_step_stats* stats
 }
 
 int sol_ensemble_configure(sol_ensemble* e, int32_t threads_per_system, int32_t systems_per_sm) {
-  if (!e || threads_per_system < 32 || threads_per_system > 1024 || (threads_per_system & 31) ||
+  if (!e || threads_per_system < 32 || threads_per_system > kMaxThreads || (threads_per_system & 31) ||
       systems_per_sm < 1 || systems_per_sm > 32) {
-    sol_set_error("threads per system must be a multiple of 32 in [32, 1024], systems per SM in [1, 32]");
+    sol_set_error("threads per system must be a multiple of 32 in [32, %d], systems per SM in [1, 32]", kMaxThreads);
     return SOL_ERR_ARG;
   }
   SOL_CUDA(cudaSetDevice(e->device));
