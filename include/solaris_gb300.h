@@ -468,7 +468,10 @@ int sol_ensemble_advance(sol_ensemble* ens, int32_t n_steps, sol_step_stats* sta
  * systems per SM (1 to 32); SOL_ERR_ARG for any other */
 int sol_ensemble_configure(sol_ensemble* ens, int32_t threads_per_system, int32_t systems_per_sm);
 /* times `steps` driver calls for each candidate launch shape on a copy of the
- * state, restores the state and keeps the fastest shape */
+ * state, restores the state and keeps the fastest shape.  Candidates: 64, 128 and
+ * 256 threads with 2, 4, 8 and 16 systems an SM; with more systems than SMs the
+ * present shape and the default ones too (with fewer the default, 640 threads, is
+ * faster than any candidate: leave it) */
 int sol_ensemble_autotune(sol_ensemble* ens, int32_t steps, int32_t* threads_per_system, int32_t* systems_per_sm,
                           double* best_ms);
 

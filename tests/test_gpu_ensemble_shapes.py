@@ -1,6 +1,8 @@
 """Launch shapes of an ensemble: the largest number of threads a system that the
 kernel can be launched with is accepted and runs, a larger one is refused when it
 is set, in both precisions."""
+import time
+
 import numpy as np
 import pytest
 
@@ -38,3 +40,28 @@ def test_larger_shapes_are_refused(threads):
         assert err.value.code == abi.SOL_ERR_ARG and str(LARGEST) in str(err.value)
         ens.set_state([systems[0].y0], [0.0], [systems[0].h0])
         ens.advance(1)  # with the shape it had
+
+
+def test_the_tuned_shape_is_not_slower_than_the_default():
+    """300 systems, about two an SM: the default shape is ~30 % faster than the
+    twelve of other sizes, so a tuner that does not try it is found out."""
+    rng = np.random.default_rng(9)
+    systems = [scenarios.config4_system(rng, k) for k in range(300)]
+    ms = {}
+    for tuned in (False, True):
+        with engine.Ensemble(systems) as ens:
+            ens.set_state([s.y0 for s in systems], [0.0] * 300, [s.h0 for s in systems])
+            before = ens.get_state()
+            if tuned:
+                ens.autotune(steps=1)
+                after = ens.get_state()
+                assert np.array_equal(np.concatenate(before[0]).view(np.uint64), np.concatenate(after[0]).view(np.uint64))
+                assert before[1] == after[1]
+            best = np.inf
+            for _ in range(6):
+                ens.set_state([s.y0 for s in systems], [0.0] * 300, [s.h0 for s in systems])
+                t = time.perf_counter()
+                ens.advance(1)
+                best = min(best, time.perf_counter() - t)
+            ms[tuned] = 1e3 * best
+    assert ms[True] <= 1.15 * ms[False], ms
