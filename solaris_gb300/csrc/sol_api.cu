@@ -11,7 +11,7 @@
 #include "sol_internal.cuh"
 
 int sol_force_tile();
-int sol_force_alloc_parts(sol_ctx* c);
+int sol_force_alloc_parts(sol_ctx* c, int precision);
 int sol_force_uses_chunk_partials(const sol_ctx* c, int precision);
 int sol_force_prepass_blocks(int npad);
 int sol_force_src_doubles();
@@ -409,9 +409,9 @@ int sol_set_precision(sol_ctx* c, int32_t p) {
     sol_set_error("precision %d: barycentric contexts compute in FP64 only", p);
     return SOL_ERR_ARG;
   }
-  if (p != SOL_PRECISION_FP64 && !c->barycentric && !c->d_part && sol_force_uses_chunk_partials(c, p)) {
+  if (p != SOL_PRECISION_FP64 && !c->barycentric && sol_force_uses_chunk_partials(c, p)) {
     RET(set_device(c));
-    RET(sol_force_alloc_parts(c));
+    RET(sol_force_alloc_parts(c, p));
   }
   if (c->precision != p) sol_adjoint_model_changed(c);
   c->precision = p;

@@ -1842,9 +1842,9 @@ int sol_force_launch_sinks(sol_ctx* c, const double* d_y, double* d_dydt, TimeSp
 
 int sol_force_tile() { return kTile; }
 int sol_force_src_doubles() { return kSrcDoubles; }
-// Partials for either split form's 2-D kernels, of this system and of every
-// smaller one it can become (removed bodies): fewer blocks can have more
-// chunks.
+// Partials for either split form's 2-D kernels and, with `blocks`, for the block
+// pairs of a SPLIT_FF system that k_pairs_sym serves, of this system and of every
+// smaller one it can become (removed bodies): fewer blocks can have more chunks.
 static size_t part_doubles(const sol_ctx* c, bool blocks) {
   const size_t np = c->npad;
   size_t most = (size_t)((c->n + kChunk - 1) / kChunk) * PART_SLOTS * np;  // SPLIT
@@ -1854,7 +1854,7 @@ static size_t part_doubles(const sol_ctx* c, bool blocks) {
     const size_t d = (size_t)((n + ch - 1) / ch) * PART_SLOTS * np;
     if (d > most) most = d;
   }
-  if (!blocks) return most;
+  if (!blocks || sym_bodies(c->n, c->cls) == 0) return most;
   size_t sym = 0;
   for (int m = 64; m <= c->cls.nm + 255 && m <= kSymMax + 255; m += 64)
     for (int block = 64; block <= 256; block *= 2)
@@ -1868,17 +1868,28 @@ static size_t part_doubles(const sol_ctx* c, bool blocks) {
     sym += ((size_t)(kTile + c->cls.n_spl + kTile - 1) / kTile + (c->cls.nm + kTile - 1) / kTile) * PART_SLOTS * np;
   return sym > most ? sym : most;
 }
-// The partials' buffer (not cleared: what is read has been written): without
-// the block pairs' where they do not fit.
-int sol_force_alloc_parts(sol_ctx* c) {
+// The partials' buffer for a split precision (not cleared: what is read has been
+// written), kept where it is large enough; without the block pairs' where they do
+// not fit.  A larger one may become necessary with another precision, or when the
+// last light body is removed; captured graphs hold the old one's address.
+int sol_force_alloc_parts(sol_ctx* c, int precision) {
   for (bool blocks : {true, false}) {
+    if (blocks && precision != SOL_PRECISION_SPLIT_FF) continue;
     const size_t doubles = part_doubles(c, blocks);
-    if (cudaMalloc((void**)&c->d_part, sizeof(double) * doubles) == cudaSuccess) {
-      c->part_doubles = doubles;
-      return SOL_OK;
+    if (c->d_part && c->part_doubles >= doubles) return SOL_OK;
+    double* part = nullptr;
+    if (cudaMalloc((void**)&part, sizeof(double) * doubles) != cudaSuccess) {
+      cudaGetLastError();
+      continue;
     }
-    c->d_part = nullptr;
-    cudaGetLastError();
+    if (c->d_part) {
+      for (DriverGraph& G : c->graphs) sol_graph_release(G);
+      SOL_CUDA(cudaStreamSynchronize(c->stream));
+      cudaFree(c->d_part);
+    }
+    c->d_part = part;
+    c->part_doubles = doubles;
+    return SOL_OK;
   }
   sol_set_error("cudaMalloc of the split partials failed");
   return SOL_ERR_NOMEM;
