@@ -110,7 +110,14 @@ GasDev make_gas_dev(const sol_gas_component* g, int barycentric) {
   return d;
 }
 
-constexpr size_t kStagedBytes = 256 * 1024;  // dydt of up to 5,461 bodies comes back through the pinned slab
+// What a host-buffer evaluation brings back through the pinned slab: dydt of up to
+// kStagedBytes (1,194 bodies), rm3 and the neighbours of up to kStagedRest (19,640).
+// A copy into pageable memory blocks for ~8 us whatever its size, up to 100 KB,
+// and takes 12 us at 480 KB; moving data again on the host ~30 us per MB.  Measured
+// (a call with few sources, us, dydt staged / copied): 500 bodies 40 / 42, 1,000 43
+// / 44, 1,500 51 / 50, 3,000 59 / 54, 5,461 71 / 58; rm3 and the neighbours: 5,462
+// 59 / 75, 10,000 67 / 78, 20,000 85 / 85, 28,000 100 / 91, 100,000 252 / 152.
+constexpr size_t kStagedBytes = 56 * 1024, kStagedRest = 384 * 1024;
 
 template <class T>
 int dev_alloc(T** p, size_t count) {
@@ -327,7 +334,7 @@ int sol_create(const sol_body_data* b, const sol_gas_component* gas, int32_t bar
   auto aligned = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t o_rm3 = aligned(sizeof(double) * NV), o_nd = o_rm3 + aligned(sizeof(double) * N),
                o_nn = o_nd + aligned(sizeof(double) * N), o_ctrl = o_nn + aligned(sizeof(int32_t) * N);
-  c->slab_from = sizeof(double) * NV <= kStagedBytes ? 0 : o_rm3;
+  c->slab_from = sizeof(double) * NV <= kStagedBytes ? 0 : o_ctrl - o_rm3 <= kStagedRest ? o_rm3 : o_ctrl;
   c->slab_bytes = o_ctrl + sizeof(sol_ctrl);
   if ((rc = dev_alloc(&c->d_slab, c->slab_bytes))) return fail(rc);
   c->d_io_out = reinterpret_cast<double*>(c->d_slab);
@@ -443,22 +450,24 @@ int sol_accel_compute(sol_ctx* c, double t, const double* y, double* dydt, doubl
   SOL_CUDA(cudaMemcpyAsync(c->d_io_in, y, sizeof(double) * c->nv, cudaMemcpyHostToDevice, c->stream));
   TimeSpec ts{nullptr, nullptr, 0.0, t};
   RET(sol_force_launch_parts(c, c->d_io_in, c->d_io_out, ts, c->eval_flags, 3, &c->d_ctrl->dev_status));
-  // A copy into pageable memory blocks for ~8 us whatever its size (measured
-  // up to 100 KB; 12 us at 480 KB), so rm3, the neighbours and the status
-  // come back in one asynchronous copy into the pinned slab.  dydt joins it
-  // while moving it again on the host (~30 us per MB) costs less than a copy
-  // of its own.
-  const size_t nb = sizeof(double) * c->nv;
+  // the slab in one copy, what lies before slab_from in copies of its own
   const size_t from = c->slab_from;
-  const bool staged = from == 0;
   SOL_CUDA(cudaMemcpyAsync(c->h_slab, c->d_slab + from, c->slab_bytes - from, cudaMemcpyDeviceToHost, c->stream));
-  if (!staged) SOL_CUDA(cudaMemcpyAsync(dydt, c->d_io_out, nb, cudaMemcpyDeviceToHost, c->stream));
+  struct {
+    void* to;
+    const void* d;
+    size_t bytes;
+  } const out[] = {{dydt, c->d_io_out, sizeof(double) * c->nv},
+                   {rm3, c->d_rm3, sizeof(double) * c->n},
+                   {nn_idx, c->d_nn_idx, sizeof(int32_t) * c->n},
+                   {nn_dist, c->d_nn_dist, sizeof(double) * c->n}};
+  auto at = [&](const void* d) { return (size_t)((const char*)d - c->d_slab); };
+  for (const auto& o : out)
+    if (o.to && at(o.d) < from) SOL_CUDA(cudaMemcpyAsync(o.to, o.d, o.bytes, cudaMemcpyDeviceToHost, c->stream));
   SOL_CUDA(cudaStreamSynchronize(c->stream));
-  auto host = [&](const void* d) { return c->h_slab + ((const char*)d - c->d_slab - from); };
-  if (staged) memcpy(dydt, host(c->d_io_out), nb);
-  if (rm3) memcpy(rm3, host(c->d_rm3), sizeof(double) * c->n);
-  if (nn_idx) memcpy(nn_idx, host(c->d_nn_idx), sizeof(int32_t) * c->n);
-  if (nn_dist) memcpy(nn_dist, host(c->d_nn_dist), sizeof(double) * c->n);
+  auto host = [&](const void* d) { return c->h_slab + (at(d) - from); };
+  for (const auto& o : out)
+    if (o.to && at(o.d) >= from) memcpy(o.to, host(o.d), o.bytes);
   memcpy(c->h_ctrl, host(c->d_ctrl), sizeof(sol_ctrl));
   c->last_eval_valid = 1;
   if (c->h_ctrl->dev_status & SOL_DEV_TIMEOUT) {

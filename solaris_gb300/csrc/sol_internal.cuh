@@ -160,10 +160,9 @@ struct sol_ctx {
   int32_t* d_nn_idx;
   double *d_y0, *d_y, *d_accel, *d_yscale, *d_err, *d_ytmp, *d_fk[13];
   double *d_io_in, *d_io_out;  // boundary staging for host-buffer calls
-  // what a host-buffer evaluation brings back, in one allocation so that one
-  // copy moves it: d_io_out, d_rm3, d_nn_dist, d_nn_idx and d_ctrl point into
-  // it, and h_slab (pinned) mirrors it from slab_from on (0, or behind dydt
-  // where that is large)
+  // what a host-buffer evaluation brings back, in one allocation: d_io_out, d_rm3,
+  // d_nn_dist, d_nn_idx and d_ctrl point into it, and h_slab (pinned) mirrors it
+  // from slab_from on (0; behind dydt, or at d_ctrl, where what lies before is large)
   char *d_slab, *h_slab;
   size_t slab_bytes, slab_from;
   double* d_partial;           // block partial maxima of the error norm
