@@ -156,7 +156,6 @@ __device__ __forceinline__ void part_sync(int id, int threads) {
 }
 
 struct Ctl {
-  double fac[4];  // RungeKutta4: ReductionFactor at the stage times t + c h
   double t, h, h_next, h_did, error_max, eps;
   long long n_acc, n_rej;
   int status, accepted, abort, nitem, ndrag, nmig;

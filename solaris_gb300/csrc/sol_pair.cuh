@@ -139,14 +139,10 @@ __device__ __forceinline__ void ff_pair_accumulate(double dxd, double dyd, doubl
 }
 
 // ---- FP32 seed, FP64 Newton step: the pieces that stay off the FP64 pipe ----
-// The FP32 seed y (positive, normal) as a double (exact), y^2 and y^3 in FP64
-// without FP64 instructions: from y's 24-bit significand m by integer
-// multiplies, y^2 = m^2 (48 bits, exact) and y^3 = m^3 (72 bits, truncated to
-// 53), with the exponents set directly.
-__device__ __forceinline__ double sol_seed_double(float yf) {
-  const int b = __float_as_int(yf);
-  return __hiloint2double((b >> 3) + 0x38000000, b << 29);
-}
+// y^2 and y^3 of the FP32 seed y (positive, normal) in FP64 without FP64
+// instructions: from y's 24-bit significand m by integer multiplies, y^2 = m^2
+// (48 bits, exact) and y^3 = m^3 (72 bits, truncated to 53), with the exponents
+// set directly.
 __device__ __forceinline__ void sol_seed_square_cube(float yf, double& u, double& y3) {
   const unsigned b = __float_as_uint(yf);
   const int E = (int)(b >> 23) - 127;  // yf = 2^E m 2^-23
@@ -168,21 +164,6 @@ __device__ __forceinline__ double sol_seed_square(float yf) {
   return __longlong_as_double(((long long)(2 * E + c2 + 1023) << 52) | ((m2 << (6 - c2)) & 0xFFFFFFFFFFFFFull));
 }
 
-// 1 + c e^2 in FP64 (0 <= c <= 2) from e's high word: for a Newton residual
-// (|e| < 2^-20) the term is below 2^-37 and is needed to 2^-53, i.e. to 16 of
-// its own bits, which FP32 gives; it is placed in the low bits of 1.0 by an
-// integer addition.  Larger |e| (only a pair at r^2 = 0, whose seed is
-// clamped) is clamped so that the result stays finite.
-__device__ __forceinline__ double sol_one_plus_ce2(double e, float c) {
-  const int eh = __double2hiint(e);
-  const int ex = (eh >> 20) & 0x7FF;
-  const int fx = min(ex, 0x47E) - 0x380;  // float exponent field of |e|
-  const float ef = fx > 0 ? __int_as_float((fx << 23) | ((eh & 0xFFFFF) << 3)) : 0.0f;
-  const float q = fminf(c * ef * ef, 4.656612873077393e-10f);  // <= 2^-31
-  const float t = __fmaf_rn(q, 4503599627370496.0f, 12582912.0f);  // q 2^52 + 1.5 2^23: rounds to an integer
-  return __longlong_as_double(0x3FF0000000000000LL + (long long)(__float_as_int(t) - 0x4B400000));
-}
-
 // t = 3/2 e + 15/8 e^2 in FP64 without FP64 instructions, for the Newton
 // correction r^-3 = y^3 (1 + t) of a residual e (|e| < 2^-20 for a seed of
 // r^2; e = 1 for r^2 = 0, whose displacement is 0).  3/2 e is 3 M exactly,
@@ -201,7 +182,7 @@ __device__ __forceinline__ double sol_split_t(double e) {
   const long long M = (eb & 0xFFFFFFFFFFFFFLL) | (1LL << 52);
   long long S = 3 * M;  // 3/2 e in units of 2^(ex - 1076)
   if (eb < 0) S = -S;
-  // 15/8 e^2 from e's high word (as sol_one_plus_ce2), clamped to 2^-31
+  // 15/8 e^2 in FP32 from e's high word, clamped to 2^-31 (larger |e|: a pair at r^2 = 0 alone)
   const int eh = (int)(eb >> 32);
   const int fx = min(ex, 0x47E) - 0x380;
   const float ef = fx > 0 ? __int_as_float((fx << 23) | ((eh & 0xFFFFF) << 3)) : 0.0f;
@@ -315,7 +296,7 @@ __device__ __forceinline__ void f2_ff_r2(const float2* h, const float2* l, float
 // product is left unnormalised: its low word, the TwoProduct error and the
 // two cross terms, stays within 3 2^-24 of the high word, and the
 // accumulation that takes it multiplies it by the displacement with one
-// rounding (f2_ff_accumulate).
+// rounding (f2_ff_accumulate_lazy).
 // (f2_ff_rinv3 gives r^-3, f2_ff_scale its product with G m.)
 __device__ __forceinline__ void f2_ff_rinv3(float2 qh, float2 ql, float2& Rh, float2& Rl) {
   const float2 y = make_float2(sol_rsqrt_normal(qh.x), sol_rsqrt_normal(qh.y));
@@ -338,11 +319,13 @@ __device__ __forceinline__ void f2_ff_gm_rinv3(float2 qh, float2 ql, float2 gh, 
   f2_ff_scale(gh, gl, Rh, Rl, sh, se);
 }
 
-// A += s d without the final renormalisation: the caller renormalises
-// (FastTwoSum of (Ah, Al)) after every second accumulation, so Al holds at
-// most two steps' errors (|Al| <= ~4 2^-24 |Ah|) and the rounding of its
-// additions stays at ~2^-46 of |A| per step, as with a renormalisation
-// after every step (f2_ff_accumulate), for 3 fewer FP32 operations.
+// A += s d for one component, float-float (|s_lo| <= 3 2^-24 |s_hi|), without
+// the final renormalisation: the caller renormalises (FastTwoSum of (Ah, Al))
+// after every second accumulation, so Al holds at most two steps' errors (|Al|
+// <= ~4 2^-24 |Ah|) and the rounding of its additions stays at ~2^-46 of |A| per
+// step, as with a renormalisation after every step, for 3 fewer FP32 operations.
+// (Knuth's TwoSum: ordering the pair by magnitude instead put a compare and two
+// selections on this accumulator's serial chain and measured 4% slower.)
 __device__ __forceinline__ void f2_ff_accumulate_lazy(float2& Ah, float2& Al, float2 sh, float2 se, float2 dh,
                                                       float2 dl) {
   float2 ah, ae;
@@ -352,18 +335,4 @@ __device__ __forceinline__ void f2_ff_accumulate_lazy(float2& Ah, float2& Al, fl
   f2_two_sum(Ah, ah, s1, s2);
   Ah = s1;
   Al = f2_add(Al, f2_add(s2, ae));
-}
-
-// A += s d for one component, float-float (s and d float-float, |s_lo| <=
-// 3 2^-24 |s_hi|; A kept normalised).
-__device__ __forceinline__ void f2_ff_accumulate(float2& Ah, float2& Al, float2 sh, float2 se, float2 dh, float2 dl) {
-  float2 ah, ae;
-  f2_two_prod(sh, dh, ah, ae);
-  ae = f2_fma(sh, dl, f2_fma(se, dh, ae));
-  float2 s1, s2;
-  // (Knuth's TwoSum: ordering the pair by magnitude instead put a compare and
-  // two selections on this accumulator's serial chain and measured 4% slower)
-  f2_two_sum(Ah, ah, s1, s2);
-  s2 = f2_add(s2, f2_add(Al, ae));
-  f2_fast_two_sum(s1, s2, Ah, Al);
 }
