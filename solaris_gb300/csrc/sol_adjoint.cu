@@ -12,7 +12,7 @@
 // and lambda_n = lambda_{n+1} + sum_k nu_k, with the mass gradient
 // accumulated from the same w_k.  Stages 11 and 12 only enter the error
 // estimate, so their adjoints are zero.  J^T w is a hand-written
-// vector-Jacobian product of the pair force (one warp per body).
+// vector-Jacobian product of the pair force (block pairs, or a CTA per body).
 #include <algorithm>
 #include <cmath>
 #include <cstring>

@@ -1566,8 +1566,8 @@ static int ff_chunk(int device, long nsink, long nsrc) {
 // How a SPLIT_FF evaluation is divided.  k_pairs_sym takes the massive bodies
 // (which attract each other) in whole blocks, the last one padded where every
 // body is massive; k_pairs_ff the rest.  From kSymMin bodies on (us an
-// evaluation with it and without: 1,025 bodies 65 and 52, 1,250 61 and 71, 2,049
-// 65 and 99, 3,100 85 and 145, 4,096 98 and 108, 7,000 191 and 236), kSymMinMixed
+// evaluation with it and without: 1,025 bodies 65 and 52, 1,250 65 and 71, 2,049
+// 67 and 99, 3,100 86 and 145, 4,096 98 and 108, 7,000 188 and 236), kSymMinMixed
 // where others are left to k_pairs_ff (two launches more: 100 light bodies beside
 // 6,200 massive 204 and 192, beside 8,300 295 and 340), up to kSymMax, beyond
 // which the block pairs' partials (10 KB each) would pass 1.4 GB.  Small blocks are many and
